@@ -6,10 +6,11 @@
 //   warp 8      TMA producer   : Q tiles once, then K/V blocks through two rings
 //   warp 9      MMA issuer     : S = Q K^T (tcgen05.mma, smem x smem -> TMEM)
 //                                O += P V  (tcgen05.mma, TMEM x smem -> TMEM)
-//                                (issuing a tcgen05.mma holds the issuing thread for about as long as the
-//                                MMA runs -- 64 cycles at 128x128x16 -- so whatever else this thread does
-//                                between two MMAs idles the tensor pipe: operand barriers are polled before
-//                                the softmax hand-over, never after it)
+//                                (one elected thread; behind elect.sync it runs a few MMAs ahead of the tensor
+//                                pipe, so its barrier polls overlap with MMAs. Behind `lane == 0` every MMA took it 61
+//                                cycles to issue, which left the pipe idle at each hand-shake and ran the 128x64
+//                                P V of head_dim 64 at half rate: 250 -> 226 us at 24 heads x 4608 tokens x 128,
+//                                40.9 -> 37.6 ms at 6 heads x 119 k)
 //   warps 10-11 idle           : complete the third warpgroup so registers can be handed over
 //                                (setmaxnreg: 72 per thread there, 216 for the softmax threads;
 //                                72 + 2 * 216 = 3 * 168, the pool the CTA was launched with --
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
         inputs_ready = __all_sync(0xffffffffu, seen);
         asm volatile("fence.proxy.async;" ::: "memory");
       }
-      if (lane == 0 && inputs_ready) {
+      if (elect_one() && inputs_ready) {
         for (int s = 0; s < p.n_q_seg; ++s) tma_prefetch_desc(&p.q_map[s]);
         for (int s = 0; s < p.n_kv_seg; ++s) {
           tma_prefetch_desc(&p.k_map[s]);
@@ -426,10 +427,8 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
       }
     } else if (warp == 9) {
       // ============================ MMA issuer ============================
-      // One thread issues for both halves. (A second issuing thread, one per half, measured slower: 852 vs
-      // 1023 TFLOP/s at the Flux shape -- concurrent issuers slow each other down more than the barrier polls
-      // of a single one idle the pipe.)
-      if (lane == 0) {
+      // One thread issues for both halves.
+      if (elect_one()) {
         constexpr uint32_t kFmt = FP16 ? 0u : 1u;
         constexpr uint32_t idesc_qk = make_idesc_f16(kBlockM, kBlockN, kFmt, 0);
         constexpr uint32_t idesc_pv = make_idesc_f16(kBlockM, D, kFmt, 1);

@@ -20,6 +20,23 @@ __device__ __forceinline__ uint32_t lane_id() {
   return l;
 }
 
+// True in one lane of a converged warp. Single-thread work (tcgen05.mma, tcgen05.commit, TMA) is guarded by this and
+// not by `lane == 0`: these instructions take their operands from uniform registers, and only behind elect.sync does
+// the compiler know that one lane is active. Measured on B200: behind `lane == 0` issuing a tcgen05.mma took 61 cycles
+// whatever its shape -- as long as a 128x128x16 MMA runs, and twice as long as a 128x64x16 one -- behind elect.sync
+// about 4 cycles, with four to six MMAs queued before the issuing thread has to wait.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}"
+      : "=r"(pred));
+  return pred != 0;
+}
+
 // ----------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
