@@ -58,6 +58,12 @@ constexpr int kNumThreads = 384;  // 2 softmax warpgroups + 1 warpgroup holding 
 constexpr int kPanelBytes = 128 * 128;  // 128 rows x 64 16-bit elements, 128B-swizzled
 constexpr uint32_t kSpinLimit = 8u * 1000u * 1000u;
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
+// P of a KV block is handed to the MMA thread in two parts, the first after this many of its four 32-column chunks: the
+// first half of P V runs while the second half is exponentiated, which takes those MMAs off the chain softmax -> P V ->
+// next Q K^T that bounds a tile (3294 -> 3057 cycles per KV block pair at head_dim 128, 2048 of them MMAs). Measured
+// against one hand-over: 24 heads x 4608 x 128 266 -> 240 us, 3 heads 44.9 -> 39.2 us, 29.7 k x 119 k tokens 10.06 -> 9.3
+// ms; after one or three chunks it is 251 / 241 us. Four hand-overs cost more in waits than they overlap.
+constexpr int kPFirst = 2;
 constexpr float kLn2 = 0.69314718055994531f;
 constexpr int kSmCount = 148;
 
@@ -94,6 +100,7 @@ enum Where : int {
   W_SM_SFULL = 7,
   W_SM_ODONE = 8,
   W_PEER_FLAGS = 9,
+  W_MMA_PREST = 10,
 };
 
 struct alignas(64) AttnKernelParams {
@@ -137,38 +144,12 @@ struct alignas(64) AttnKernelParams {
   unsigned wait_spins;
 };
 
-// Tuning switches (compile-time so that variants can be measured against each other). The defaults are what
-// measured fastest on B200: the stale maximum, the polynomial exp2 and a third V stage each measured neutral or
-// slower (the S -> P -> MMA chain, not the special-function unit or the loads, bounds a KV block).
-//   HDIT_ATTN_STALE_MAX  1: from the second KV block on, exponentiate against the running maximum known
-//                           *before* the block (its own maximum is computed alongside and takes effect one
-//                           block later), which takes the row-maximum pass off the S -> P critical path.
-//   HDIT_ATTN_POLY8      of every 8 scores, how many (0, 2, 4) take a degree-3 polynomial exp2 on the FMA
-//                           pipe instead of ex2 on the special-function unit.
-//   HDIT_ATTN_VSTAGES128 V ring depth at head_dim 128 (K stays at 2: 227 KB of shared memory).
-#ifndef HDIT_ATTN_STALE_MAX
-#define HDIT_ATTN_STALE_MAX 0
-#endif
-#ifndef HDIT_ATTN_POLY8
-#define HDIT_ATTN_POLY8 0
-#endif
-#ifndef HDIT_ATTN_SPLIT_P
-#define HDIT_ATTN_SPLIT_P 0  // 1: head_dim 64 keeps P in TMEM columns of its own (see Cfg::kSplitP); measured slower
-#endif
-#ifndef HDIT_ATTN_LATE_KWAIT
-#define HDIT_ATTN_LATE_KWAIT 1  // 1: poll the next K block between P V and Q K^T instead of before the hand-over
-#endif
-#ifndef HDIT_ATTN_VSTAGES128
-#define HDIT_ATTN_VSTAGES128 2
-#endif
-constexpr float kOverflowGuard = 64.0f;  // log2 units a block may exceed the stale maximum before it is redone
-
 template <int D>
 struct Cfg {
   static constexpr int kPanels = D / 64;
   static constexpr int kTileBytes = kPanels * kPanelBytes;
   static constexpr int kStagesK = (D == 128) ? 2 : 4;
-  static constexpr int kStagesV = (D == 128) ? HDIT_ATTN_VSTAGES128 : 4;
+  static constexpr int kStagesV = (D == 128) ? 2 : 4;
   static constexpr int kSmemQ = 2 * kTileBytes;
   static constexpr int kSmemK = kStagesK * kTileBytes;
   static constexpr int kSmemV = kStagesV * kTileBytes;
@@ -177,14 +158,13 @@ struct Cfg {
   static constexpr uint32_t kTmemCols = 512;
   static constexpr uint32_t kColS = 0;      // + t * 128
   static constexpr uint32_t kColO = 256;    // + t * D
-  // head_dim 64 leaves 128 TMEM columns free. With HDIT_ATTN_SPLIT_P, P gets columns of its own there instead of
-  // overwriting S, so the next Q K^T of a tile may run as soon as the softmax threads have *read* S, which cuts
-  // the S -> P -> P V -> Q K^T chain. Measured on B200 it is slower than the aliased layout (499 vs 596 TFLOP/s at
-  // 24 heads x 4429 tokens): both softmax groups then run in phase and contend for the special-function unit,
-  // where the aliased schedule keeps them half a block apart. Off by default.
-  static constexpr bool kSplitP = (D == 64) && (HDIT_ATTN_SPLIT_P != 0);
-  static constexpr uint32_t kColP = kSplitP ? 384 : kColS;  // + t * 64 when split, + t * 128 when aliased on S
-  static constexpr uint32_t kStrideP = kSplitP ? 64 : 128;
+  // Of every 8 scores, how many take the polynomial exp2 on the FMA pipe instead of ex2 on the special-function unit
+  // (16 per clock and SM). At head_dim 64 a KV block has as many scores as at 128 and half the MMAs, so the
+  // special-function unit is what both softmax groups compete for: two of eight moved off it took 24 heads x 4429 tokens,
+  // batch 2, from 371 to 353 us and 48 heads x 11.4 k x 33.7 k from 6.39 to 5.93 ms; four of eight are slower (the FMA and
+  // ALU work of a pair, 25 cycles of a warp, then exceeds the 16 cycles of its two ex2). At head_dim 128 it is neutral in
+  // long runs (242 / 239 us at 24 x 4608) and slower where the SMs run at full clock (39.1 -> 40.7 us at 3 x 4608).
+  static constexpr int kPoly8 = (D == 64) ? 2 : 0;
 };
 
 struct KvCursor {
@@ -221,9 +201,10 @@ __device__ __forceinline__ void load_tile(const CUtensorMap* map, bool swapped, 
   }
 }
 
+// Largest of three, NaN if one of them is.
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
 
@@ -238,9 +219,10 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   }
 }
 
-// 2^x for a pair of scores on the FMA pipe: x = n + f with n = round(x), f in [-0.5, 0.5]; 2^f by a degree-3
-// polynomial (relative error 7.5e-5, well below the 16-bit rounding of P), 2^n by adding n to the exponent
-// field. Inputs below -126 (masked scores are -inf) clamp to 2^-126.
+// 2^x for a pair of scores on the FMA pipe: x = n + f with n = round(x), f in [-0.5, 0.5]; 2^f by a degree-5
+// polynomial with constant term 1, fitted for the smallest largest relative error (9.1e-8; evaluated in fp32 at most
+// 1.7e-7, below the 2^-22 that ex2.approx is documented with), 2^n by adding n to the exponent field. Inputs below -126
+// (masked scores are -inf) clamp to 2^-126, and so does NaN: the row maximum carries NaN instead.
 __device__ __forceinline__ float2 ex2_poly2(float2 x) {
   x.x = fmaxf(x.x, -126.0f);
   x.y = fmaxf(x.y, -126.0f);
@@ -248,9 +230,11 @@ __device__ __forceinline__ float2 ex2_poly2(float2 x) {
   const float2 t = __fadd2_rn(x, magic);
   const float2 r = __fadd2_rn(t, make_float2(-12582912.0f, -12582912.0f));
   const float2 f = __ffma2_rn(r, make_float2(-1.0f, -1.0f), x);
-  float2 q = __ffma2_rn(f, make_float2(0.05517167f, 0.05517167f), make_float2(0.24261113f, 0.24261113f));
-  q = __ffma2_rn(q, f, make_float2(0.69326097f, 0.69326097f));
-  q = __ffma2_rn(q, f, make_float2(0.99992806f, 0.99992806f));
+  float2 q = __ffma2_rn(f, make_float2(0.00132647273f, 0.00132647273f), make_float2(0.00967151299f, 0.00967151299f));
+  q = __ffma2_rn(q, f, make_float2(0.0555073358f, 0.0555073358f));
+  q = __ffma2_rn(q, f, make_float2(0.240222424f, 0.240222424f));
+  q = __ffma2_rn(q, f, make_float2(0.693147004f, 0.693147004f));
+  q = __ffma2_rn(q, f, make_float2(1.0f, 1.0f));
   float2 out;
   out.x = __int_as_float(__float_as_int(q.x) + (__float_as_int(t.x) << 23));
   out.y = __int_as_float(__float_as_int(q.y) + (__float_as_int(t.y) << 23));
@@ -275,9 +259,8 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
   uint64_t* p_ready = s_full + 2;                // [2]
   uint64_t* o_done = p_ready + 2;                // [2]
   uint64_t* merge_bar = o_done + 2;              // [1] interleaved mode: half 1's partial result is in smem
-  uint64_t* s_free = merge_bar + 1;              // [2] split-P: the softmax threads have read S into registers
-  uint64_t* pv_done = s_free + 2;                // [2] split-P: P V is done (P may be overwritten, O is stable)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
+  uint64_t* p_rest = merge_bar + 1;              // [2] the second part of P is in TMEM (p_ready: the first)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_rest + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -314,8 +297,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
       mbar_init(&s_full[i], 1);
       mbar_init(&p_ready[i], 4);  // one arrival per softmax warp
       mbar_init(&o_done[i], 1);
-      mbar_init(&s_free[i], 4);
-      mbar_init(&pv_done[i], 1);
+      mbar_init(&p_rest[i], 4);
     }
     mbar_init(merge_bar, 4);
     for (int i = 0; i < C::kStagesK; ++i) {
@@ -394,17 +376,9 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
               break;
             }
           }
-#if defined(HDIT_ATTN_PROBE) && HDIT_ATTN_PROBE == 3
-          // timing probe (wrong results): after the first ring fill nothing is loaded any more
-          if (j >= C::kStagesK) {
-            mbar_arrive(&k_full[sk]);
-          } else
-#endif
-          {
-            mbar_expect_tx(&k_full[sk], C::kTileBytes);
-            load_tile(&p.k_map[cur.seg], p.k_swap[cur.seg], smem_k + sk * C::kTileBytes, &k_full[sk], C::kPanels, h,
-                      cur.row0, b);
-          }
+          mbar_expect_tx(&k_full[sk], C::kTileBytes);
+          load_tile(&p.k_map[cur.seg], p.k_swap[cur.seg], smem_k + sk * C::kTileBytes, &k_full[sk], C::kPanels, h,
+                    cur.row0, b);
           if (j >= C::kStagesV) {
             if (!mbar_wait_bounded(&v_empty[sv], (nv - 1) & 1, abort_flag, kSpinLimit)) {
               report_failure(p.status, abort_flag, HDIT_ERR_PEER_TIMEOUT, W_PROD_VEMPTY, j);
@@ -412,16 +386,9 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
               break;
             }
           }
-#if defined(HDIT_ATTN_PROBE) && HDIT_ATTN_PROBE == 3
-          if (j >= C::kStagesV) {
-            mbar_arrive(&v_full[sv]);
-          } else
-#endif
-          {
-            mbar_expect_tx(&v_full[sv], C::kTileBytes);
-            load_tile(&p.v_map[cur.seg], p.v_swap[cur.seg], smem_v + sv * C::kTileBytes, &v_full[sv], C::kPanels, h,
-                      cur.row0, b);
-          }
+          mbar_expect_tx(&v_full[sv], C::kTileBytes);
+          load_tile(&p.v_map[cur.seg], p.v_swap[cur.seg], smem_v + sv * C::kTileBytes, &v_full[sv], C::kPanels, h,
+                    cur.row0, b);
           cur.advance(p);
         }
       }
@@ -451,12 +418,12 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
             umma_ss(d_tmem, a0 + off, b0 + off, idesc_qk, kk > 0 ? 1u : 0u);
           }
         };
-        auto issue_pv = [&](int t, int stage, bool accumulate) {
+        auto issue_pv = [&](int t, int stage, bool accumulate, int kk0, int kk1) {
           const uint32_t d_tmem = tmem_base + C::kColO + t * D;
-          const uint32_t a_tmem = tmem_base + C::kColP + t * C::kStrideP;
+          const uint32_t a_tmem = tmem_base + C::kColS + t * 128;
           const uint64_t b0 = v_desc0 + static_cast<uint32_t>((stage * C::kTileBytes) >> 4);
 #pragma unroll
-          for (int kk = 0; kk < kBlockN / 16; ++kk) {
+          for (int kk = kk0; kk < kk1; ++kk) {
             umma_ts(d_tmem, a_tmem + kk * 8, b0 + static_cast<uint32_t>((kk * 2048) >> 4), idesc_pv,
                     (accumulate || kk > 0) ? 1u : 0u);
           }
@@ -503,36 +470,6 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
           g_attn_trace_mma[0][63][1] = static_cast<long long>(ns);
         }
 #endif
-        if constexpr (C::kSplitP) {
-          // P has its own columns: per round, first the next Q K^T of every half (needs only that the softmax
-          // threads have read the current S), then the P V of every half as its P arrives.
-          for (int i = 0; i < n_iter && ok; ++i) {
-            for (int t = 0; t <= last_t && ok; ++t) {
-              const int j = il ? 2 * i + t : i;
-              const int jn = j + blk_step;
-              if (j >= nblk || jn >= nblk) continue;
-              if (il || t == 0) wait(&k_full[k_stage(jn)], k_phase(jn), W_MMA_KFULL, jn);
-              wait(&s_free[t], i & 1, W_MMA_PREADY, 1000 + i * 2 + t);
-              if (!ok) break;
-              tc_fence_after();
-              issue_qk(t, k_stage(jn));
-              tc_commit(&s_full[t]);
-              if (il || t == last_t) tc_commit(&k_empty[k_stage(jn)]);
-            }
-            for (int t = 0; t <= last_t && ok; ++t) {
-              const int j = il ? 2 * i + t : i;
-              if (j >= nblk) break;
-              if (il || t == 0) wait(&v_full[v_stage(j)], v_phase(j), W_MMA_VFULL, j);
-              wait(&p_ready[t], i & 1, W_MMA_PREADY, i * 2 + t);
-              if (!ok) break;
-              tc_fence_after();
-              issue_pv(t, v_stage(j), i > 0);
-              tc_commit(&pv_done[t]);
-              if (j + blk_step >= nblk) tc_commit(&o_done[t]);
-              if (il || t == last_t) tc_commit(&v_empty[v_stage(j)]);
-            }
-          }
-        } else
         for (int i = 0; i < n_iter && ok; ++i) {
           for (int t = 0; t <= last_t && ok; ++t) {
             // half t's i-th KV block and the one after it
@@ -543,22 +480,21 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
             const bool releases = il || t == last_t;  // the last reader of a stage hands it back
             if (il || t == 0) {
               wait(&v_full[v_stage(j)], v_phase(j), W_MMA_VFULL, j);
-#if !HDIT_ATTN_LATE_KWAIT
-              if (has_next) wait(&k_full[k_stage(jn)], k_phase(jn), W_MMA_KFULL, jn);
-#endif
             }
             HDIT_TRACE_MMA(t, i, 0);
             wait(&p_ready[t], i & 1, W_MMA_PREADY, i * 2 + t);
             HDIT_TRACE_MMA(t, i, 1);
             if (!ok) break;
             tc_fence_after();
-            issue_pv(t, v_stage(j), i > 0);
+            issue_pv(t, v_stage(j), i > 0, 0, 2 * kPFirst);
+            wait(&p_rest[t], i & 1, W_MMA_PREST, i * 2 + t);
+            if (!ok) break;
+            tc_fence_after();
+            issue_pv(t, v_stage(j), true, 2 * kPFirst, kBlockN / 16);
             if (releases) tc_commit(&v_empty[v_stage(j)]);  // at once: the V ring is only two deep at head_dim 128
             if (has_next) {
-#if HDIT_ATTN_LATE_KWAIT
               if (il || t == 0) wait(&k_full[k_stage(jn)], k_phase(jn), W_MMA_KFULL, jn);
               if (!ok) break;
-#endif
               issue_qk(t, k_stage(jn));
               tc_commit(&s_full[t]);
               if (releases) tc_commit(&k_empty[k_stage(jn)]);
@@ -588,11 +524,10 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
     if (active) {
       const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
       const uint32_t tm_s = tmem_base + lane_base + C::kColS + t * 128;
-      const uint32_t tm_p = tmem_base + lane_base + C::kColP + t * C::kStrideP;
+      const uint32_t tm_p = tmem_base + lane_base + C::kColS + t * 128;
       const uint32_t tm_o = tmem_base + lane_base + C::kColO + t * D;
       const float scale_log2 = p.scale_log2;
       float m_run = -INFINITY;   // maximum the stored P and O are scaled against (log2 units)
-      float m_pend = -INFINITY;  // largest score seen so far; m_run catches up with it lazily
       float l_run = 0.f;
       bool ok = true;
       const int first = il ? t : 0;
@@ -612,39 +547,11 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
         HDIT_TRACE_SM(1);
         const int valid = min(kBlockN, p.kv_len[cur.seg] - cur.row0);
         for (int i = 0; i < blk_step; ++i) cur.advance(p);
-#if defined(HDIT_ATTN_PROBE) && (HDIT_ATTN_PROBE == 1 || HDIT_ATTN_PROBE == 3)
-        // timing probe (wrong results): no softmax work at all, only the barrier hand-shake
-        m_run = 0.f;
-        l_run = 1.f;
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&p_ready[t]);
-        continue;
-#endif
         uint32_t s[4][32];
 #pragma unroll
         for (int c = 0; c < 4; ++c) tmem_ld32(tm_s + c * 32, s[c]);
         tc_wait_ld();
         HDIT_TRACE_SM(2);
-        if constexpr (C::kSplitP) {
-          // S is in registers: the issuer may overwrite it with the next block's scores
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&s_free[t]);
-        }
-
-#if defined(HDIT_ATTN_PROBE) && HDIT_ATTN_PROBE == 2
-        // timing probe (wrong results): S is read and P written, but nothing is computed
-        m_run = 0.f;
-        l_run = 1.f;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_st16(tm_s + c * 16, s[c]);
-        tc_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&p_ready[t]);
-        continue;
-#endif
         if (valid < kBlockN) {
 #pragma unroll
           for (int c = 0; c < 4; ++c)
@@ -653,27 +560,13 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
               if (c * 32 + i >= valid) s[c][i] = 0xff800000u;  // -inf
         }
 
-        // split-P: the previous P V of this half must be done before its P is overwritten or O is rescaled. The
-        // wait sits as late as possible (before the first P store / inside the rare rescale), so that the P V
-        // runs under this block's load and maximum passes.
-        bool pv_waited = !C::kSplitP || j == 0;
-        auto wait_pv_done = [&]() {
-          if (pv_waited) return;
-          pv_waited = true;
-          if (!__all_sync(0xffffffffu, mbar_wait_bounded(&pv_done[t], (j - 1) & 1, abort_flag, kSpinLimit))) {
-            report_failure(p.status, abort_flag, HDIT_ERR_PEER_TIMEOUT, W_SM_ODONE, 100 + j * 2 + t);
-            ok = false;
-          }
-          tc_fence_after();
-        };
         // Rescale the running state to a larger maximum (rare: only when it grows by more than 2^8).
         auto rescale_to = [&](bool grow, float m_new) {
           const float alpha = grow ? ex2_approx(m_run - m_new) : 1.0f;
           if (grow) m_run = m_new;
           l_run *= alpha;
           if (j > 0) {
-            // O(t) is stable here: the commit that raised s_full covered the previous P V (split-P: wait for it)
-            wait_pv_done();
+            // O(t) is stable here: the commit that raised s_full covered the previous P V
 #pragma unroll
             for (int c = 0; c < D / 32; ++c) {
               uint32_t o[32];
@@ -685,14 +578,13 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
             }
           }
         };
-        // P = 2^(s * scale - m_run) for the whole row, stored over S as packed 16-bit pairs; returns the row sum.
-        // With track_max the row maximum of the raw scores is computed in the same pass. Packed fp32x2 FMA and
-        // add halve the issue slots; of every 8 scores the last HDIT_ATTN_POLY8 take the polynomial exp2.
-        auto exp_pass = [&](auto track_max, float& raw_max) -> float {
+        // P = 2^(s * scale - m_run) for the whole row, stored over S as packed 16-bit pairs; returns the row sum. The
+        // first part is handed over on the way. Packed fp32x2 FMA and add halve the issue slots; of every 8 scores the
+        // last kPoly8 take the polynomial exp2.
+        auto exp_pass = [&]() -> float {
           const float2 scale2 = make_float2(scale_log2, scale_log2);
           const float2 neg_m2 = make_float2(-m_run, -m_run);
           float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
-          float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             uint32_t pk[16];
@@ -700,14 +592,10 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
             for (int i = 0; i < 32; i += 4) {
               const float2 r0 = make_float2(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
               const float2 r1 = make_float2(__uint_as_float(s[c][i + 2]), __uint_as_float(s[c][i + 3]));
-              if constexpr (decltype(track_max)::value) {
-                mx0 = max3(mx0, r0.x, r0.y);
-                mx1 = max3(mx1, r1.x, r1.y);
-              }
               const float2 x0 = __ffma2_rn(r0, scale2, neg_m2);
               const float2 x1 = __ffma2_rn(r1, scale2, neg_m2);
               // position of this group of four within its group of eight decides the pipe
-              constexpr int kPolyPairs = HDIT_ATTN_POLY8 / 2;
+              constexpr int kPolyPairs = C::kPoly8 / 2;
               const bool second_half = (i & 4) != 0;
               const bool poly0 = second_half ? (kPolyPairs >= 2) : (kPolyPairs >= 4);
               const bool poly1 = second_half ? (kPolyPairs >= 1) : (kPolyPairs >= 3);
@@ -718,31 +606,18 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
               pk[i >> 1] = pack2<FP16>(p0.x, p0.y);
               pk[(i >> 1) + 1] = pack2<FP16>(p1.x, p1.y);
             }
-            if (c == 0) wait_pv_done();
             tmem_st16(tm_p + c * 16, pk);
+            if (c == kPFirst - 1) {
+              tc_wait_st();
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&p_ready[t]);
+            }
           }
-          raw_max = fmaxf(mx0, mx1);
           return (acc0.x + acc0.y) + (acc1.x + acc1.y);
         };
 
-        bool classic = (j == 0) || (HDIT_ATTN_STALE_MAX == 0);
-        if (!classic) {
-          // The maximum used for this block is the one known before it; what the previous block added to it
-          // takes effect now.
-          const bool grow = (m_pend - m_run) > kRescaleThreshold;
-          if (__any_sync(0xffffffffu, grow)) rescale_to(grow, m_pend);
-          HDIT_TRACE_SM(3);
-          float raw_max;
-          const float sum = exp_pass(std::true_type{}, raw_max);
-          const float m_blk = raw_max * scale_log2;
-          if (__any_sync(0xffffffffu, (m_blk - m_run) > kOverflowGuard)) {
-            classic = true;  // a score far above everything seen so far: redo the block against its own maximum
-          } else {
-            l_run += sum;
-            m_pend = fmaxf(m_run, m_blk);
-          }
-        }
-        if (classic) {
+        {
           float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
 #pragma unroll
           for (int c = 0; c < 4; ++c)
@@ -753,14 +628,13 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
               mx2 = max3(mx2, __uint_as_float(s[c][i + 4]), __uint_as_float(s[c][i + 5]));
               mx3 = max3(mx3, __uint_as_float(s[c][i + 6]), __uint_as_float(s[c][i + 7]));
             }
-          const float m_blk = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * scale_log2;
-          const float m_new = fmaxf(m_run, m_blk);
+          const float m_blk = max3(max3(mx0, mx1, mx2), mx3, mx3) * scale_log2;
+          const float m_new = max3(m_run, m_blk, m_blk);
           const bool grow = (m_new - m_run) > kRescaleThreshold;  // true on the first block (m_run = -inf)
           if (__any_sync(0xffffffffu, grow)) rescale_to(grow, m_new);
-          if (j == 0) HDIT_TRACE_SM(3);
-          float unused;
-          l_run += exp_pass(std::false_type{}, unused);
-          m_pend = fmaxf(m_run, m_blk);
+          l_run += m_new - m_new;  // 0, or NaN for a row with a NaN score or without a finite maximum
+          HDIT_TRACE_SM(3);
+          l_run += exp_pass();
         }
         HDIT_TRACE_SM(4);
         if (!ok) break;
@@ -768,7 +642,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
         tc_fence_before();
         // one arrival per warp: 128 arrivals on one barrier word would serialise on the S -> P -> MMA path
         __syncwarp();
-        if (lane == 0) mbar_arrive(&p_ready[t]);
+        if (lane == 0) mbar_arrive(&p_rest[t]);
         HDIT_TRACE_SM(5);
       }
 

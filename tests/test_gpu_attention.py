@@ -93,6 +93,25 @@ def test_large_score_range():
     _check(out, lse, [q], [k], [v])
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("key", [0, 5, 6, 7, 63, 64, 126, 127, 130, 199])
+def test_special_values_reach_the_output(key, D, dtype):
+    """Whatever unit exponentiates a column and whichever part of P it is in: a NaN key makes every output row of its
+    head NaN; a key so far below the others that its weight is zero (scores spread over more than 2^126) leaves the
+    rest exact; the other head is untouched."""
+    gen = torch.Generator().manual_seed(key + D)
+    q, k, v = (_mk((1, n, 2, D), dtype, gen) for n in (140, 200, 200))
+    far = k.clone()
+    q[..., 0] = 40.0
+    far[:, key, 0, 0] = -60.0
+    out, lse = _run([q], [far], [v], softmax_scale=1.0)
+    _check(out, lse, [q], [far], [v], scale=1.0)
+    k[:, key, 0, 3] = float("nan")
+    out, _ = _run([q], [k], [v])
+    assert torch.isnan(out[:, :, 0]).all() and torch.isfinite(out[:, :, 1]).all()
+
+
 @pytest.mark.parametrize("D", [64, 128])
 def test_partial_and_merge_modes(D):
     """Ring-style accumulation: PARTIAL_FIRST, PARTIAL_MERGE, MERGE_FINAL over KV blocks == one shot."""
