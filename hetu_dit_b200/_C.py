@@ -167,7 +167,55 @@ class GemmArgs(ctypes.Structure):
     ]
 
 
-GEMM_BIAS, GEMM_BIAS_GELU_TANH, GEMM_BIAS_GATE_RESIDUAL = 0, 1, 2
+GEMM_BIAS, GEMM_BIAS_GELU_TANH, GEMM_BIAS_GATE_RESIDUAL, GEMM_BIAS_NORM_ROPE = 0, 1, 2, 3
+MAX_LINEAR_ITEMS = 8
+
+
+class LinearItem(ctypes.Structure):
+    _fields_ = [
+        ("m", ctypes.c_int64),
+        ("n", ctypes.c_int64),
+        ("a", ctypes.c_void_p),
+        ("lda", ctypes.c_int64),
+        ("w", ctypes.c_void_p),
+        ("ldw", ctypes.c_int64),
+        ("bias", ctypes.c_void_p),
+        ("out", ctypes.c_void_p),
+        ("ldo", ctypes.c_int64),
+        ("residual", ctypes.c_void_p),
+        ("ldr", ctypes.c_int64),
+        ("gate", ctypes.c_void_p),
+        ("gate_batch_stride", ctypes.c_int64),
+        ("rows_per_batch", ctypes.c_int64),
+        ("epilogue", ctypes.c_int32),
+        ("head_dim", ctypes.c_int32),
+        ("norm", ctypes.c_int32),
+        ("rope", ctypes.c_int32),
+        ("norm_weight", ctypes.c_void_p),
+        ("norm_bias", ctypes.c_void_p),
+        ("rope_seq_start", ctypes.c_int64),
+        ("rope_row0", ctypes.c_int64),
+        ("eps", ctypes.c_float),
+        ("reserved0", ctypes.c_int32),
+    ]
+
+
+class LinearGroupArgs(ctypes.Structure):
+    _fields_ = [
+        ("dtype", ctypes.c_int32),
+        ("n_items", ctypes.c_int32),
+        ("k", ctypes.c_int64),
+        ("cos", ctypes.c_void_p),
+        ("sin", ctypes.c_void_p),
+        ("rope_rows", ctypes.c_int64),
+        ("stream", ctypes.c_void_p),
+        ("tile_m", ctypes.c_int32),
+        ("tile_n", ctypes.c_int32),
+        ("cta_pair", ctypes.c_int32),
+        ("max_ctas", ctypes.c_int32),
+        ("item", LinearItem * MAX_LINEAR_ITEMS),
+    ]
+
 
 _lib = None
 _lock = threading.Lock()
@@ -206,6 +254,8 @@ def _declare(lib):
                                                                                  ctypes.c_void_p]
     lib.hdit_linear_fused.restype = ctypes.c_int
     lib.hdit_linear_fused.argtypes = [ctypes.POINTER(GemmArgs)]
+    lib.hdit_linear_group.restype = ctypes.c_int
+    lib.hdit_linear_group.argtypes = [ctypes.POINTER(LinearGroupArgs)]
     lib.hdit_heap_alloc.restype = ctypes.c_int
     lib.hdit_heap_alloc.argtypes = [ctypes.c_int64, ctypes.POINTER(ctypes.c_void_p)]
     lib.hdit_heap_free.restype = ctypes.c_int

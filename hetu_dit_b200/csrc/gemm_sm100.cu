@@ -7,17 +7,26 @@
 //   warp 1      MMA issuer   : four tcgen05.mma (K = 16 each) per stage and 128-row block of the tile. The issuing
 //                              thread is picked by elect.sync, not by `lane == 0`, which costs 61 cycles of issue per
 //                              MMA (4608 x 12288 x 3072 + GELU 257 -> 241 us, 4608 x 9216 x 3072 202 -> 185 us)
-//   warps 2..   epilogue     : four warps per 128-row block. A thread reads its accumulator row from TMEM 64
+//   warps 2..   epilogue     : four warps per 128 x 128 or 128 x 256 (one CTA per 256-row tile) block, eight where a
+//                              128 x 256 block is all the CTA has. A thread reads its accumulator row from TMEM 64
 //                              columns at a time, adds the bias in fp32 and rounds to the storage type (the value
 //                              an unfused linear layer would have written); the warp transposes the 32 x 64 piece
 //                              through a swizzled 4 KB staging buffer so that eight lanes cover one 128-byte row
-//                              segment, applies the tail there -- nothing, tanh-GELU, or residual + gate * value --
-//                              and every global load and store of the tail is a full 128-byte line
+//                              segment, applies the tail there -- nothing, tanh-GELU, residual + gate * value, or
+//                              per-head norm and rotary embedding -- and every global load and store of the tail is a
+//                              full 128-byte line
+//
+// A launch takes up to eight layers ("items") of one K; their tiles form one list, so that layers with few rows (the text
+// stream beside the image stream) and layers on one input (Q, K, V) share one partly filled last wave. Measured against
+// a library GEMM and a tail kernel per layer, 4096 image + 512 text rows, hidden 3072: Q, K, V with norm and rotation 352 ->
+// 199 us, output projections + gated residual 97.5 -> 68.6, MLP up + GELU 389 -> 252, MLP down + gated residual 344 -> 261.
+//
+// The main loop runs at the tensor pipe's rate: 296.8 k cycles against 294.9 k of MMAs for 4608 x 12288 x 3072 on pairs. What
+// bounds it is the power limit, which holds the SM clock near 1.25-1.35 GHz in such loops (1465-1510 TFLOP/s).
 //
 // Tile shapes (rows x columns of the output one CTA owns at a time):
 //   128 x 256, 128 x 128  two accumulators in TMEM: the tensor pipe starts the next tile while the previous one is
-//                         written out. At full tensor rate a 128 x 256 tile asks L2 for 96 bytes per clock per SM;
-//                         measured, the MMA thread waits for operands a fifth of the time.
+//                         written out. At full tensor rate a 128 x 256 tile asks L2 for 96 bytes per clock per SM.
 //   256 x 256             fills all 512 TMEM columns with one tile (its write-out is exposed) but asks for a third
 //                         fewer operand bytes per flop.
 //   pair                  two CTAs of a cluster (an SM pair) share a 256 x 256 tile with tcgen05.mma.cta_group::2:
@@ -47,6 +56,7 @@
 #include <mutex>
 
 #include "host_common.h"
+#include "norm_rope_math.cuh"
 #include "ptx_sm100.cuh"
 
 namespace hdit {
@@ -55,9 +65,10 @@ namespace {
 constexpr int kTileK = 64;  // one 128-byte swizzle row of 16-bit elements
 constexpr uint32_t kSpinLimit = 8u * 1000u * 1000u;
 constexpr int kMaxSmem = 232448;  // 227 KiB opt-in limit per CTA
-// Relative time per 128 x 128 of output for each work-unit shape (1 = the tensor pipe never waits), from
-// measurement; used only to choose a shape.
-constexpr double kCost128x256 = 1.2, kCost128x128 = 1.75, kCost256x256 = 1.3, kCostPair = 1.05;
+// Relative time per 128 x 128 of output for each work-unit shape, from measurement; used only to choose a shape. 256 x 256
+// pair : 128 x 256 : 128 x 128, us per wave: 10.6 : 11.8 : 6.8 per (2 : 2 : 1) blocks at K = 1536, 20.8 : 25 : 15.5 at 12464
+// rows and K = 3072, 30 : 31 : 15.2 at 1280 rows, where the clock is not held down.
+constexpr double kCost128x256 = 1.18, kCost128x128 = 1.25, kCost256x256 = 1.3, kCostPair = 1.05;
 
 #ifdef HDIT_GEMM_TRACE
 // per CTA: MMA thread {total, waiting for operands, waiting for a free accumulator, tiles}, epilogue warp 2
@@ -77,7 +88,11 @@ struct GemmCfg {
   static_assert(!PAIR || (BM == 128 && BN == 256), "a CTA of a pair owns 128 x 256 of the pair's 256 x 256 tile");
   static constexpr int kHalves = BM / 128;                 // 128-row MMA blocks per CTA tile
   static constexpr int kAccBufs = (kHalves == 1) ? 2 : 1;  // accumulator tiles resident in TMEM
-  static constexpr int kEpiWarps = 4 * kHalves;
+  // Four warps reach all 128 lanes of an accumulator block; a 256-column accumulator has two such teams, each with half
+  // of the columns. With one team the norm + rotation tail took 28.6 k cycles per 128 x 256 accumulator, longer than the
+  // 24.6 k of the main loop at K = 3072 that it hides behind.
+  static constexpr int kColTeams = (kHalves == 1 && BN == 256) ? 2 : 1;
+  static constexpr int kEpiWarps = 4 * kHalves * kColTeams;
   static constexpr int kThreads = 64 + 32 * kEpiWarps;
   static constexpr int kTileRows = PAIR ? 2 * BM : BM;     // rows of the scheduling unit's tile
   static constexpr int kBRows = PAIR ? BN / 2 : BN;        // rows of W this CTA loads per stage
@@ -94,11 +109,12 @@ struct GemmCfg {
   static_assert(kStages >= 3, "ring too short");
 };
 
-struct GemmParams {
+// One linear layer of a launch. Items share K; their output tiles are numbered one after the other from tile0 on.
+struct alignas(64) GemmItem {
   CUtensorMap a_map;
   CUtensorMap w_map;
-  int M, N, K;
-  int m_tiles, n_tiles, k_blocks;
+  int M, N;
+  int m_tiles, n_tiles, tile0;
   int group_m;  // tiles are walked in bands of group_m tile rows, so that a wave of CTAs covers a near-square region
   int epilogue;
   int rows_per_batch;
@@ -109,12 +125,32 @@ struct GemmParams {
   long long ldr;
   const uint16_t* gate;
   long long gate_batch_stride;
+  // HDIT_GEMM_BIAS_NORM_ROPE
+  const uint16_t* norm_weight;
+  const uint16_t* norm_bias;
+  int head_dim, norm, rope;
+  float eps;
+  int rope_seq_start, rope_row0;
+};
+
+struct GemmParams {
+  GemmItem item[HDIT_MAX_LINEAR_ITEMS];
+  int n_items, k_blocks, total_tiles;
+  const float* cos_tab;
+  const float* sin_tab;
   int32_t* status;
 };
 
+__device__ __forceinline__ int item_of(const GemmParams& p, int tile) {
+  int i = 0;
+  while (i + 1 < p.n_items && tile >= p.item[i + 1].tile0) ++i;
+  return i;
+}
+
 // Tile index -> (tile row, tile column): bands of group_m tile rows, column-major inside a band. CTAs that run
 // at the same time then share both a few A row blocks and a few W row blocks in L2, instead of one W block and all of A.
-__device__ __forceinline__ void tile_coords(const GemmParams& p, int tile, int& m_t, int& n_t) {
+__device__ __forceinline__ void tile_coords(const GemmItem& p, int tile, int& m_t, int& n_t) {
+  tile -= p.tile0;
   const int per_band = p.group_m * p.n_tiles;
   const int band = tile / per_band, r = tile - band * per_band;
   const int m0 = band * p.group_m;
@@ -217,6 +253,116 @@ __device__ __forceinline__ float gelu_tanh_f(float x) {
   return 0.5f * x * (1.0f + t);
 }
 
+// {mean, 1 / deviation} of this thread's row over the head whose accumulator columns start at `taddr`, from the values
+// rounded to the storage type as the linear layer writes them. Sums run in the order of norm_rope_kernel (eight columns in
+// a row, then pairs of partial sums), so both give the same bits. The columns are read from TMEM once more for it: a
+// second read costs less than keeping 128 columns in registers until the row is complete.
+template <bool FP16>
+__device__ __forceinline__ float2 head_stats(const GemmItem& p, uint32_t taddr, int col0) {
+  float part[16];
+  float mean = 0.f;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) part[i] = 0.f;
+#pragma unroll
+  for (int pc = 0; pc < 2; ++pc) {
+    if (pc * 64 >= p.head_dim) break;
+    uint32_t r[64];
+    tmem_ld32(taddr + pc * 64, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+    tmem_ld32(taddr + pc * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
+    tc_wait_ld();
+    float sum[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      uint4 bv = make_uint4(0, 0, 0, 0);
+      const int col = col0 + pc * 64 + j * 8;
+      if (p.bias != nullptr && col < p.N) bv = __ldg(reinterpret_cast<const uint4*>(p.bias + col));
+      float be[8];
+      nr_unpack8<FP16>(bv, be);
+      sum[j] = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; k += 2) {
+        float lo, hi;
+        nr_unpack<FP16>(nr_pack<FP16>(__uint_as_float(r[j * 8 + k]) + be[k], __uint_as_float(r[j * 8 + k + 1]) + be[k + 1]), lo, hi);
+        r[j * 8 + k] = __float_as_uint(lo);
+        r[j * 8 + k + 1] = __float_as_uint(hi);
+        sum[j] += lo;
+        sum[j] += hi;
+      }
+    }
+    if (p.norm == 2) {  // head_dim 64: the head is complete
+      const float total = ((sum[0] + sum[4]) + (sum[2] + sum[6])) + ((sum[1] + sum[5]) + (sum[3] + sum[7]));
+      mean = total * (1.0f / 64);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float d = __uint_as_float(r[j * 8 + k]) - mean;
+        part[pc * 8 + j] = fmaf(d, d, part[pc * 8 + j]);
+      }
+  }
+  float ss;
+  if (p.head_dim == 128) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) part[i] += part[i + 8];
+  }
+  ss = ((part[0] + part[4]) + (part[2] + part[6])) + ((part[1] + part[5]) + (part[3] + part[7]));
+  return make_float2(mean, rsqrtf(ss * (p.head_dim == 128 ? 1.0f / 128 : 1.0f / 64) + p.eps));
+}
+
+// Norm and rotary embedding of a staged 32 x 64 piece, eight columns of one row per lane and pass; the whole warp takes
+// part (n is a multiple of 64 here, so a piece lies inside or outside as a whole). Four rows' table entries are requested
+// before the first is used.
+template <bool FP16>
+__device__ __forceinline__ void norm_rope_rows(const GemmItem& p, const float* __restrict__ cos_tab,
+                                               const float* __restrict__ sin_tab, const uint8_t* staging, float2 stats,
+                                               long long row0, long long batch0, long long next_batch_row, int col) {
+  const int lane = threadIdx.x & 31;
+  const int sub_row = lane >> 3, chunk = lane & 7;
+  const int hcol = col & (p.head_dim - 1);
+  uint4 w = make_uint4(0, 0, 0, 0), bi = make_uint4(0, 0, 0, 0);
+  if (p.norm != 0 && p.norm_weight != nullptr) w = __ldg(reinterpret_cast<const uint4*>(p.norm_weight + hcol));
+  if (p.norm == 2 && p.norm_bias != nullptr) bi = __ldg(reinterpret_cast<const uint4*>(p.norm_bias + hcol));
+#pragma unroll 1
+  for (int g = 0; g < 2; ++g) {
+    float4 c0[4], c1[4], s0[4], s1[4];
+    bool rot[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const long long row = row0 + (g * 4 + i) * 4 + sub_row;
+      const long long s = row - (row >= next_batch_row ? next_batch_row : batch0 * p.rows_per_batch);
+      rot[i] = p.rope != 0 && row < p.M && s >= p.rope_seq_start;
+      if (rot[i]) {
+        const long long at = (s - p.rope_seq_start + p.rope_row0) * p.head_dim + hcol;
+        c0[i] = __ldg(reinterpret_cast<const float4*>(cos_tab + at));
+        c1[i] = __ldg(reinterpret_cast<const float4*>(cos_tab + at + 4));
+        s0[i] = __ldg(reinterpret_cast<const float4*>(sin_tab + at));
+        s1[i] = __ldg(reinterpret_cast<const float4*>(sin_tab + at + 4));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int rl = (g * 4 + i) * 4 + sub_row;
+      const long long row = row0 + rl;
+      const float mean = __shfl_sync(0xffffffffu, stats.x, rl), rstd = __shfl_sync(0xffffffffu, stats.y, rl);
+      uint4 v = *reinterpret_cast<const uint4*>(staging + rl * 128 + ((chunk ^ (rl & 7)) << 4));
+      if (p.norm != 0) {
+        float f[8];
+        nr_unpack8<FP16>(v, f);
+        if (p.norm == 2) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) f[k] -= mean;
+          v = nr_layer8<FP16>(f, rstd, p.norm_weight != nullptr, w, p.norm_bias != nullptr, bi);
+        } else {
+          v = nr_rms8<FP16>(f, rstd, p.norm_weight != nullptr, w);
+        }
+      }
+      if (rot[i]) v = nr_rotate8<FP16>(v, c0[i], c1[i], s0[i], s1[i]);
+      if (row < p.M) *reinterpret_cast<uint4*>(p.out + row * p.ldo + col) = v;
+    }
+  }
+}
+
 template <int BM, int BN, bool PAIR, bool FP16>
 __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
     linear_fused_kernel(const __grid_constant__ GemmParams p) {
@@ -241,8 +387,10 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
   const int n_units = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
   if (threadIdx.x == 0) {
-    tma_prefetch_desc(&p.a_map);
-    tma_prefetch_desc(&p.w_map);
+    for (int i = 0; i < p.n_items; ++i) {
+      tma_prefetch_desc(&p.item[i].a_map);
+      tma_prefetch_desc(&p.item[i].w_map);
+    }
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(&full[s], 1);  // pair: only the even CTA's is used; both CTAs' copies complete on it
       mbar_init(&empty[s], 1);
@@ -271,7 +419,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  const int total_tiles = p.m_tiles * p.n_tiles;
+  const int total_tiles = p.total_tiles;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -280,7 +428,8 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
       bool ok = true;
       for (int tile = unit; tile < total_tiles && ok; tile += n_units) {
         int m_t, n_t;
-        tile_coords(p, tile, m_t, n_t);
+        const GemmItem& im = p.item[item_of(p, tile)];
+        tile_coords(im, tile, m_t, n_t);
         const int a_row = m_t * C::kTileRows + static_cast<int>(rank) * BM;
         const int w_row = n_t * BN + static_cast<int>(rank) * C::kBRows;
         for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
@@ -296,12 +445,12 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
             // even CTA's MMAs of the previous round have released the stage, i.e. never into an earlier phase.
             if (leader) mbar_expect_tx(&full[s], 2 * C::kStageBytes);
             const uint32_t bar = map_to_cta(&full[s], 0);
-            tma_load_2d_pair(a_dst, &p.a_map, bar, kb * kTileK, a_row);
-            tma_load_2d_pair(a_dst + C::kABytes, &p.w_map, bar, kb * kTileK, w_row);
+            tma_load_2d_pair(a_dst, &im.a_map, bar, kb * kTileK, a_row);
+            tma_load_2d_pair(a_dst + C::kABytes, &im.w_map, bar, kb * kTileK, w_row);
           } else {
             mbar_expect_tx(&full[s], C::kStageBytes);
-            tma_load_2d(a_dst, &p.a_map, &full[s], kb * kTileK, a_row);
-            tma_load_2d(a_dst + C::kABytes, &p.w_map, &full[s], kb * kTileK, w_row);
+            tma_load_2d(a_dst, &im.a_map, &full[s], kb * kTileK, a_row);
+            tma_load_2d(a_dst + C::kABytes, &im.w_map, &full[s], kb * kTileK, w_row);
           }
         }
       }
@@ -398,7 +547,10 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
   } else {
     // ------------------------------------------------------------------ epilogue
     const int quarter = warp & 3;  // the TMEM lanes this warp may read: [32 * quarter, 32 * quarter + 32)
-    const int half = (warp - 2) >> 2;  // which 128-row block of the tile
+    const int team = (warp - 2) >> 2;
+    const int half = C::kColTeams == 1 ? team : 0;  // which 128-row block of the tile
+    constexpr int kPieces = BN / 64 / C::kColTeams;   // 64-column pieces of this warp
+    const int c0 = C::kColTeams == 1 ? 0 : team * kPieces;
     uint8_t* staging = staging_base + (warp - 2) * 4096;
     const int sub_row = lane >> 3, chunk = lane & 7;  // store phase: 4 rows per instruction, 8 lanes per row
     uint32_t local = 0;
@@ -408,7 +560,8 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
 #endif
     for (int tile = unit; tile < total_tiles && ok; tile += n_units, ++local) {
       int m_t, n_t;
-        tile_coords(p, tile, m_t, n_t);
+      const GemmItem& im = p.item[item_of(p, tile)];
+      tile_coords(im, tile, m_t, n_t);
       const uint32_t acc = local % C::kAccBufs, use = local / C::kAccBufs;
       if (!__all_sync(0xffffffffu, mbar_wait_bounded(&acc_full[acc], use & 1, abort_flag, kSpinLimit))) {
         if (lane == 0) report_failure(p.status, abort_flag, HDIT_ERR_PEER_TIMEOUT, G_EPI_ACC_FULL, static_cast<int>(local));
@@ -423,18 +576,21 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
       const long long row0 = static_cast<long long>(m_t) * C::kTileRows + static_cast<long long>(rank) * BM + half * 128 +
                              quarter * 32;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + (acc * C::kHalves + half) * BN;
-      long long batch0 = 0, next_batch_row = p.M;
-      if (p.epilogue == HDIT_GEMM_BIAS_GATE_RESIDUAL && row0 < p.M) {
-        batch0 = static_cast<long long>(static_cast<unsigned>(row0) / static_cast<unsigned>(p.rows_per_batch));
-        next_batch_row = (batch0 + 1) * p.rows_per_batch;
+      long long batch0 = 0, next_batch_row = im.M;
+      if (im.epilogue >= HDIT_GEMM_BIAS_GATE_RESIDUAL && row0 < im.M) {
+        batch0 = static_cast<long long>(static_cast<unsigned>(row0) / static_cast<unsigned>(im.rows_per_batch));
+        next_batch_row = (batch0 + 1) * im.rows_per_batch;
       }
+      float2 stats = make_float2(0.f, 0.f);
 #pragma unroll 1
-      for (int c = 0; c < BN / 64; ++c) {
+      for (int c = c0; c < c0 + kPieces; ++c) {
+        if (im.epilogue == HDIT_GEMM_BIAS_NORM_ROPE && im.norm != 0 && ((c * 64) & (im.head_dim - 1)) == 0)
+          stats = head_stats<FP16>(im, taddr + c * 64, n_t * BN + c * 64);
         uint32_t r[64];
         tmem_ld32(taddr + c * 64, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
         tmem_ld32(taddr + c * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
         tc_wait_ld();
-        if (c == BN / 64 - 1) {
+        if (c == c0 + kPieces - 1) {
           // the accumulator is in registers: hand it back to the MMA warp before the rest of the last piece
           tc_fence_before();
           __syncwarp();
@@ -451,7 +607,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           uint4 bv = make_uint4(0, 0, 0, 0);
-          if (p.bias != nullptr && col0 + j * 8 < p.N) bv = __ldg(reinterpret_cast<const uint4*>(p.bias + col0 + j * 8));
+          if (im.bias != nullptr && col0 + j * 8 < im.N) bv = __ldg(reinterpret_cast<const uint4*>(im.bias + col0 + j * 8));
           const uint16_t* be = reinterpret_cast<const uint16_t*>(&bv);
           uint4 v;
           v.x = pack2<FP16>(__uint_as_float(r[j * 8 + 0]) + to_f<FP16>(be[0]), __uint_as_float(r[j * 8 + 1]) + to_f<FP16>(be[1]));
@@ -463,24 +619,26 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
         __syncwarp();
         // phase 2: eight lanes per row, 128 contiguous bytes; the tail runs here
         const int col = col0 + chunk * 8;
-        if (col < p.N) {
-          if (p.epilogue == HDIT_GEMM_BIAS_GATE_RESIDUAL) {
+        if (im.epilogue == HDIT_GEMM_BIAS_NORM_ROPE) {
+          if (col0 < im.N) norm_rope_rows<FP16>(im, p.cos_tab, p.sin_tab, staging, stats, row0, batch0, next_batch_row, col);
+        } else if (col < im.N) {
+          if (im.epilogue == HDIT_GEMM_BIAS_GATE_RESIDUAL) {
             uint4 xv[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const long long row = row0 + i * 4 + sub_row;
-              xv[i] = (row < p.M) ? *reinterpret_cast<const uint4*>(p.residual + row * p.ldr + col) : make_uint4(0, 0, 0, 0);
+              xv[i] = (row < im.M) ? *reinterpret_cast<const uint4*>(im.residual + row * im.ldr + col) : make_uint4(0, 0, 0, 0);
             }
             // the 32 rows of this warp lie in at most two batch entries
-            const uint4 g_lo = __ldg(reinterpret_cast<const uint4*>(p.gate + batch0 * p.gate_batch_stride + col));
-            const uint4 g_hi = (row0 + 31 >= next_batch_row && next_batch_row < p.M)
-                                   ? __ldg(reinterpret_cast<const uint4*>(p.gate + (batch0 + 1) * p.gate_batch_stride + col))
+            const uint4 g_lo = __ldg(reinterpret_cast<const uint4*>(im.gate + batch0 * im.gate_batch_stride + col));
+            const uint4 g_hi = (row0 + 31 >= next_batch_row && next_batch_row < im.M)
+                                   ? __ldg(reinterpret_cast<const uint4*>(im.gate + (batch0 + 1) * im.gate_batch_stride + col))
                                    : g_lo;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const int rl = i * 4 + sub_row;
               const long long row = row0 + rl;
-              if (row >= p.M) continue;
+              if (row >= im.M) continue;
               uint4 v = *reinterpret_cast<const uint4*>(staging + rl * 128 + ((chunk ^ (rl & 7)) << 4));
               const uint4 gv = row >= next_batch_row ? g_hi : g_lo;
               const uint16_t* xe = reinterpret_cast<const uint16_t*>(&xv[i]);
@@ -489,21 +647,21 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
 #pragma unroll
               for (int k = 0; k < 8; ++k)
                 ve[k] = from_f<FP16>(fmaf(to_f<FP16>(ge[k]), to_f<FP16>(ve[k]), to_f<FP16>(xe[k])));
-              *reinterpret_cast<uint4*>(p.out + row * p.ldo + col) = v;
+              *reinterpret_cast<uint4*>(im.out + row * im.ldo + col) = v;
             }
           } else {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const int rl = i * 4 + sub_row;
               const long long row = row0 + rl;
-              if (row >= p.M) continue;
+              if (row >= im.M) continue;
               uint4 v = *reinterpret_cast<const uint4*>(staging + rl * 128 + ((chunk ^ (rl & 7)) << 4));
-              if (p.epilogue == HDIT_GEMM_BIAS_GELU_TANH) {
+              if (im.epilogue == HDIT_GEMM_BIAS_GELU_TANH) {
                 uint16_t* ve = reinterpret_cast<uint16_t*>(&v);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) ve[k] = from_f<FP16>(gelu_tanh_f(to_f<FP16>(ve[k])));
               }
-              *reinterpret_cast<uint4*>(p.out + row * p.ldo + col) = v;
+              *reinterpret_cast<uint4*>(im.out + row * im.ldo + col) = v;
             }
           }
         }
@@ -582,33 +740,40 @@ int sm_count() {
 }
 
 template <int BM, int BN, bool PAIR, bool FP16>
-int launch_gemm(GemmParams& kp, const hdit_gemm_args* a, cudaStream_t stream) {
+int launch_gemm(GemmParams& kp, const hdit_linear_group_args* a) {
   using C = GemmCfg<BM, BN, PAIR>;
   auto kernel = linear_fused_kernel<BM, BN, PAIR, FP16>;
-  static int last_dev = -1;
+  // The attribute is per device: set it whenever this thread meets a new device.
+  static thread_local int last_dev = -1;
   int dev = 0;
   HDIT_CUDA_OK(cudaGetDevice(&dev));
   if (dev != last_dev) {
     HDIT_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
     last_dev = dev;
   }
-  int rc = encode_matrix(&kp.a_map, a->a, a->m, a->k, a->lda, BM, a->dtype);
-  if (rc != HDIT_OK) return rc;
-  rc = encode_matrix(&kp.w_map, a->w, a->n, a->k, a->ldw, C::kBRows, a->dtype);
-  if (rc != HDIT_OK) return rc;
-  kp.m_tiles = static_cast<int>((a->m + C::kTileRows - 1) / C::kTileRows);
-  kp.n_tiles = static_cast<int>((a->n + BN - 1) / BN);
-  const long long tiles = static_cast<long long>(kp.m_tiles) * kp.n_tiles;
-  if (tiles > 0x7fffffffLL) return set_error(HDIT_ERR_TOO_LARGE, "more than 2^31 output tiles");
   long long ctas = a->max_ctas > 0 ? a->max_ctas : sm_count();
-  {
+  long long tiles = 0;
+  for (int i = 0; i < kp.n_items; ++i) {
+    GemmItem& im = kp.item[i];
+    const hdit_linear_item& h = a->item[i];
+    int rc = encode_matrix(&im.a_map, h.a, h.m, a->k, h.lda, BM, a->dtype);
+    if (rc != HDIT_OK) return rc;
+    rc = encode_matrix(&im.w_map, h.w, h.n, a->k, h.ldw, C::kBRows, a->dtype);
+    if (rc != HDIT_OK) return rc;
+    im.m_tiles = static_cast<int>((h.m + C::kTileRows - 1) / C::kTileRows);
+    im.n_tiles = static_cast<int>((h.n + BN - 1) / BN);
+    im.tile0 = static_cast<int>(tiles);
+    tiles += static_cast<long long>(im.m_tiles) * im.n_tiles;
+    if (tiles > 0x7fffffffLL) return set_error(HDIT_ERR_TOO_LARGE, "more than 2^31 output tiles");
     // band height: a wave of `units` tiles should read about as many A bytes as W bytes
     const double units = static_cast<double>(PAIR ? (ctas / 2 > 0 ? ctas / 2 : 1) : ctas);
     int g = static_cast<int>(sqrt(units * BN / C::kTileRows) + 0.5);
     if (g < 1) g = 1;
-    if (g > kp.m_tiles) g = kp.m_tiles;
-    kp.group_m = g;
+    if (g > im.m_tiles) g = im.m_tiles;
+    im.group_m = g;
   }
+  kp.total_tiles = static_cast<int>(tiles);
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(a->stream);
   if (PAIR) {
     long long pairs = ctas / 2 > 0 ? ctas / 2 : 1;
     if (pairs > tiles) pairs = tiles;
@@ -633,6 +798,69 @@ int launch_gemm(GemmParams& kp, const hdit_gemm_args* a, cudaStream_t stream) {
   return HDIT_OK;
 }
 
+// Checks one item and fills the kernel's form of it (all but the tensor maps and tile counts).
+int fill_item(GemmItem* im, const hdit_linear_item& a, const hdit_linear_group_args& g) {
+  if (a.epilogue < HDIT_GEMM_BIAS || a.epilogue > HDIT_GEMM_BIAS_NORM_ROPE)
+    return set_error(HDIT_ERR_BAD_ARG, "unknown epilogue %d", a.epilogue);
+  if (a.m > 0x7fffffffLL || a.n > 0x7fffffffLL || g.k > 0x7fffffffLL)
+    return set_error(HDIT_ERR_TOO_LARGE, "m, n, k must fit 31 bits");
+  if (a.a == nullptr || a.w == nullptr || a.out == nullptr) return set_error(HDIT_ERR_BAD_ARG, "null a / w / out");
+  if (a.n % 8 != 0 || g.k % 8 != 0) return set_error(HDIT_ERR_SHAPE, "n and k must be multiples of 8");
+  auto bad = [](const void* ptr, long long ld) { return (reinterpret_cast<uintptr_t>(ptr) & 15) != 0 || ld % 8 != 0; };
+  if (bad(a.a, a.lda) || bad(a.w, a.ldw) || bad(a.out, a.ldo) || a.lda < g.k || a.ldw < g.k || a.ldo < a.n)
+    return set_error(HDIT_ERR_SHAPE, "a / w / out need 16-byte aligned pointers and row strides that are multiples of 8 "
+                                     "and cover a row");
+  if (a.bias != nullptr && (reinterpret_cast<uintptr_t>(a.bias) & 15) != 0)
+    return set_error(HDIT_ERR_SHAPE, "bias pointer not 16-byte aligned");
+  const bool gated = a.epilogue == HDIT_GEMM_BIAS_GATE_RESIDUAL, normed = a.epilogue == HDIT_GEMM_BIAS_NORM_ROPE;
+  if (gated && (a.residual == nullptr || a.gate == nullptr || a.rows_per_batch <= 0))
+    return set_error(HDIT_ERR_BAD_ARG, "the gated-residual epilogue needs residual, gate and rows_per_batch > 0");
+  if ((gated || (normed && a.rope != 0)) && a.rows_per_batch < 32 && a.rows_per_batch < a.m)
+    return set_error(HDIT_ERR_SHAPE, "the gated-residual and rotary epilogues need at least 32 rows per batch entry "
+                                     "(a warp's 32 rows may span two entries, not more)");
+  if (gated && (bad(a.residual, a.ldr) || bad(a.gate, a.gate_batch_stride) || a.ldr < a.n))
+    return set_error(HDIT_ERR_SHAPE, "residual / gate need 16-byte aligned pointers and strides that are multiples of 8");
+  if (normed) {
+    if (a.head_dim != 64 && a.head_dim != 128) return set_error(HDIT_ERR_SHAPE, "head_dim must be 64 or 128");
+    if (a.n % a.head_dim != 0) return set_error(HDIT_ERR_SHAPE, "n must be a multiple of head_dim");
+    if (a.norm < 0 || a.norm > 2) return set_error(HDIT_ERR_BAD_ARG, "norm must be 0, 1 or 2");
+    if (a.norm == 2 && a.head_dim != 64) return set_error(HDIT_ERR_SHAPE, "the LayerNorm epilogue takes head_dim 64");
+    if (((reinterpret_cast<uintptr_t>(a.norm_weight) | reinterpret_cast<uintptr_t>(a.norm_bias)) & 15) != 0)
+      return set_error(HDIT_ERR_SHAPE, "norm weight / bias must be 16-byte aligned");
+    if (a.rope != 0) {
+      if (g.cos == nullptr || g.sin == nullptr) return set_error(HDIT_ERR_BAD_ARG, "rope requested without cos/sin tables");
+      if (((reinterpret_cast<uintptr_t>(g.cos) | reinterpret_cast<uintptr_t>(g.sin)) & 15) != 0)
+        return set_error(HDIT_ERR_SHAPE, "cos/sin tables must be 16-byte aligned");
+      const long long seq = a.rows_per_batch < a.m ? a.rows_per_batch : a.m;
+      if (a.rows_per_batch <= 0) return set_error(HDIT_ERR_BAD_ARG, "the rotary epilogue needs rows_per_batch > 0");
+      if (a.rope_seq_start < 0 || a.rope_row0 < 0 || a.rope_seq_start > 0x7fffffffLL || a.rope_row0 > 0x7fffffffLL ||
+          (seq > a.rope_seq_start && a.rope_row0 + (seq - a.rope_seq_start) > g.rope_rows))
+        return set_error(HDIT_ERR_SHAPE, "rope table of %lld rows does not cover rows [%lld, %lld)",
+                         (long long)g.rope_rows, (long long)a.rope_seq_start, seq);
+    }
+  }
+  im->M = static_cast<int>(a.m);
+  im->N = static_cast<int>(a.n);
+  im->epilogue = a.epilogue;
+  im->rows_per_batch = static_cast<int>(a.rows_per_batch > 0x7fffffffLL ? 0x7fffffffLL : (a.rows_per_batch > 0 ? a.rows_per_batch : 0x7fffffffLL));
+  im->bias = static_cast<const uint16_t*>(a.bias);
+  im->out = static_cast<uint16_t*>(a.out);
+  im->ldo = a.ldo;
+  im->residual = static_cast<const uint16_t*>(a.residual);
+  im->ldr = a.ldr;
+  im->gate = static_cast<const uint16_t*>(a.gate);
+  im->gate_batch_stride = a.gate_batch_stride;
+  im->norm_weight = static_cast<const uint16_t*>(a.norm_weight);
+  im->norm_bias = static_cast<const uint16_t*>(a.norm_bias);
+  im->head_dim = normed ? a.head_dim : 64;
+  im->norm = normed ? a.norm : 0;
+  im->rope = normed ? a.rope : 0;
+  im->eps = a.eps;
+  im->rope_seq_start = static_cast<int>(a.rope_seq_start);
+  im->rope_row0 = static_cast<int>(a.rope_row0);
+  return HDIT_OK;
+}
+
 }  // namespace
 }  // namespace hdit
 
@@ -645,57 +873,36 @@ extern "C" HDIT_API int hdit_gemm_trace_read(long long* out) {
 }
 #endif
 
-extern "C" int hdit_linear_fused(const hdit_gemm_args* a) {
+extern "C" int hdit_linear_group(const hdit_linear_group_args* a) {
   using namespace hdit;
   if (a == nullptr) return set_error(HDIT_ERR_BAD_ARG, "null args");
   if (a->dtype != HDIT_BF16 && a->dtype != HDIT_FP16) return set_error(HDIT_ERR_BAD_ARG, "dtype must be bf16 or fp16");
-  if (a->epilogue < HDIT_GEMM_BIAS || a->epilogue > HDIT_GEMM_BIAS_GATE_RESIDUAL)
-    return set_error(HDIT_ERR_BAD_ARG, "unknown epilogue %d", a->epilogue);
-  if (a->m < 0 || a->n <= 0 || a->k <= 0) return set_error(HDIT_ERR_BAD_ARG, "bad m / n / k");
-  if (a->m == 0) return HDIT_OK;
-  if (a->m > 0x7fffffffLL || a->n > 0x7fffffffLL || a->k > 0x7fffffffLL)
-    return set_error(HDIT_ERR_TOO_LARGE, "m, n, k must fit 31 bits");
-  if (a->a == nullptr || a->w == nullptr || a->out == nullptr) return set_error(HDIT_ERR_BAD_ARG, "null a / w / out");
-  if (a->n % 8 != 0 || a->k % 8 != 0) return set_error(HDIT_ERR_SHAPE, "n and k must be multiples of 8");
-  auto bad = [](const void* ptr, long long ld) { return (reinterpret_cast<uintptr_t>(ptr) & 15) != 0 || ld % 8 != 0; };
-  if (bad(a->a, a->lda) || bad(a->w, a->ldw) || bad(a->out, a->ldo) || a->lda < a->k || a->ldw < a->k || a->ldo < a->n)
-    return set_error(HDIT_ERR_SHAPE, "a / w / out need 16-byte aligned pointers and row strides that are multiples of 8 "
-                                     "and cover a row");
-  if (a->bias != nullptr && (reinterpret_cast<uintptr_t>(a->bias) & 15) != 0)
-    return set_error(HDIT_ERR_SHAPE, "bias pointer not 16-byte aligned");
-  if (a->epilogue == HDIT_GEMM_BIAS_GATE_RESIDUAL) {
-    if (a->residual == nullptr || a->gate == nullptr || a->rows_per_batch <= 0)
-      return set_error(HDIT_ERR_BAD_ARG, "the gated-residual epilogue needs residual, gate and rows_per_batch > 0");
-    if (a->rows_per_batch < 32 && a->rows_per_batch < a->m)
-      return set_error(HDIT_ERR_SHAPE, "the gated-residual epilogue needs at least 32 rows per batch entry "
-                                       "(a warp's 32 rows may span two entries, not more)");
-    if (bad(a->residual, a->ldr) || bad(a->gate, a->gate_batch_stride) || a->ldr < a->n)
-      return set_error(HDIT_ERR_SHAPE, "residual / gate need 16-byte aligned pointers and strides that are multiples of 8");
+  if (a->n_items < 1 || a->n_items > HDIT_MAX_LINEAR_ITEMS)
+    return set_error(HDIT_ERR_BAD_ARG, "n_items must be 1..%d", HDIT_MAX_LINEAR_ITEMS);
+  GemmParams kp;
+  memset(&kp, 0, sizeof(kp));
+  // items without rows are dropped: the kernel never sees an empty tile list
+  hdit_linear_group_args live = *a;
+  live.n_items = 0;
+  for (int i = 0; i < a->n_items; ++i) {
+    const hdit_linear_item& im = a->item[i];
+    if (im.m < 0 || im.n <= 0 || a->k <= 0) return set_error(HDIT_ERR_BAD_ARG, "bad m / n / k");
+    if (im.m == 0) continue;
+    const int rc = fill_item(&kp.item[live.n_items], im, *a);
+    if (rc != HDIT_OK) return rc;
+    live.item[live.n_items++] = im;
   }
+  if (live.n_items == 0) return HDIT_OK;
   if (a->tile_n != 0 && a->tile_n != 128 && a->tile_n != 256) return set_error(HDIT_ERR_BAD_ARG, "tile_n must be 0, 128 or 256");
   if (a->tile_m != 0 && a->tile_m != 128 && a->tile_m != 256) return set_error(HDIT_ERR_BAD_ARG, "tile_m must be 0, 128 or 256");
   if (a->tile_m == 256 && a->tile_n == 128) return set_error(HDIT_ERR_BAD_ARG, "256-row tiles are 256 columns wide");
   if (a->cta_pair < 0 || a->cta_pair > 2) return set_error(HDIT_ERR_BAD_ARG, "cta_pair must be 0 (choose), 1 (never) or 2 (always)");
   if (a->cta_pair == 2 && (a->tile_m == 128 || a->tile_n == 128))
     return set_error(HDIT_ERR_BAD_ARG, "a CTA pair works on 256 x 256 tiles");
-
-  GemmParams kp;
-  kp.M = static_cast<int>(a->m);
-  kp.N = static_cast<int>(a->n);
-  kp.K = static_cast<int>(a->k);
-  kp.m_tiles = 0;
-  kp.n_tiles = 0;
-  kp.group_m = 1;
+  kp.n_items = live.n_items;
   kp.k_blocks = static_cast<int>((a->k + kTileK - 1) / kTileK);
-  kp.epilogue = a->epilogue;
-  kp.rows_per_batch = static_cast<int>(a->rows_per_batch > 0x7fffffffLL ? 0x7fffffffLL : (a->rows_per_batch > 0 ? a->rows_per_batch : 1));
-  kp.bias = static_cast<const uint16_t*>(a->bias);
-  kp.out = static_cast<uint16_t*>(a->out);
-  kp.ldo = a->ldo;
-  kp.residual = static_cast<const uint16_t*>(a->residual);
-  kp.ldr = a->ldr;
-  kp.gate = static_cast<const uint16_t*>(a->gate);
-  kp.gate_batch_stride = a->gate_batch_stride;
+  kp.cos_tab = a->cos;
+  kp.sin_tab = a->sin;
   kp.status = device_status_ptr();
   if (kp.status == nullptr) return HDIT_ERR_CUDA;
 
@@ -723,17 +930,52 @@ extern "C" int hdit_linear_fused(const hdit_gemm_args* a) {
       if (c.shape == 3 && a->cta_pair == 1) continue;
       if (c.shape == 2 && a->tile_m != 256) continue;  // one CTA per 256 x 256 tile only on request
       const long long units = sms / c.units_div > 0 ? sms / c.units_div : 1;
-      const long long tiles = ((a->m + c.rows - 1) / c.rows) * ((a->n + c.cols - 1) / c.cols);
+      long long tiles = 0;
+      for (int i = 0; i < live.n_items; ++i)
+        tiles += ((live.item[i].m + c.rows - 1) / c.rows) * ((live.item[i].n + c.cols - 1) / c.cols);
       const double cost = static_cast<double>((tiles + units - 1) / units) * c.per_tile;
       if (best < 0 || cost < best) best = cost, shape = c.shape;
     }
   }
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(a->stream);
   const bool fp16 = a->dtype == HDIT_FP16;
   switch (shape) {
-    case 3: return fp16 ? launch_gemm<128, 256, true, true>(kp, a, stream) : launch_gemm<128, 256, true, false>(kp, a, stream);
-    case 2: return fp16 ? launch_gemm<256, 256, false, true>(kp, a, stream) : launch_gemm<256, 256, false, false>(kp, a, stream);
-    case 1: return fp16 ? launch_gemm<128, 128, false, true>(kp, a, stream) : launch_gemm<128, 128, false, false>(kp, a, stream);
-    default: return fp16 ? launch_gemm<128, 256, false, true>(kp, a, stream) : launch_gemm<128, 256, false, false>(kp, a, stream);
+    case 3: return fp16 ? launch_gemm<128, 256, true, true>(kp, &live) : launch_gemm<128, 256, true, false>(kp, &live);
+    case 2: return fp16 ? launch_gemm<256, 256, false, true>(kp, &live) : launch_gemm<256, 256, false, false>(kp, &live);
+    case 1: return fp16 ? launch_gemm<128, 128, false, true>(kp, &live) : launch_gemm<128, 128, false, false>(kp, &live);
+    default: return fp16 ? launch_gemm<128, 256, false, true>(kp, &live) : launch_gemm<128, 256, false, false>(kp, &live);
   }
+}
+
+extern "C" int hdit_linear_fused(const hdit_gemm_args* a) {
+  using namespace hdit;
+  if (a == nullptr) return set_error(HDIT_ERR_BAD_ARG, "null args");
+  if (a->epilogue < HDIT_GEMM_BIAS || a->epilogue > HDIT_GEMM_BIAS_GATE_RESIDUAL)
+    return set_error(HDIT_ERR_BAD_ARG, "unknown epilogue %d", a->epilogue);
+  hdit_linear_group_args g;
+  memset(&g, 0, sizeof(g));
+  g.dtype = a->dtype;
+  g.n_items = 1;
+  g.k = a->k;
+  g.stream = a->stream;
+  g.tile_m = a->tile_m;
+  g.tile_n = a->tile_n;
+  g.cta_pair = a->cta_pair;
+  g.max_ctas = a->max_ctas;
+  hdit_linear_item& im = g.item[0];
+  im.m = a->m;
+  im.n = a->n;
+  im.a = a->a;
+  im.lda = a->lda;
+  im.w = a->w;
+  im.ldw = a->ldw;
+  im.bias = a->bias;
+  im.out = a->out;
+  im.ldo = a->ldo;
+  im.residual = a->residual;
+  im.ldr = a->ldr;
+  im.gate = a->gate;
+  im.gate_batch_stride = a->gate_batch_stride;
+  im.rows_per_batch = a->rows_per_batch;
+  im.epilogue = a->epilogue;
+  return hdit_linear_group(&g);
 }

@@ -528,19 +528,111 @@ def linear_fused(x, weight, bias=None, epilogue="bias", residual=None, gate=None
     return out
 
 
-# Whether linear_tail() may run the fused tensor-core kernel (csrc/gemm_sm100.cu) instead of the library GEMM
-# followed by the one-pass tail kernel, and for which tails. Measured inside the whole step (same box, alternating
-# runs): fusing the GELU wins (Flux-shaped 68.3-68.8 against 68.9-69.3 ms, SD3-shaped 11.77 against 11.99 ms per
-# step); fusing the gated residuals as well loses (69.5 against 68.1-69.1 ms, 12.32 against 12.00 ms) although alone
-# it ties the pair of kernels it replaces -- without multicast loads the kernel moves more operand bytes from L2 per
-# flop than the library's, and under the power cap that costs clock. So only the GELU is fused by default.
-# HDIT_FUSED_LINEAR=0 turns the fused kernel off, HDIT_FUSED_LINEAR_TAILS=gelu_tanh,gate_residual fuses both tails.
+class Lin:
+    """One linear layer of a linear_group() call: y = tail(x @ weight.T + bias). x (B, S, K) with evenly strided rows.
+
+    epilogue "bias", "gelu_tanh", "gate_residual" (residual, gate) as in linear_fused(), or "norm_rope": per-head norm
+    (norm = (kind, weight, bias, eps), kind 1 RMSNorm, 2 LayerNorm with head_dim 64, None for no norm) and rotary
+    embedding (rope = (rope_seq_start, rope_row0) into the call's cos / sin tables, None for no rotation) over heads of
+    `head_dim` columns, as qk_norm_rope() computes them."""
+    __slots__ = ("x", "weight", "bias", "epilogue", "residual", "gate", "out", "head_dim", "norm", "rope")
+
+    def __init__(self, x, linear, epilogue="bias", residual=None, gate=None, out=None, head_dim=0, norm=None, rope=None):
+        self.x, self.weight, self.bias, self.epilogue = x, linear.weight, linear.bias, epilogue
+        self.residual, self.gate, self.out = residual, gate, out
+        self.head_dim, self.norm, self.rope = head_dim, norm, rope
+
+    def _entry(self, b):
+        """This layer on one batch entry."""
+        e = Lin.__new__(Lin)
+        for name in self.__slots__:
+            v = getattr(self, name)
+            setattr(e, name, v[b:b + 1] if name in ("x", "residual", "gate", "out") and v is not None else v)
+        return e
+
+    def _entries(self):
+        """[self], or one layer per batch entry where rows are not evenly strided over the batch (a slice of the rows of
+        every entry)."""
+        if all(t is None or _even_rows(t) for t in (self.x, self.residual, self.out)):
+            return [self]
+        if self.out is None:
+            self.out = torch.empty((self.x.shape[0], self.x.shape[1], self.weight.shape[0]), dtype=self.x.dtype,
+                                   device=self.x.device)
+        return [self._entry(b) for b in range(self.x.shape[0])]
+
+
+_EPILOGUES = {"bias": _C.GEMM_BIAS, "gelu_tanh": _C.GEMM_BIAS_GELU_TANH, "gate_residual": _C.GEMM_BIAS_GATE_RESIDUAL,
+              "norm_rope": _C.GEMM_BIAS_NORM_ROPE}
+
+
+def linear_group(items, cos=None, sin=None, tile_m=0, tile_n=0, cta_pair=0, max_ctas=0):
+    """Several independent linear layers with one inner dimension in one launch (csrc/gemm_sm100.cu), see Lin. A layer
+    whose rows are not evenly strided over the batch counts once per batch entry. No item may read what another one
+    writes. Returns their results in order."""
+    x0 = items[0].x
+    _require_cuda(x0)
+    whole, items = items, [e for it in items for e in it._entries()]
+    if not 1 <= len(items) <= _C.MAX_LINEAR_ITEMS:
+        raise ValueError("between 1 and %d linear layers" % _C.MAX_LINEAR_ITEMS)
+    a = _C.LinearGroupArgs()
+    a.dtype, a.n_items, a.k = _DTYPE_CODE[x0.dtype], len(items), x0.shape[2]
+    a.tile_m, a.tile_n, a.cta_pair, a.max_ctas = tile_m, tile_n, cta_pair, max_ctas
+    if cos is not None:
+        if cos.dtype != torch.float32 or sin.dtype != torch.float32 or not cos.is_contiguous() or not sin.is_contiguous() \
+                or cos.shape != sin.shape:
+            raise TypeError("cos / sin must be contiguous fp32 (rows, D) tables")
+        a.cos, a.sin, a.rope_rows = cos.data_ptr(), sin.data_ptr(), cos.shape[0]
+    for it, d in zip(items, a.item):
+        x, w, bias, out = it.x, it.weight, it.bias, it.out
+        rows, k, rpb, xs = _rows_view(x)
+        n = w.shape[0]
+        if w.dim() != 2 or w.shape[1] != k or k != a.k or w.stride(1) != 1 or w.dtype != x0.dtype or x.dtype != x0.dtype:
+            raise ValueError("every weight must be (N, K), K-contiguous, of x's dtype, with one K")
+        if out is None:
+            out = it.out = torch.empty((x.shape[0], x.shape[1], n), dtype=x.dtype, device=x.device)
+        rows_o, n_o, _, os_ = _rows_view(out)
+        if (rows_o, n_o) != (rows, n) or out.dtype != x.dtype:
+            raise ValueError("out does not match (rows, N)")
+        d.m, d.n, d.a, d.lda, d.w, d.ldw = rows, n, x.data_ptr(), xs, w.data_ptr(), w.stride(0)
+        if bias is not None:
+            if bias.numel() != n or not bias.is_contiguous() or bias.dtype != x.dtype:
+                raise ValueError("bias must be N contiguous elements of x's dtype")
+            d.bias = bias.data_ptr()
+        d.out, d.ldo, d.epilogue, d.rows_per_batch = out.data_ptr(), os_, _EPILOGUES[it.epilogue], rpb
+        if it.epilogue == "gate_residual":
+            rows_r, n_r, _, rs = _rows_view(it.residual)
+            if (rows_r, n_r) != (rows, n) or it.residual.dtype != x.dtype:
+                raise ValueError("residual does not match (rows, N)")
+            gate = it.gate
+            if gate.dim() != 2 or tuple(gate.shape) != (x.shape[0], n) or gate.stride(1) != 1 or gate.dtype != x.dtype:
+                raise ValueError("gate must be (B, N)")
+            d.residual, d.ldr, d.gate, d.gate_batch_stride = it.residual.data_ptr(), rs, gate.data_ptr(), gate.stride(0)
+        elif it.epilogue == "norm_rope":
+            d.head_dim = it.head_dim
+            if it.norm is not None:
+                d.norm, nw, nb, d.eps = it.norm
+                for t in (nw, nb):
+                    if t is not None and (t.dtype != x.dtype or t.numel() != it.head_dim or not t.is_contiguous()):
+                        raise ValueError("norm weight / bias must be head_dim contiguous elements of x's dtype")
+                d.norm_weight = nw.data_ptr() if nw is not None else None
+                d.norm_bias = nb.data_ptr() if nb is not None else None
+            if it.rope is not None:
+                if cos is None or cos.shape[1] != it.head_dim:
+                    raise ValueError("rope needs cos / sin tables of head_dim columns")
+                d.rope, d.rope_seq_start, d.rope_row0 = 1, int(it.rope[0]), int(it.rope[1])
+    with torch.cuda.device(x0.device):
+        a.stream = _stream_ptr(x0.device)
+        _C.check(_C.lib().hdit_linear_group(ctypes.byref(a)))
+    _count()
+    return [it.out for it in whole]
+
+
+# Whether linear layers may run the fused tensor-core kernel (csrc/gemm_sm100.cu) instead of the library GEMM followed by
+# one-pass kernels, for which tails, and from / to how many rows on top of the rule in _group_pays(). HDIT_FUSED_LINEAR=0
+# turns the fused kernel off, HDIT_FUSED_LINEAR_TAILS=gelu_tanh fuses only that tail.
 FUSED_LINEAR = os.environ.get("HDIT_FUSED_LINEAR", "1") == "1"
-FUSED_LINEAR_TAILS = set(os.environ.get("HDIT_FUSED_LINEAR_TAILS", "gelu_tanh").split(","))
-# The fused kernel is used from this row count on. Below, the library's split-K GEMMs fill the GPU better than
-# whole output tiles do (measured at 576 to 2304 rows: the fused kernel takes 1.2x to 2x the library GEMM + tail
-# kernel).
-FUSED_LINEAR_MIN_ROWS = int(os.environ.get("HDIT_FUSED_LINEAR_MIN_ROWS", "4096"))
+FUSED_LINEAR_TAILS = set(os.environ.get("HDIT_FUSED_LINEAR_TAILS", "gelu_tanh,gate_residual").split(","))
+FUSED_LINEAR_MIN_ROWS = int(os.environ.get("HDIT_FUSED_LINEAR_MIN_ROWS", "0"))
 FUSED_LINEAR_MAX_ROWS = int(os.environ.get("HDIT_FUSED_LINEAR_MAX_ROWS", str(1 << 40)))
 
 
@@ -551,7 +643,8 @@ def linear_tail(linear, x, epilogue, residual=None, gate=None, out=None):
     fusable = (FUSED_LINEAR and epilogue in FUSED_LINEAR_TAILS and x.is_cuda and x.dim() == 3 and _even_rows(x) and not torch.is_grad_enabled()
                and FUSED_LINEAR_MIN_ROWS <= x.shape[0] * x.shape[1] <= FUSED_LINEAR_MAX_ROWS
                and (out is None or _even_rows(out)) and (residual is None or _even_rows(residual))
-               and (gate is None or (gate.stride(-1) == 1 and (x.shape[0] == 1 or x.shape[1] >= 32))))
+               and (gate is None or (gate.stride(-1) == 1 and (x.shape[0] == 1 or x.shape[1] >= 32)))
+               and _group_pays([(x.shape[0] * x.shape[1], linear.weight.shape[0])], x.shape[2]))
     if fusable:
         return linear_fused(x, linear.weight, linear.bias, epilogue, residual=residual, gate=gate, out=out)
     y = linear(x)
@@ -560,6 +653,92 @@ def linear_tail(linear, x, epilogue, residual=None, gate=None, out=None):
     if epilogue == "gate_residual":
         return gate_residual(residual, gate, y, out=out)
     raise ValueError(epilogue)
+
+
+def can_group_linears(xs, linears):
+    """Whether these plain torch.nn.Linear layers on these (B, S, K) inputs may go through linear_group(): the switch is
+    on, no gradient is recorded, layouts and types are what the kernel takes, and no hook waits for a layer's call."""
+    if not FUSED_LINEAR or torch.is_grad_enabled():
+        return False
+    k, dtype, dev = xs[0].shape[-1], xs[0].dtype, xs[0].device
+    for x in xs:
+        if not x.is_cuda or x.dim() != 3 or x.dtype != dtype or x.device != dev or dtype not in _DTYPE_CODE or \
+                x.shape[2] != k or k % 8 or x.stride(2) != 1 or x.stride(1) % 8 or x.stride(0) % 8 or x.data_ptr() % 16 or \
+                (x.shape[0] > 1 and x.shape[1] < 32):
+            return False
+    for l in linears:
+        if type(l) is not torch.nn.Linear or l._forward_hooks or l._forward_pre_hooks:
+            return False
+        w, b = l.weight, l.bias
+        if w.dtype != dtype or w.device != dev or w.shape[1] != k or w.shape[0] % 8 or w.stride(1) != 1 or \
+                w.stride(0) % 8 or w.data_ptr() % 16 or \
+                (b is not None and (b.dtype != dtype or not b.is_contiguous() or b.data_ptr() % 16)):
+            return False
+    return True
+
+
+def _group_cost(shapes):
+    """Time of one launch over the (rows, n) output shapes in units of one SM's work on a 128 x 128 block of output: waves
+    of output tiles times the time of a tile, smallest over the kernel's tile shapes (the constants are the library's
+    own, csrc/gemm_sm100.cu). Second result: the same if every SM always had work."""
+    best = None
+    for tm, tn, units, per_tile in ((128, 256, _SM_COUNT, 2.36), (128, 128, _SM_COUNT, 1.25), (256, 256, _SM_COUNT // 2, 2.1)):
+        tiles = sum(-(-m // tm) * -(-n // tn) for m, n in shapes)
+        cost = -(-tiles // units) * per_tile
+        best = cost if best is None else min(best, cost)
+    return best, sum(m * n for m, n in shapes) / 16384.0 / _SM_COUNT
+
+
+# An SM takes 4 cycles per unit of the inner dimension for a 128 x 128 block: 2.3 ns. What a separate library GEMM plus
+# tail kernel costs beyond its arithmetic, and how far the library is from the kernel's best rate.
+_NS_PER_K, _SAVED_US_PER_LAYER, _LIBRARY_RATE = 2.3e-3, 5.0, 1.15
+
+
+def _group_pays(shapes, k):
+    """Whether one launch over these outputs beats a library GEMM and a tail kernel per layer: what the partly filled last
+    wave wastes (the library splits K there) has to stay below what the launches and the extra pass over the output
+    cost. Measured, us, this kernel / library: 2 layers of 1961 + 231 rows, K = 12288: 163 / 150 (not taken); K = 3072:
+    41 / 46; 1024 + 256 rows, K = 12288: 94 / 101; 256 + 77 rows, K = 12288: 53 / 46 (not taken); 4096 + 512 rows, K =
+    12288: 266 / 318; Q, K, V of 2 x (1024 + 77) rows, K = 1536: 33 / 43, of 4096 + 512 rows, K = 3072 with norm and
+    rotation: 236 / 313."""
+    cost, ideal = _group_cost(shapes)
+    return (cost - _LIBRARY_RATE * ideal) * k * _NS_PER_K <= _SAVED_US_PER_LAYER * len(shapes)
+
+
+def use_linear_group(items):
+    """Whether one linear_group() launch beats separate library GEMMs and tail kernels."""
+    items = [e for it in items for e in it._entries()]
+    rows = sum(it.x.shape[0] * it.x.shape[1] for it in items)
+    return 1 <= len(items) <= _C.MAX_LINEAR_ITEMS and FUSED_LINEAR_MIN_ROWS <= rows <= FUSED_LINEAR_MAX_ROWS and \
+        all(it.epilogue not in ("gelu_tanh", "gate_residual") or it.epilogue in FUSED_LINEAR_TAILS for it in items) and \
+        _group_pays([(it.x.shape[0] * it.x.shape[1], it.weight.shape[0]) for it in items], items[0].x.shape[2])
+
+
+def try_linear_tails(specs):
+    """The layers of linear_tails() in one launch, or None where that is not possible or does not pay."""
+    xs, linears = [sp[1] for sp in specs], [sp[0] for sp in specs]
+    if not can_group_linears(xs, linears):
+        return None
+    items = []
+    for linear, x, epilogue, *rest in specs:
+        residual, gate = rest if rest else (None, None)
+        if residual is not None:
+            aligned = residual.data_ptr() % 16 == 0 and gate.data_ptr() % 16 == 0 and \
+                all(v % 8 == 0 for v in (residual.stride(0), residual.stride(1), gate.stride(0)))
+            if not aligned or residual.stride(2) != 1 or gate.stride(-1) != 1 or residual.dtype != x.dtype or gate.dtype != x.dtype:
+                return None
+        items.append(Lin(x, linear, epilogue, residual=residual, gate=gate))
+    return linear_group(items) if use_linear_group(items) else None
+
+
+def linear_tails(specs):
+    """linear_tail() of several independent layers, specs = [(linear, x, epilogue[, residual, gate])]: in one launch where
+    that is possible and pays, else one after the other."""
+    outs = try_linear_tails(specs)
+    if outs is None:
+        outs = [linear_tail(l, x, ep, residual=rest[0] if rest else None, gate=rest[1] if rest else None)
+                for l, x, ep, *rest in specs]
+    return outs
 
 
 def cfg_euler_step(noise_pred, sample, sigmas, step_index, guidance_scale, cfg=True, out=None, out_peer_ptr=None):

@@ -48,6 +48,41 @@ def _norm_rope(attn, q, k, wq, wk, rope, row0, rope_seq_start=0):
                          cos=cos, sin=sin, rope_seq_start=rope_seq_start, rope_row0=row0)
 
 
+def _qkv(attn, streams, rope):
+    """Q, K and V of one or two streams, normalised and rotated where the layer does that. streams: list of
+    (x, projections, (norm_q, norm_k), ranges): ranges are (lo, hi, rotate, row0, rope_seq_start) row ranges of x, row
+    lo + rope_seq_start of a rotated range takes table row row0. One launch computes everything when
+    kernels.use_linear_group says so, else each projection is a library GEMM and norm + RoPE run in place after them.
+    Returns one [q, k, v] of (B, S, H, D) tensors per stream."""
+    H, D = attn.heads, attn.head_dim
+    linears = [p for _, projs, _, _ in streams for p in projs]
+    if kernels.can_group_linears([x for x, _, _, _ in streams], linears):
+        items, outs = [], []
+        for x, projs, norms, ranges in streams:
+            bufs = [torch.empty((x.shape[0], x.shape[1], H * D), dtype=x.dtype, device=x.device) for _ in projs]
+            outs.append([_heads(b, attn) for b in bufs])
+            for lo, hi, rotate, row0, seq_start in ranges:
+                for p, w, buf in zip(projs, (*norms, None), bufs):
+                    is_v = buf is bufs[2]
+                    norm = None if w is None else (w.kind, w.weight, getattr(w, "bias", None), w.eps)
+                    rp = (seq_start, row0) if rotate and not is_v else None
+                    ep = "bias" if norm is None and rp is None else "norm_rope"
+                    whole = lo == 0 and hi == x.shape[1]
+                    items.append(kernels.Lin(x if whole else x[:, lo:hi], p, ep, out=buf if whole else buf[:, lo:hi],
+                                             head_dim=D, norm=norm, rope=rp))
+        if kernels.use_linear_group(items):
+            cos, sin = rope if rope is not None else (None, None)
+            kernels.linear_group(items, cos, sin)
+            return outs
+    outs = []
+    for x, projs, (wq, wk), ranges in streams:
+        q, k, v = (_heads(p(x), attn) for p in projs)
+        for lo, hi, rotate, row0, seq_start in ranges:
+            _norm_rope(attn, q[:, lo:hi], k[:, lo:hi], wq, wk, rope if rotate else None, row0, seq_start)
+        outs.append([q, k, v])
+    return outs
+
+
 def _prologue_range(lo, hi, wq, wk, rope, row0):
     """One row range of the operator's qk_prologue: norm weights (or None), eps, rotary tables, first table row."""
     do_norm = wq is not None
@@ -145,12 +180,13 @@ class JointAttnProcessor:
         if text_offset is not None and ps.get_sequence_parallel_world_size() > 1:
             return self._sharded_text(attn, hidden_states, encoder_hidden_states, image_rotary_emb,
                                       int(text_len or S_txt), token_offset, text_offset, tails)
-        q, k, v = (_heads(p(hidden_states), attn) for p in (attn.to_q, attn.to_k, attn.to_v))
-        tq, tk, tv = (_heads(p(encoder_hidden_states), attn) for p in (attn.add_q_proj, attn.add_k_proj, attn.add_v_proj))
+        rope = image_rotary_emb
         text_rows = S_txt if attn.rope_on_text else 0
-        _norm_rope(attn, q, k, attn.norm_q, attn.norm_k, image_rotary_emb, text_rows + token_offset)
-        _norm_rope(attn, tq, tk, attn.norm_added_q, attn.norm_added_k,
-                   image_rotary_emb if attn.rope_on_text else None, 0)
+        (q, k, v), (tq, tk, tv) = _qkv(attn, [
+            (hidden_states, (attn.to_q, attn.to_k, attn.to_v), (attn.norm_q, attn.norm_k),
+             [(0, S_img, rope is not None, text_rows + token_offset, 0)]),
+            (encoder_hidden_states, (attn.add_q_proj, attn.add_k_proj, attn.add_v_proj),
+             (attn.norm_added_q, attn.norm_added_k), [(0, S_txt, rope is not None and attn.rope_on_text, 0, 0)])], rope)
 
         if ps.get_sequence_parallel_world_size() > 1:
             cls = hetuDiTFluxLongContextAttention if strategy == "front" else hetuDiTJointLongContextAttention
@@ -168,6 +204,9 @@ class JointAttnProcessor:
             img, txt = out[:, :S_img], out[:, S_img:]
         else:
             txt, img = out[:, :S_txt], out[:, S_txt:]
+        if tails[0] is not None and tails[1] is not None:
+            return tuple(kernels.linear_tails([(attn.to_out[0], img, "gate_residual", *tails[0]),
+                                               (attn.to_add_out, txt, "gate_residual", *tails[1])]))
         return _out_proj(attn.to_out[0], img, tails[0]), _out_proj(attn.to_add_out, txt, tails[1])
 
 
@@ -193,7 +232,6 @@ class SingleAttnProcessor:
         of a text stream of text_total tokens that is sharded over the sequence-parallel ranks (see
         JointAttnProcessor); None = the whole text stream is present on every rank, as in the reference."""
         B, S, _ = hidden_states.shape
-        q, k, v = (_heads(p(hidden_states), attn) for p in (attn.to_q, attn.to_k, attn.to_v))
         out4 = None if out is None else out.view(B, S, attn.heads, attn.head_dim)
         S_txt = int(text_len or 0)
         front = attn.text_first
@@ -203,6 +241,7 @@ class SingleAttnProcessor:
         rope_txt = rope if attn.rope_on_text else None
         sp = ps.get_sequence_parallel_world_size()
         if text_offset is not None and sp > 1:
+            q, k, v = (_heads(p(hidden_states), attn) for p in (attn.to_q, attn.to_k, attn.to_v))
             text_rows = int(text_total) if attn.rope_on_text else 0
             ranges = [_prologue_range(t_lo, t_hi, attn.norm_q, attn.norm_k, rope_txt, text_offset),
                       _prologue_range(i_lo, i_hi, attn.norm_q, attn.norm_k, rope, text_rows + token_offset)]
@@ -210,13 +249,15 @@ class SingleAttnProcessor:
                                                              qk_prologue=sorted(ranges, key=lambda r: r[0]))
             return ctx.reshape(B, S, attn.heads * attn.head_dim)
         text_rows = S_txt if attn.rope_on_text else 0
+        rotates = rope is not None
         if front and attn.rope_on_text and token_offset == 0:
-            _norm_rope(attn, q, k, attn.norm_q, attn.norm_k, rope, 0)
+            ranges = [(0, S, rotates, 0, 0)]
         elif front and not attn.rope_on_text:
-            _norm_rope(attn, q, k, attn.norm_q, attn.norm_k, rope, token_offset, rope_seq_start=S_txt)
+            ranges = [(0, S, rotates, token_offset, S_txt)]
         else:
-            _norm_rope(attn, q[:, t_lo:t_hi], k[:, t_lo:t_hi], attn.norm_q, attn.norm_k, rope_txt, 0)
-            _norm_rope(attn, q[:, i_lo:i_hi], k[:, i_lo:i_hi], attn.norm_q, attn.norm_k, rope, text_rows + token_offset)
+            ranges = [(t_lo, t_hi, rope_txt is not None, 0, 0), (i_lo, i_hi, rotates, text_rows + token_offset, 0)]
+        (q, k, v), = _qkv(attn, [(hidden_states, (attn.to_q, attn.to_k, attn.to_v), (attn.norm_q, attn.norm_k), ranges)],
+                          rope)
         if sp > 1:
             strategy = "front" if front else "rear"
             cls = hetuDiTFluxLongContextAttention if front else hetuDiTJointLongContextAttention
@@ -251,8 +292,8 @@ class CogVideoXAttnProcessor:
                  token_offset: int = 0, **_):
         B, S, _ = hidden_states.shape
         T = int(text_len or 0)
-        q, k, v = (_heads(p(hidden_states), attn) for p in (attn.to_q, attn.to_k, attn.to_v))
-        _norm_rope(attn, q, k, attn.norm_q, attn.norm_k, image_rotary_emb, token_offset, rope_seq_start=T)
+        (q, k, v), = _qkv(attn, [(hidden_states, (attn.to_q, attn.to_k, attn.to_v), (attn.norm_q, attn.norm_k),
+                                  [(0, S, image_rotary_emb is not None, token_offset, T)])], image_rotary_emb)
         if ps.get_sequence_parallel_world_size() > 1:
             out = self._ops.get(hetuDiTJointLongContextAttention)(
                 None, q[:, T:], k[:, T:], v[:, T:], dropout_p=0.0, causal=False, joint_tensor_query=q[:, :T],

@@ -16,8 +16,11 @@ the reference's wrapped layout (`attn.module.to_q`, `ff.module.net.0.proj`,
 ...) because parameter-slice migration addresses Linear layers by those names
 (hetu_dit/model_executor/cache/transformer_cache.py:113-154).
 
-GEMMs, LayerNorm and GELU run through torch (cuBLAS / ATen); QK-norm, RoPE,
-the K/V cache and attention run through this package's kernels.
+The blocks' linear layers with their tails (QK-norm + RoPE, GELU, gated
+residual), LayerNorm + modulation, the K/V cache and attention run through
+this package's kernels; the embedders, the adaLN matrix-vector products and
+linear layers that would fill the GPU badly (kernels.use_linear_group) through
+torch (cuBLAS).
 """
 import math
 import os
@@ -136,6 +139,22 @@ class FeedForward(nn.Module):
         if residual is None:
             return self.net[2](x)
         return kernels.linear_tail(self.net[2], x, "gate_residual", residual=residual, gate=gate)
+
+
+def _hooked(ff):
+    """Whether a hook waits for the call of a wrapped MLP or of one of the modules in it."""
+    return any(m._forward_hooks or m._forward_pre_hooks for m in ff.modules())
+
+
+def feed_forward_pair(ff, x, x_res, x_gate, ff_c, c, c_res, c_gate):
+    """ff(x, x_res, x_gate), ff_c(c, c_res, c_gate): the two streams' wrapped MLPs layer by layer, both streams in one
+    launch where that pays (kernels.linear_tails)."""
+    if _hooked(ff) or _hooked(ff_c):
+        return ff(x, residual=x_res, gate=x_gate), ff_c(c, residual=c_res, gate=c_gate)
+    ff, ff_c = ff.module, ff_c.module
+    x, c = kernels.linear_tails([(ff.net[0].proj, x, "gelu_tanh"), (ff_c.net[0].proj, c, "gelu_tanh")])
+    return kernels.linear_tails([(ff.net[2], x, "gate_residual", x_res, x_gate),
+                                 (ff_c.net[2], c, "gate_residual", c_res, c_gate)])
 
 
 class RMSNormWeight(nn.Module):
@@ -270,10 +289,9 @@ class JointBlock(nn.Module):
             br.join()
             return hidden, context
         hidden = a_img if fuse else kernels.gate_residual(hidden, mod[2], a_img)
-        hidden = self.ff(kernels.ln_modulate(hidden, mod[3], mod[4]), residual=hidden, gate=mod[5])
         context = a_txt if fuse else kernels.gate_residual(context, cmod[2], a_txt)
-        context = self.ff_context(kernels.ln_modulate(context, cmod[3], cmod[4]), residual=context, gate=cmod[5])
-        return hidden, context
+        return feed_forward_pair(self.ff, kernels.ln_modulate(hidden, mod[3], mod[4]), hidden, mod[5],
+                                 self.ff_context, kernels.ln_modulate(context, cmod[3], cmod[4]), context, cmod[5])
 
 
 class SingleBlock(nn.Module):
@@ -345,15 +363,26 @@ class CogVideoXBlock(nn.Module):
         kernels.ln_modulate(context, m1[3], m1[4], out=x[:, :S_txt])
         kernels.ln_modulate(hidden, m1[0], m1[1], out=x[:, S_txt:])
         attn = self.attn1.module
-        a = attn.to_out[0](self.attn1(x, image_rotary_emb=rope, text_len=S_txt, token_offset=token_offset))
-        hidden = kernels.gate_residual(hidden, m1[2], a[:, S_txt:])
-        context = kernels.gate_residual(context, m1[5], a[:, :S_txt])
+        a = self.attn1(x, image_rotary_emb=rope, text_len=S_txt, token_offset=token_offset)
+        hidden, context = self._gated(attn.to_out[0], a, S_txt, hidden, m1[2], context, m1[5])
         kernels.ln_modulate(context, m2[3], m2[4], out=x[:, :S_txt])
         kernels.ln_modulate(hidden, m2[0], m2[1], out=x[:, S_txt:])
-        f = self.ff(x)
-        hidden = kernels.gate_residual(hidden, m2[2], f[:, S_txt:])
-        context = kernels.gate_residual(context, m2[5], f[:, :S_txt])
-        return hidden, context
+        if _hooked(self.ff):
+            f = self.ff(x)
+            return kernels.gate_residual(hidden, m2[2], f[:, S_txt:]), kernels.gate_residual(context, m2[5], f[:, :S_txt])
+        ff = self.ff.module
+        return self._gated(ff.net[2], ff.net[0](x), S_txt, hidden, m2[2], context, m2[5])
+
+    @staticmethod
+    def _gated(linear, x, S_txt, hidden, h_gate, context, c_gate):
+        """hidden + h_gate * linear(x video rows), context + c_gate * linear(x text rows): one launch with the gated
+        residuals in the linear layer's epilogue where that pays, else the layer and one pass per stream."""
+        outs = kernels.try_linear_tails([(linear, x[:, S_txt:], "gate_residual", hidden, h_gate),
+                                         (linear, x[:, :S_txt], "gate_residual", context, c_gate)])
+        if outs is None:
+            y = linear(x)
+            outs = (kernels.gate_residual(hidden, h_gate, y[:, S_txt:]), kernels.gate_residual(context, c_gate, y[:, :S_txt]))
+        return outs
 
 
 def rope_tables(ids: torch.Tensor, axes, theta: float = 10000.0):

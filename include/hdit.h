@@ -454,6 +454,66 @@ typedef struct hdit_gemm_args {
 
 HDIT_API int hdit_linear_fused(const hdit_gemm_args* args);
 
+/*
+ * Up to HDIT_MAX_LINEAR_ITEMS independent linear layers of one inner dimension k in one launch: the output tiles of all
+ * items form one list that the persistent CTAs walk, so a layer with few rows (a text stream beside an image stream)
+ * or several layers on the same input (Q, K and V) pay for one partly filled last wave instead of one each. No item may
+ * read what another item writes. Each item has its own tail, one of the three above or
+ *   HDIT_GEMM_BIAS_NORM_ROPE     : per-head norm and rotary embedding of the rounded value, exactly as
+ *                                  hdit_qk_norm_rope computes them: head_dim 64 or 128, n a multiple of it;
+ *                                  norm 0 = none, 1 = RMSNorm, 2 = LayerNorm (head_dim 64 only), norm_weight /
+ *                                  norm_bias (head_dim) or NULL; with rope != 0 row s >= rope_seq_start of a batch entry
+ *                                  (rows_per_batch rows each, >= 32 unless there is a single entry) is rotated by
+ *                                  row s - rope_seq_start + rope_row0 of the cos / sin tables, (rope_rows, head_dim)
+ *                                  fp32 each.
+ * Alignment and ragged sizes as for hdit_linear_fused.
+ *
+ * In the reference Q, K, V and the added text projections are torch.nn.Linear calls of their own, followed by eager norm
+ * and rotary kernels (layers/attention_processor.py:68-120, 632-793, 797-987).
+ */
+#define HDIT_GEMM_BIAS_NORM_ROPE 3
+#define HDIT_MAX_LINEAR_ITEMS 8
+
+typedef struct hdit_linear_item {
+  int64_t m, n;
+  const void* a;
+  int64_t lda;
+  const void* w;
+  int64_t ldw;
+  const void* bias;
+  void* out;
+  int64_t ldo;
+  const void* residual;
+  int64_t ldr;
+  const void* gate;
+  int64_t gate_batch_stride;
+  int64_t rows_per_batch;
+  int32_t epilogue;
+  int32_t head_dim;
+  int32_t norm;
+  int32_t rope;
+  const void* norm_weight;
+  const void* norm_bias;
+  int64_t rope_seq_start;
+  int64_t rope_row0;
+  float eps;
+  int32_t reserved0;
+} hdit_linear_item;
+
+typedef struct hdit_linear_group_args {
+  int32_t dtype;
+  int32_t n_items;
+  int64_t k;
+  const float* cos;
+  const float* sin;
+  int64_t rope_rows;
+  void* stream;
+  int32_t tile_m, tile_n, cta_pair, max_ctas; /* as in hdit_gemm_args */
+  hdit_linear_item item[HDIT_MAX_LINEAR_ITEMS];
+} hdit_linear_group_args;
+
+HDIT_API int hdit_linear_group(const hdit_linear_group_args* args);
+
 #ifdef __cplusplus
 }
 #endif

@@ -124,3 +124,86 @@ def test_linear_fused_flux_mlp_shapes():
         torch.cuda.synchronize()
         _check(buf[:, rows, d:], _want(x[:, rows], w1, b1, "gelu_tanh"))
         _check(out[:, rows], _want(buf[:, rows], w2, b2, "gate_residual", x[:, rows], gate))
+
+
+def _group_case(D, norm, rope, S, B, dtype, seed, H=6, K=328):
+    gen = torch.Generator().manual_seed(seed)
+    lin = torch.nn.Linear(K, H * D, device=DEV, dtype=dtype)
+    with torch.no_grad():
+        lin.weight.copy_(torch.randn(H * D, K, generator=gen) / K ** 0.5)
+        lin.bias.copy_(torch.randn(H * D, generator=gen))
+    x = torch.randn(B, S, K, generator=gen).to(dtype).to(DEV)
+    w = (1 + 0.2 * torch.randn(D, generator=gen)).to(dtype).to(DEV) if norm else None
+    b = (0.2 * torch.randn(D, generator=gen)).to(dtype).to(DEV) if norm == 2 else None
+    return lin, x, (norm, w, b, 1e-6) if norm else None, rope
+
+
+# (head_dim, norm kind, (rope_seq_start, rope_row0) or None, rows per batch entry, batch): rows around the 32-row slices,
+# the 128- and 256-row tiles, batch entries that end inside a slice, rotation that starts inside a tile
+NORM_ROPE = [(128, 1, (0, 0), 1, 1), (128, 1, (0, 3), 257, 1), (64, 1, None, 127, 2), (64, 2, (17, 0), 129, 2),
+             (64, 2, (0, 5), 33, 5), (128, 0, (40, 0), 300, 1), (64, 0, (0, 0), 256, 1), (128, 1, (31, 1), 96, 3)]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tile", TILES, ids=lambda t: f"tile{t[0]}x{t[1]}pair{t[2]}")
+@pytest.mark.parametrize("D,norm,rope,S,B", NORM_ROPE)
+def test_linear_group_norm_rope_is_the_linear_layer_then_qk_norm_rope(D, norm, rope, S, B, tile, dtype):
+    """Same accumulators, same rounding points and order of sums: the bits of the two launches it replaces. The second
+    item (another row count) has no norm; the third writes rows in the middle of a wider buffer."""
+    from hetu_dit_b200 import _C, kernels
+    lin, x, nrm, rp = _group_case(D, norm, rope, S, B, dtype, 100 * D + S)
+    lin2, x2, _, _ = _group_case(D, 0, None, 77, 1, dtype, 5)
+    gen = torch.Generator().manual_seed(3)
+    rows = S + 8
+    cos, sin = (torch.randn(rows, D, generator=gen).to(DEV) for _ in range(2))
+    kw = dict(tile_m=tile[0], tile_n=tile[1], cta_pair=tile[2])
+    wide = torch.full((B, S, 6 * D + 64), 3.0, dtype=dtype, device=DEV)
+    with torch.no_grad():
+        got, got2, got3 = kernels.linear_group(
+            [kernels.Lin(x, lin, "norm_rope", head_dim=D, norm=nrm, rope=rp), kernels.Lin(x2, lin2),
+             kernels.Lin(x, lin, "gelu_tanh", out=wide[..., 64:])], cos, sin, **kw)
+        plain = kernels.linear_fused(x, lin.weight, lin.bias, **kw)
+        want = plain.clone().view(B, S, 6, D)
+        kind, w, b, eps = nrm if nrm else (0, None, None, 1e-6)
+        kernels.qk_norm_rope([(want, w, kind, rp is not None, b)], eps=eps, cos=cos, sin=sin,
+                             rope_seq_start=rp[0] if rp else 0, rope_row0=rp[1] if rp else 0)
+        want2 = kernels.linear_fused(x2, lin2.weight, lin2.bias, **kw)
+        want3 = kernels.linear_fused(x, lin.weight, lin.bias, "gelu_tanh", **kw)
+    torch.cuda.synchronize()
+    assert _C.device_status(0, clear=True)[0] == 0
+    if tile != (0, 0, 0):  # the library may choose other tile shapes for one item than for three: another order of sums
+        assert torch.equal(got.view(B, S, 6, D), want) and torch.equal(got2, want2) and torch.equal(got3, want3)
+    _check(got.view(B, S, 6, D), want)
+    _check(got2, want2)
+    _check(got3, want3)
+    assert (wide[..., :64] == 3).all()
+
+
+def test_linear_group_argument_errors():
+    from hetu_dit_b200 import _C, kernels
+    lin, x, nrm, _ = _group_case(128, 1, None, 40, 2, torch.bfloat16, 1)
+    cos = torch.zeros(30, 128, device=DEV)
+    with torch.no_grad():
+        for it in (kernels.Lin(x, lin, "norm_rope", head_dim=96), kernels.Lin(x, lin, "norm_rope", head_dim=128, rope=(0, 0)),
+                   kernels.Lin(x, lin, "norm_rope", head_dim=128, norm=(2, None, None, 1e-6)),
+                   kernels.Lin(x[:, :20].contiguous(), lin, "norm_rope", head_dim=128, rope=(0, 0))):
+            with pytest.raises((_C.HditError, ValueError)):
+                kernels.linear_group([it], cos, cos)
+        with pytest.raises(ValueError):
+            kernels.linear_group([kernels.Lin(x, lin)] * 9)
+
+
+def test_linear_group_on_row_slices_of_a_batch():
+    """Rows that are a slice of every batch entry (the image and text rows of one attention output): same result as on
+    contiguous copies, nothing written outside."""
+    from hetu_dit_b200 import kernels
+    gen = torch.Generator().manual_seed(9)
+    x = torch.randn(2, 300, 256, generator=gen).to(torch.bfloat16).to(DEV)
+    lin = torch.nn.Linear(256, 192, device=DEV, dtype=torch.bfloat16)
+    gate = torch.randn(2, 192, generator=gen).to(torch.bfloat16).to(DEV)
+    res = [torch.randn(2, n, 192, generator=gen).to(torch.bfloat16).to(DEV) for n in (223, 77)]
+    with torch.no_grad():
+        parts = [x[:, :223], x[:, 223:]]
+        got = kernels.linear_tails([(lin, p, "gate_residual", r, gate) for p, r in zip(parts, res)])
+        for g, p, r in zip(got, parts, res):
+            _check(g, _want(p.contiguous(), lin.weight, lin.bias, "gate_residual", r, gate))
