@@ -313,3 +313,19 @@ def test_peer_heap_mark_and_rewind():
     heap.rewind(mark)
     assert heap.alloc((4, 256), torch.bfloat16, name="usp_q_a")[1] == off_a
     assert heap.alloc((1000,), torch.float32, name="usp_k_a")[1] == off_b
+
+
+def test_copy_pieces_of_very_different_sizes():
+    """CTAs are dealt out in proportion to the bytes: every byte of large, tiny and odd pieces arrives, nothing else."""
+    from hetu_dit_b200 import kernels
+    gen = torch.Generator().manual_seed(2)
+    src, dst, pieces = [], [], []
+    for rows, pitch, width in [(1, 7, 7), (3000, 4096, 4096), (1, 1, 1), (777, 100, 33), (2, 1 << 20, 1 << 20), (50, 48, 16)] * 8:
+        a = torch.randint(0, 255, (rows, pitch), generator=gen, dtype=torch.uint8).to("cuda:0")
+        b = torch.zeros(rows, pitch, dtype=torch.uint8, device="cuda:0")
+        src.append(a), dst.append(b)
+        pieces.append((a.data_ptr(), b.data_ptr(), 1, 0, 0, rows, pitch, pitch, width))
+    kernels.copy_pieces(pieces, torch.device("cuda:0"))
+    for a, b, pc in zip(src, dst, pieces):
+        w = pc[-1]
+        assert torch.equal(a[:, :w], b[:, :w]) and (b[:, w:] == 0).all()
