@@ -217,6 +217,21 @@ class LinearGroupArgs(ctypes.Structure):
     ]
 
 
+
+class LnItem(ctypes.Structure):
+    _fields_ = [
+        ("x", ctypes.c_void_p),
+        ("shift", ctypes.c_void_p),
+        ("scale", ctypes.c_void_p),
+        ("out", ctypes.c_void_p),
+        ("rows", ctypes.c_int64),
+        ("rows_per_batch", ctypes.c_int64),
+        ("x_row_stride", ctypes.c_int64),
+        ("out_row_stride", ctypes.c_int64),
+        ("mod_batch_stride", ctypes.c_int64),
+    ]
+
+
 _lib = None
 _lock = threading.Lock()
 
@@ -244,6 +259,9 @@ def _declare(lib):
     lib.hdit_ln_modulate.restype = ctypes.c_int
     lib.hdit_ln_modulate.argtypes = [ctypes.c_int32] + [ctypes.c_void_p] * 4 + [ctypes.c_int64] * 6 + [
         ctypes.c_float, ctypes.c_void_p]
+    lib.hdit_ln_modulate_items.restype = ctypes.c_int
+    lib.hdit_ln_modulate_items.argtypes = [ctypes.c_int32, ctypes.POINTER(LnItem), ctypes.c_int32, ctypes.c_int64,
+                                           ctypes.c_float, ctypes.c_void_p]
     lib.hdit_gate_residual.restype = ctypes.c_int
     lib.hdit_gate_residual.argtypes = [ctypes.c_int32] + [ctypes.c_void_p] * 4 + [ctypes.c_int64] * 7 + [ctypes.c_void_p]
     lib.hdit_gelu_tanh.restype = ctypes.c_int

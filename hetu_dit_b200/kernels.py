@@ -441,6 +441,27 @@ def ln_modulate(x, shift, scale, eps=1e-6, out=None):
     return out
 
 
+def ln_modulate_pair(x, x_shift, x_scale, c, c_shift, c_scale, eps=1e-6, x_out=None, c_out=None):
+    """ln_modulate() of two tensors of one row length, in one launch where both have evenly strided rows."""
+    pair = ((x, x_shift, x_scale, x_out), (c, c_shift, c_scale, c_out))
+    if not x.is_cuda or x.shape[2] != c.shape[2] or x.dtype != c.dtype or \
+            not all(_even_rows(t) and (out is None or _even_rows(out)) and sh.stride(-1) == 1 and sc.stride(-1) == 1 and
+                    sh.stride(0) == sc.stride(0) for t, sh, sc, out in pair):
+        return ln_modulate(x, x_shift, x_scale, eps, x_out), ln_modulate(c, c_shift, c_scale, eps, c_out)
+    items, outs = (_C.LnItem * 2)(), []
+    for it, (t, sh, sc, out) in zip(items, pair):
+        if out is None:
+            out = torch.empty(tuple(t.shape), dtype=t.dtype, device=t.device)
+        it.rows, dim, it.rows_per_batch, it.x_row_stride = _rows_view(t)
+        it.x, it.shift, it.scale, it.out = t.data_ptr(), sh.data_ptr(), sc.data_ptr(), out.data_ptr()
+        it.out_row_stride, it.mod_batch_stride = out.stride(1), sh.stride(0)
+        outs.append(out)
+    with torch.cuda.device(x.device):
+        _C.check(_C.lib().hdit_ln_modulate_items(_DTYPE_CODE[x.dtype], items, 2, x.shape[2], eps, _stream_ptr(x.device)))
+    _count()
+    return outs
+
+
 def gate_residual(x, gate, y, out=None):
     """x + gate[:, None] * y for x, y (B, S, Dm) and gate a (B, Dm) view."""
     _require_cuda(x)

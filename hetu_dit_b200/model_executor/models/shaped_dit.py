@@ -267,8 +267,7 @@ class JointBlock(nn.Module):
         d = self.d
         mod, cmod = mods if mods is not None else self.modulation(F.silu(temb))
         # LayerNorm + modulation and gate + residual are one fused pass each (csrc/elementwise.cu)
-        h = kernels.ln_modulate(hidden, mod[0], mod[1])
-        c = kernels.ln_modulate(context, cmod[0], cmod[1])
+        h, c = kernels.ln_modulate_pair(hidden, mod[0], mod[1], context, cmod[0], cmod[1])
         sp = (ps.get_sequence_parallel_world_size() > 1 or BRANCH_TEXT_TAIL_ALWAYS) and hidden.is_cuda
         # with fused linear layers the gated residual of the image stream rides on the attention's output
         # projection (and the text stream's too, unless its tail runs on the branch stream below)
@@ -290,8 +289,8 @@ class JointBlock(nn.Module):
             return hidden, context
         hidden = a_img if fuse else kernels.gate_residual(hidden, mod[2], a_img)
         context = a_txt if fuse else kernels.gate_residual(context, cmod[2], a_txt)
-        return feed_forward_pair(self.ff, kernels.ln_modulate(hidden, mod[3], mod[4]), hidden, mod[5],
-                                 self.ff_context, kernels.ln_modulate(context, cmod[3], cmod[4]), context, cmod[5])
+        h, c = kernels.ln_modulate_pair(hidden, mod[3], mod[4], context, cmod[3], cmod[4])
+        return feed_forward_pair(self.ff, h, hidden, mod[5], self.ff_context, c, context, cmod[5])
 
 
 class SingleBlock(nn.Module):
@@ -360,13 +359,11 @@ class CogVideoXBlock(nn.Module):
         B, S_vid, d = hidden.shape
         S_txt = context.shape[1]
         x = torch.empty((B, S_txt + S_vid, d), dtype=hidden.dtype, device=hidden.device)
-        kernels.ln_modulate(context, m1[3], m1[4], out=x[:, :S_txt])
-        kernels.ln_modulate(hidden, m1[0], m1[1], out=x[:, S_txt:])
+        kernels.ln_modulate_pair(hidden, m1[0], m1[1], context, m1[3], m1[4], x_out=x[:, S_txt:], c_out=x[:, :S_txt])
         attn = self.attn1.module
         a = self.attn1(x, image_rotary_emb=rope, text_len=S_txt, token_offset=token_offset)
         hidden, context = self._gated(attn.to_out[0], a, S_txt, hidden, m1[2], context, m1[5])
-        kernels.ln_modulate(context, m2[3], m2[4], out=x[:, :S_txt])
-        kernels.ln_modulate(hidden, m2[0], m2[1], out=x[:, S_txt:])
+        kernels.ln_modulate_pair(hidden, m2[0], m2[1], context, m2[3], m2[4], x_out=x[:, S_txt:], c_out=x[:, :S_txt])
         if _hooked(self.ff):
             f = self.ff(x)
             return kernels.gate_residual(hidden, m2[2], f[:, S_txt:]), kernels.gate_residual(context, m2[5], f[:, :S_txt])

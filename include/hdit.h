@@ -375,6 +375,19 @@ HDIT_API int hdit_attn_fwd_split_static(const hdit_attn_args* args, int32_t firs
 HDIT_API int hdit_ln_modulate(int32_t dtype, const void* x, const void* shift, const void* scale, void* out,
                               int64_t rows, int64_t dim, int64_t rows_per_batch, int64_t x_row_stride,
                               int64_t out_row_stride, int64_t mod_batch_stride, float eps, void* stream);
+
+/* hdit_ln_modulate of one or two tensors of the same row length in one launch (the image and the text stream of a
+ * block). */
+typedef struct hdit_ln_item {
+  const void* x;
+  const void* shift;
+  const void* scale;
+  void* out;
+  int64_t rows, rows_per_batch, x_row_stride, out_row_stride, mod_batch_stride;
+} hdit_ln_item;
+
+HDIT_API int hdit_ln_modulate_items(int32_t dtype, const hdit_ln_item* items, int32_t n_items, int64_t dim, float eps,
+                                    void* stream);
 HDIT_API int hdit_gate_residual(int32_t dtype, const void* x, const void* gate, const void* y, void* out,
                                 int64_t rows, int64_t dim, int64_t rows_per_batch, int64_t x_row_stride,
                                 int64_t y_row_stride, int64_t out_row_stride, int64_t gate_batch_stride, void* stream);

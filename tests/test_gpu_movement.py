@@ -315,6 +315,30 @@ def test_peer_heap_mark_and_rewind():
     assert heap.alloc((1000,), torch.float32, name="usp_k_a")[1] == off_b
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("dim", [256, 768, 1536, 2048, 3072, 4096, 1544])
+@pytest.mark.parametrize("B,n,m", [(1, 1, 1), (2, 33, 7), (1, 300, 2500)])
+def test_ln_modulate_pair_is_two_calls(B, n, m, dim, dtype):
+    """Two tensors in one launch give the bits of a launch each, also into row ranges of one wider buffer."""
+    from hetu_dit_b200 import kernels
+    gen = torch.Generator().manual_seed(dim + n)
+
+    def mk(*s):
+        return torch.randn(*s, generator=gen).to(dtype).to("cuda:0")
+
+    x, c, mod, cmod = mk(B, n, dim), mk(B, m, dim), mk(B, 2 * dim), mk(B, 2 * dim)
+    a, b = kernels.ln_modulate_pair(x, mod[:, :dim], mod[:, dim:], c, cmod[:, :dim], cmod[:, dim:])
+    assert torch.equal(a, kernels.ln_modulate(x, mod[:, :dim], mod[:, dim:]))
+    assert torch.equal(b, kernels.ln_modulate(c, cmod[:, :dim], cmod[:, dim:]))
+    # against fp64: one 16-bit rounding of a value computed in fp32
+    ref = torch.nn.functional.layer_norm(x.double(), (dim,), eps=1e-6) * (1 + mod[:, None, dim:].double()) + mod[:, None, :dim].double()
+    eps16 = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    assert ((a.double() - ref).abs() <= eps16 * ref.abs() + 2e-5).all()
+    buf = torch.full((B, n + m, dim), 5.0, dtype=dtype, device="cuda:0")
+    kernels.ln_modulate_pair(x, mod[:, :dim], mod[:, dim:], c, cmod[:, :dim], cmod[:, dim:], x_out=buf[:, m:], c_out=buf[:, :m])
+    assert torch.equal(buf, torch.cat([b, a], dim=1))
+
+
 def test_copy_pieces_of_very_different_sizes():
     """CTAs are dealt out in proportion to the bytes: every byte of large, tiny and odd pieces arrives, nothing else."""
     from hetu_dit_b200 import kernels
