@@ -319,6 +319,8 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_release();
+  grid_dependency_wait();
 
   // Register hand-over between warpgroups: a softmax thread keeps a whole 128-column row of S.
   // Each warpgroup changes its budget at the top of its own branch so the allocation of the code
@@ -891,8 +893,7 @@ int launch(const AttnKernelParams& kp, int grid, int grid_y, cudaStream_t stream
     HDIT_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<D>::kSmemBytes));
     last_dev = dev;
   }
-  kernel<<<dim3(grid, grid_y), kNumThreads, Cfg<D>::kSmemBytes, stream>>>(kp);
-  HDIT_CUDA_OK(cudaGetLastError());
+  HDIT_CUDA_OK(launch_overlapped(kernel, dim3(grid, grid_y), dim3(kNumThreads), Cfg<D>::kSmemBytes, stream, 1, kp));
   return HDIT_OK;
 }
 
@@ -916,6 +917,8 @@ __global__ void __launch_bounds__(256) attn_combine_kernel(const float* __restri
                                                           long long sq, int heads, void* out, long long out_sb,
                                                           long long out_ss, long long out_sh, float* lse,
                                                           const __grid_constant__ ScatterParams sc) {
+  grid_dependency_release();
+  grid_dependency_wait();
   constexpr int E = D / 32;  // floats per lane: 4 (D = 128) or 2 (D = 64)
   constexpr int kMaxNs = NS > 0 ? NS : 1;
   const int lane = threadIdx.x & 31;
@@ -1194,9 +1197,9 @@ int attn_fwd_impl(const hdit_attn_args* a, int n_split, float* split_out, float*
   long long blocks = (n_rows + 7) / 8;
   if (blocks > 148LL * 8) blocks = 148LL * 8;
 #define HDIT_COMBINE_NS(DD, FF, NN)                                                                                \
-  attn_combine_kernel<DD, FF, NN><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(                               \
-      split_out, split_lse, grid_y, kp.split_acc_stride, kp.split_lse_stride, a->batch, sq, a->heads, a->out,      \
-      a->out_stride_b, a->out_stride_s, a->out_stride_h, a->lse, sc)
+  HDIT_CUDA_OK(launch_overlapped(attn_combine_kernel<DD, FF, NN>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, 1, \
+                                 split_out, split_lse, grid_y, kp.split_acc_stride, kp.split_lse_stride, a->batch, sq, \
+                                 a->heads, a->out, a->out_stride_b, a->out_stride_s, a->out_stride_h, a->lse, sc))
 #define HDIT_COMBINE(DD, FF)                                                                                       \
   do {                                                                                                             \
     if (grid_y == 2) HDIT_COMBINE_NS(DD, FF, 2);                                                                   \
@@ -1211,7 +1214,6 @@ int attn_fwd_impl(const hdit_attn_args* a, int n_split, float* split_out, float*
   }
 #undef HDIT_COMBINE_NS
 #undef HDIT_COMBINE
-  HDIT_CUDA_OK(cudaGetLastError());
   return HDIT_OK;
 }
 

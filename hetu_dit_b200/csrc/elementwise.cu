@@ -64,6 +64,8 @@ struct LnSegs {
 
 template <bool FP16, int NCH>
 __global__ void __launch_bounds__(kLnThreads) ln_modulate_kernel(const __grid_constant__ LnSegs segs, int dim, float eps) {
+  grid_dependency_release();
+  grid_dependency_wait();
   __shared__ float2 red[kLnThreads / 32];
   const int n_chunks = dim / 8;
   const long long rows = segs.s[0].rows + segs.s[1].rows;
@@ -124,6 +126,8 @@ __global__ void __launch_bounds__(kLnThreads) ln_modulate_kernel(const __grid_co
 // (4096 rows: 9.2 against 10.9 us).
 template <bool FP16, int CH>
 __global__ void __launch_bounds__(256) ln_modulate_warp_kernel(const __grid_constant__ LnSegs segs, int dim, float eps) {
+  grid_dependency_release();
+  grid_dependency_wait();
   const int lane = threadIdx.x & 31;
   const long long warp_global = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   const long long n_warps = static_cast<long long>(gridDim.x) * 8;
@@ -184,21 +188,21 @@ __global__ void __launch_bounds__(256) ln_modulate_warp_kernel(const __grid_cons
 }
 
 template <bool FP16, int CH>
-void launch_ln_warp(const LnSegs& segs, int dim, float eps, cudaStream_t st) {
+cudaError_t launch_ln_warp(const LnSegs& segs, int dim, float eps, cudaStream_t st) {
   long long blocks = (segs.s[0].rows + segs.s[1].rows + 7) / 8;
   if (blocks > 148LL * 8) blocks = 148LL * 8;
-  ln_modulate_warp_kernel<FP16, CH><<<static_cast<unsigned>(blocks), 256, 0, st>>>(segs, dim, eps);
+  return launch_overlapped(ln_modulate_warp_kernel<FP16, CH>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, 1, segs, dim, eps);
 }
 
-// The row lengths the warp-per-row kernel is built for.
+// For the row lengths the warp-per-row kernel is built for; *err is the launch's result.
 template <bool FP16>
-bool try_ln_warp(const LnSegs& segs, int dim, float eps, cudaStream_t st) {
+bool try_ln_warp(const LnSegs& segs, int dim, float eps, cudaStream_t st, cudaError_t* err) {
   if (dim % 256 != 0) return false;
   switch (dim / 256) {
-    case 1: launch_ln_warp<FP16, 1>(segs, dim, eps, st); return true;
-    case 2: launch_ln_warp<FP16, 2>(segs, dim, eps, st); return true;
-    case 4: launch_ln_warp<FP16, 4>(segs, dim, eps, st); return true;
-    case 6: launch_ln_warp<FP16, 6>(segs, dim, eps, st); return true;
+    case 1: *err = launch_ln_warp<FP16, 1>(segs, dim, eps, st); return true;
+    case 2: *err = launch_ln_warp<FP16, 2>(segs, dim, eps, st); return true;
+    case 4: *err = launch_ln_warp<FP16, 4>(segs, dim, eps, st); return true;
+    case 6: *err = launch_ln_warp<FP16, 6>(segs, dim, eps, st); return true;
     default: return false;
   }
 }
@@ -209,6 +213,8 @@ __global__ void __launch_bounds__(256) gate_residual_kernel(const uint16_t* __re
                                                            long long rows, int dim, long long rows_per_batch,
                                                            long long x_row_stride, long long y_row_stride,
                                                            long long out_row_stride, long long gate_batch_stride) {
+  grid_dependency_release();
+  grid_dependency_wait();
   const int chunks_per_row = dim / 8;
   const long long total = rows * chunks_per_row;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -249,6 +255,8 @@ template <bool FP16>
 __global__ void __launch_bounds__(256) gelu_tanh_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ out,
                                                        long long rows, int dim, long long x_row_stride,
                                                        long long out_row_stride) {
+  grid_dependency_release();
+  grid_dependency_wait();
   const unsigned chunks_per_row = static_cast<unsigned>(dim / 8);
   const long long total = rows * chunks_per_row;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -303,6 +311,8 @@ __global__ void __launch_bounds__(256) cfg_euler_step_kernel(const uint16_t* __r
                                                             const uint16_t* __restrict__ sample, uint16_t* __restrict__ out,
                                                             uint16_t* __restrict__ out2, long long n_vec, float guidance,
                                                             const float* __restrict__ sigmas, int step) {
+  grid_dependency_release();
+  grid_dependency_wait();
   const float sigma = sigmas[step];
   const float dt = __fsub_rn(sigmas[step + 1], sigma);
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -355,15 +365,8 @@ extern "C" int hdit_cfg_euler_step(int32_t dtype, const void* uncond, const void
   long long blocks = (n_vec + 255) / 256;
   if (blocks > 148LL * 8) blocks = 148LL * 8;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (dtype == HDIT_FP16)
-    cfg_euler_step_kernel<true><<<static_cast<unsigned>(blocks), 256, 0, st>>>(
-        static_cast<const uint16_t*>(uncond), static_cast<const uint16_t*>(cond), static_cast<const uint16_t*>(sample),
-        static_cast<uint16_t*>(out), static_cast<uint16_t*>(out_peer), n_vec, guidance_scale, sigmas, step_index);
-  else
-    cfg_euler_step_kernel<false><<<static_cast<unsigned>(blocks), 256, 0, st>>>(
-        static_cast<const uint16_t*>(uncond), static_cast<const uint16_t*>(cond), static_cast<const uint16_t*>(sample),
-        static_cast<uint16_t*>(out), static_cast<uint16_t*>(out_peer), n_vec, guidance_scale, sigmas, step_index);
-  HDIT_CUDA_OK(cudaGetLastError());
+  HDIT_CUDA_OK(launch_overlapped(dtype == HDIT_FP16 ? cfg_euler_step_kernel<true> : cfg_euler_step_kernel<false>, dim3(static_cast<unsigned>(blocks)),
+                                 dim3(256), 0, st, 1,  static_cast<const uint16_t*>(uncond), static_cast<const uint16_t*>(cond), static_cast<const uint16_t*>(sample), static_cast<uint16_t*>(out), static_cast<uint16_t*>(out_peer), n_vec, guidance_scale, sigmas, step_index));
   return HDIT_OK;
 }
 
@@ -392,8 +395,9 @@ extern "C" int hdit_ln_modulate_items(int32_t dtype, const hdit_ln_item* items, 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int d = static_cast<int>(dim);
   if (segs.s[1].rows_per_batch == 0) segs.s[1].rows_per_batch = 1;
-  if (dtype == HDIT_FP16 ? try_ln_warp<true>(segs, d, eps, st) : try_ln_warp<false>(segs, d, eps, st)) {
-    HDIT_CUDA_OK(cudaGetLastError());
+  cudaError_t err = cudaSuccess;
+  if (dtype == HDIT_FP16 ? try_ln_warp<true>(segs, d, eps, st, &err) : try_ln_warp<false>(segs, d, eps, st, &err)) {
+    HDIT_CUDA_OK(err);
     return HDIT_OK;
   }
   const int nch = static_cast<int>((dim / 8 + kLnThreads - 1) / kLnThreads);
@@ -401,8 +405,8 @@ extern "C" int hdit_ln_modulate_items(int32_t dtype, const hdit_ln_item* items, 
   const unsigned grid = static_cast<unsigned>(rows < 148LL * 16 ? rows : 148LL * 16);
 #define HDIT_LN_CASE(N)                                                                                             \
   case N:                                                                                                           \
-    if (dtype == HDIT_FP16) ln_modulate_kernel<true, N><<<grid, kLnThreads, 0, st>>>(segs, d, eps);                 \
-    else ln_modulate_kernel<false, N><<<grid, kLnThreads, 0, st>>>(segs, d, eps);                                   \
+    HDIT_CUDA_OK(launch_overlapped(dtype == HDIT_FP16 ? ln_modulate_kernel<true, N> : ln_modulate_kernel<false, N>, \
+                                   dim3(grid), dim3(kLnThreads), 0, st, 1, segs, d, eps));                          \
     break;
   switch (nch) {
     HDIT_LN_CASE(1) HDIT_LN_CASE(2) HDIT_LN_CASE(3) HDIT_LN_CASE(4) HDIT_LN_CASE(5) HDIT_LN_CASE(6) HDIT_LN_CASE(7)
@@ -410,7 +414,6 @@ extern "C" int hdit_ln_modulate_items(int32_t dtype, const hdit_ln_item* items, 
     default: return set_error(HDIT_ERR_SHAPE, "row too long");
   }
 #undef HDIT_LN_CASE
-  HDIT_CUDA_OK(cudaGetLastError());
   return HDIT_OK;
 }
 
@@ -440,15 +443,8 @@ extern "C" int hdit_gate_residual(int32_t dtype, const void* x, const void* gate
   auto gp = static_cast<const uint16_t*>(gate);
   auto yp = static_cast<const uint16_t*>(y);
   auto op = static_cast<uint16_t*>(out);
-  if (dtype == HDIT_FP16)
-    gate_residual_kernel<true><<<static_cast<unsigned>(blocks), 256, 0, st>>>(
-        xp, gp, yp, op, rows, static_cast<int>(dim), rows_per_batch, x_row_stride, y_row_stride, out_row_stride,
-        gate_batch_stride);
-  else
-    gate_residual_kernel<false><<<static_cast<unsigned>(blocks), 256, 0, st>>>(
-        xp, gp, yp, op, rows, static_cast<int>(dim), rows_per_batch, x_row_stride, y_row_stride, out_row_stride,
-        gate_batch_stride);
-  HDIT_CUDA_OK(cudaGetLastError());
+  HDIT_CUDA_OK(launch_overlapped(dtype == HDIT_FP16 ? gate_residual_kernel<true> : gate_residual_kernel<false>, dim3(static_cast<unsigned>(blocks)),
+                                 dim3(256), 0, st, 1,  xp, gp, yp, op, rows, static_cast<int>(dim), rows_per_batch, x_row_stride, y_row_stride, out_row_stride, gate_batch_stride));
   return HDIT_OK;
 }
 
@@ -465,14 +461,7 @@ extern "C" int hdit_gelu_tanh(int32_t dtype, const void* x, void* out, int64_t r
   long long blocks = (total + 511) / 512;
   if (blocks > 148LL * 16) blocks = 148LL * 16;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (dtype == HDIT_FP16)
-    gelu_tanh_kernel<true><<<static_cast<unsigned>(blocks), 256, 0, st>>>(
-        static_cast<const uint16_t*>(x), static_cast<uint16_t*>(out), rows, static_cast<int>(dim), x_row_stride,
-        out_row_stride);
-  else
-    gelu_tanh_kernel<false><<<static_cast<unsigned>(blocks), 256, 0, st>>>(
-        static_cast<const uint16_t*>(x), static_cast<uint16_t*>(out), rows, static_cast<int>(dim), x_row_stride,
-        out_row_stride);
-  HDIT_CUDA_OK(cudaGetLastError());
+  HDIT_CUDA_OK(launch_overlapped(dtype == HDIT_FP16 ? gelu_tanh_kernel<true> : gelu_tanh_kernel<false>, dim3(static_cast<unsigned>(blocks)),
+                                 dim3(256), 0, st, 1,  static_cast<const uint16_t*>(x), static_cast<uint16_t*>(out), rows, static_cast<int>(dim), x_row_stride, out_row_stride));
   return HDIT_OK;
 }

@@ -418,6 +418,8 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
   if constexpr (PAIR) cluster_sync_all();  // the partner's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_release();
+  grid_dependency_wait();
 
   const int total_tiles = p.total_tiles;
 
@@ -777,24 +779,12 @@ int launch_gemm(GemmParams& kp, const hdit_linear_group_args* a) {
   if (PAIR) {
     long long pairs = ctas / 2 > 0 ? ctas / 2 : 1;
     if (pairs > tiles) pairs = tiles;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs));
-    cfg.blockDim = dim3(C::kThreads);
-    cfg.dynamicSmemBytes = C::kSmemBytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    HDIT_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, kp));
+    HDIT_CUDA_OK(launch_overlapped(kernel, dim3(static_cast<unsigned>(2 * pairs)), dim3(C::kThreads), C::kSmemBytes, stream, 2,
+                                   kp));
     return HDIT_OK;
   }
   if (ctas > tiles) ctas = tiles;
-  kernel<<<static_cast<unsigned>(ctas), C::kThreads, C::kSmemBytes, stream>>>(kp);
-  HDIT_CUDA_OK(cudaGetLastError());
+  HDIT_CUDA_OK(launch_overlapped(kernel, dim3(static_cast<unsigned>(ctas)), dim3(C::kThreads), C::kSmemBytes, stream, 1, kp));
   return HDIT_OK;
 }
 

