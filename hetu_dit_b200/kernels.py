@@ -1,5 +1,7 @@
 """Tensor-level entry points over the C ABI (torch is used for device memory and streams only)."""
+import contextlib
 import ctypes
+import functools
 import os
 
 import torch
@@ -43,8 +45,20 @@ def _count(n=1):
     _launches += n
 
 
+_NO_SWITCH = contextlib.nullcontext()
+
+
+def _on(device):
+    """A context in which `device` is the current one; entering it costs nothing when it already is, as in a process
+    that drives one GPU."""
+    index = torch.device(device).index
+    return _NO_SWITCH if index is None or index == torch.cuda.current_device() else torch.cuda.device(index)
+
+
 def _stream_ptr(device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    """The current stream of `device` as an address, without a Stream object around it (1.5 us of a 14 us call)."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def _fill_seg(seg, t):
@@ -52,11 +66,8 @@ def _fill_seg(seg, t):
         raise ValueError(f"expected a (B, S, H, D) tensor, got shape {tuple(t.shape)}")
     if t.stride(3) != 1 and t.shape[3] != 1:
         raise ValueError("the head dimension must be contiguous")
-    seg.ptr = t.data_ptr()
-    seg.len = t.shape[1]
-    seg.stride_b = t.stride(0)
-    seg.stride_s = t.stride(1)
-    seg.stride_h = t.stride(2)
+    seg.ptr, seg.len = t.data_ptr(), t.shape[1]
+    seg.stride_b, seg.stride_s, seg.stride_h = t.stride()[:3]
 
 
 def attn_fwd(
@@ -165,7 +176,7 @@ def attn_fwd(
     n_split = 1
     if mode == _C.ATTN_FINAL:
         n_split = _pick_kv_split(q_segs, k_segs, B, H, kv_interleave) if kv_split is None else int(kv_split)
-    with torch.cuda.device(q0.device):
+    with _on(q0.device):
         if n_split > 1:
             part_out = torch.empty((n_split, B, sq, H, D), dtype=torch.float32, device=q0.device)
             part_lse = torch.empty((n_split, B, H, sq), dtype=torch.float32, device=q0.device)
@@ -206,15 +217,15 @@ def _pick_kv_split(q_segs, k_segs, batch, heads, kv_interleave=0):
     length and pays a fixed cost per CTA plus the merge pass. Costs are in units of one KV block of one CTA
     (about 2 us at head_dim 128), fitted to timings of 3..12 heads at 4.6k and 17.8k tokens; a split must
     promise 10 % to be taken."""
-    q_tiles = sum((int(t.shape[1]) + 127) // 128 for t in q_segs)
+    q_lens, kv_lens = [t.shape[1] for t in q_segs], [t.shape[1] for t in k_segs]
+    q_tiles = sum([(n + 127) // 128 for n in q_lens])
     ctas = (q_tiles + 1) // 2 * heads * batch
-    kv_blocks = sum((int(t.shape[1]) + 127) // 128 for t in k_segs)
+    kv_blocks = sum([(n + 127) // 128 for n in kv_lens])
     if ctas <= 0:
         return 1
     if kv_interleave == 2:
         return 1
-    sq = sum(int(t.shape[1]) for t in q_segs)
-    part_bytes = batch * sq * heads * int(q_segs[0].shape[3]) * 4
+    part_bytes = batch * sum(q_lens) * heads * q_segs[0].shape[3] * 4
 
     def cost(s):
         waves = -(-ctas * s // _SM_COUNT)
@@ -241,7 +252,7 @@ def copy_pieces(pieces, device):
     for i, pc in enumerate(pieces):
         (arr[i].src, arr[i].dst, arr[i].n_outer, arr[i].src_outer_pitch, arr[i].dst_outer_pitch, arr[i].rows,
          arr[i].src_pitch, arr[i].dst_pitch, arr[i].row_bytes) = pc
-    with torch.cuda.device(device):
+    with _on(device):
         _C.check(_C.lib().hdit_copy_pieces(arr, n, _stream_ptr(device)))
     _count((n + 39) // 40)
 
@@ -303,7 +314,7 @@ def kv_scatter(kv_cache, new_k, new_v, token_start):
     if nk.stride(2) != 1 or nv.stride(2) != 1 or nk.stride() != nv.stride():
         raise ValueError("new_k / new_v rows must be contiguous and share strides")
     es = kv_cache.element_size()
-    with torch.cuda.device(kv_cache.device):
+    with _on(kv_cache.device):
         _C.check(_C.lib().hdit_kv_scatter(kv_cache.data_ptr(), nk.data_ptr(), nv.data_ptr(), B, S, int(token_start), n,
                                           R * es, nk.stride(1) * es, nk.stride(0) * es, _stream_ptr(kv_cache.device)))
     _count()
@@ -399,7 +410,7 @@ def qk_norm_rope(tensors, *, eps=1e-6, cos=None, sin=None, rope_seq_start=0, rop
             a.signal_slots[i] = ptr
         a.epoch_counter, a.ticket = signal.epoch_ptr, signal.ticket_ptr
     a.stream = _stream_ptr(x0.device)
-    with torch.cuda.device(x0.device):
+    with _on(x0.device):
         _C.check(_C.lib().hdit_qk_norm_rope(ctypes.byref(a)))
     _count()
 
@@ -433,7 +444,7 @@ def ln_modulate(x, shift, scale, eps=1e-6, out=None):
     rows, dim, rpb, xs = _rows_view(x)
     if shift.stride(-1) != 1 or scale.stride(-1) != 1 or shift.stride(0) != scale.stride(0):
         raise ValueError("shift / scale must be (B, Dm) views with contiguous last dim and equal batch stride")
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         _C.check(_C.lib().hdit_ln_modulate(_DTYPE_CODE[x.dtype], x.data_ptr(), shift.data_ptr(), scale.data_ptr(),
                                            out.data_ptr(), rows, dim, rpb, xs, out.stride(1), shift.stride(0), eps,
                                            _stream_ptr(x.device)))
@@ -456,7 +467,7 @@ def ln_modulate_pair(x, x_shift, x_scale, c, c_shift, c_scale, eps=1e-6, x_out=N
         it.x, it.shift, it.scale, it.out = t.data_ptr(), sh.data_ptr(), sc.data_ptr(), out.data_ptr()
         it.out_row_stride, it.mod_batch_stride = out.stride(1), sh.stride(0)
         outs.append(out)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         _C.check(_C.lib().hdit_ln_modulate_items(_DTYPE_CODE[x.dtype], items, 2, x.shape[2], eps, _stream_ptr(x.device)))
     _count()
     return outs
@@ -475,7 +486,7 @@ def gate_residual(x, gate, y, out=None):
         return out
     rows, dim, rpb, xs = _rows_view(x)
     _, _, _, ys = _rows_view(y)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         _C.check(_C.lib().hdit_gate_residual(_DTYPE_CODE[x.dtype], x.data_ptr(), gate.data_ptr(), y.data_ptr(),
                                              out.data_ptr(), rows, dim, rpb, xs, ys, out.stride(1), gate.stride(0),
                                              _stream_ptr(x.device)))
@@ -493,7 +504,7 @@ def gelu_tanh(x, out=None):
     rows_o, dim_o, _, os_ = _rows_view(out)
     if (rows_o, dim_o) != (rows, dim):
         raise ValueError("out differs from x in shape")
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         _C.check(_C.lib().hdit_gelu_tanh(_DTYPE_CODE[x.dtype], x.data_ptr(), out.data_ptr(), rows, dim, xs, os_,
                                          _stream_ptr(x.device)))
     _count()
@@ -542,7 +553,7 @@ def linear_fused(x, weight, bias=None, epilogue="bias", residual=None, gate=None
         a.gate, a.gate_batch_stride = gate.data_ptr(), gate.stride(0)
         a.rows_per_batch = rows // gate.shape[0]
     a.tile_n, a.max_ctas, a.tile_m, a.cta_pair = tile_n, max_ctas, tile_m, cta_pair
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         a.stream = _stream_ptr(x.device)
         _C.check(_C.lib().hdit_linear_fused(ctypes.byref(a)))
     _count()
@@ -563,6 +574,9 @@ class Lin:
         self.residual, self.gate, self.out = residual, gate, out
         self.head_dim, self.norm, self.rope = head_dim, norm, rope
 
+    def _even(self):
+        return self.x.shape[0] == 1 or all(t is None or _even_rows(t) for t in (self.x, self.residual, self.out))
+
     def _entry(self, b):
         """This layer on one batch entry."""
         e = Lin.__new__(Lin)
@@ -574,7 +588,7 @@ class Lin:
     def _entries(self):
         """[self], or one layer per batch entry where rows are not evenly strided over the batch (a slice of the rows of
         every entry)."""
-        if all(t is None or _even_rows(t) for t in (self.x, self.residual, self.out)):
+        if self._even():
             return [self]
         if self.out is None:
             self.out = torch.empty((self.x.shape[0], self.x.shape[1], self.weight.shape[0]), dtype=self.x.dtype,
@@ -603,9 +617,12 @@ def linear_group(items, cos=None, sin=None, tile_m=0, tile_n=0, cta_pair=0, max_
                 or cos.shape != sin.shape:
             raise TypeError("cos / sin must be contiguous fp32 (rows, D) tables")
         a.cos, a.sin, a.rope_rows = cos.data_ptr(), sin.data_ptr(), cos.shape[0]
+    x_prev = None
     for it, d in zip(items, a.item):
         x, w, bias, out = it.x, it.weight, it.bias, it.out
-        rows, k, rpb, xs = _rows_view(x)
+        if x is not x_prev:
+            rows, k, rpb, xs = _rows_view(x)
+            x_prev, x_ptr = x, x.data_ptr()
         n = w.shape[0]
         if w.dim() != 2 or w.shape[1] != k or k != a.k or w.stride(1) != 1 or w.dtype != x0.dtype or x.dtype != x0.dtype:
             raise ValueError("every weight must be (N, K), K-contiguous, of x's dtype, with one K")
@@ -614,7 +631,7 @@ def linear_group(items, cos=None, sin=None, tile_m=0, tile_n=0, cta_pair=0, max_
         rows_o, n_o, _, os_ = _rows_view(out)
         if (rows_o, n_o) != (rows, n) or out.dtype != x.dtype:
             raise ValueError("out does not match (rows, N)")
-        d.m, d.n, d.a, d.lda, d.w, d.ldw = rows, n, x.data_ptr(), xs, w.data_ptr(), w.stride(0)
+        d.m, d.n, d.a, d.lda, d.w, d.ldw = rows, n, x_ptr, xs, w.data_ptr(), w.stride(0)
         if bias is not None:
             if bias.numel() != n or not bias.is_contiguous() or bias.dtype != x.dtype:
                 raise ValueError("bias must be N contiguous elements of x's dtype")
@@ -641,7 +658,7 @@ def linear_group(items, cos=None, sin=None, tile_m=0, tile_n=0, cta_pair=0, max_
                 if cos is None or cos.shape[1] != it.head_dim:
                     raise ValueError("rope needs cos / sin tables of head_dim columns")
                 d.rope, d.rope_seq_start, d.rope_row0 = 1, int(it.rope[0]), int(it.rope[1])
-    with torch.cuda.device(x0.device):
+    with _on(x0.device):
         a.stream = _stream_ptr(x0.device)
         _C.check(_C.lib().hdit_linear_group(ctypes.byref(a)))
     _count()
@@ -665,7 +682,7 @@ def linear_tail(linear, x, epilogue, residual=None, gate=None, out=None):
                and FUSED_LINEAR_MIN_ROWS <= x.shape[0] * x.shape[1] <= FUSED_LINEAR_MAX_ROWS
                and (out is None or _even_rows(out)) and (residual is None or _even_rows(residual))
                and (gate is None or (gate.stride(-1) == 1 and (x.shape[0] == 1 or x.shape[1] >= 32)))
-               and _group_pays([(x.shape[0] * x.shape[1], linear.weight.shape[0])], x.shape[2]))
+               and _group_pays(((x.shape[0] * x.shape[1], linear.weight.shape[0]),), x.shape[2]))
     if fusable:
         return linear_fused(x, linear.weight, linear.bias, epilogue, residual=residual, gate=gate, out=out)
     y = linear(x)
@@ -682,18 +699,27 @@ def can_group_linears(xs, linears):
     if not FUSED_LINEAR or torch.is_grad_enabled():
         return False
     k, dtype, dev = xs[0].shape[-1], xs[0].dtype, xs[0].device
+    if dtype not in _DTYPE_CODE or k % 8:
+        return False
     for x in xs:
-        if not x.is_cuda or x.dim() != 3 or x.dtype != dtype or x.device != dev or dtype not in _DTYPE_CODE or \
-                x.shape[2] != k or k % 8 or x.stride(2) != 1 or x.stride(1) % 8 or x.stride(0) % 8 or x.data_ptr() % 16 or \
-                (x.shape[0] > 1 and x.shape[1] < 32):
+        if not x.is_cuda or x.dim() != 3 or x.dtype != dtype or x.device != dev:
+            return False
+        (B, S, kx), (sb, ss, sk) = x.shape, x.stride()
+        if kx != k or sk != 1 or ss % 8 or sb % 8 or x.data_ptr() % 16 or (B > 1 and S < 32):
             return False
     for l in linears:
         if type(l) is not torch.nn.Linear or l._forward_hooks or l._forward_pre_hooks:
             return False
-        w, b = l.weight, l.bias
-        if w.dtype != dtype or w.device != dev or w.shape[1] != k or w.shape[0] % 8 or w.stride(1) != 1 or \
-                w.stride(0) % 8 or w.data_ptr() % 16 or \
-                (b is not None and (b.dtype != dtype or not b.is_contiguous() or b.data_ptr() % 16)):
+        w, b = l._parameters.get("weight"), l._parameters.get("bias")
+        if w is None or w.dtype != dtype or w.device != dev or w.data_ptr() % 16:
+            return False
+        (n, kw), (sn, sk) = w.shape, w.stride()
+        if kw != k or n % 8 or sk != 1 or sn % 8:
+            return False
+        if b is None:
+            if l.bias is not None:
+                return False
+        elif b.dtype != dtype or not b.is_contiguous() or b.data_ptr() % 16:
             return False
     return True
 
@@ -715,6 +741,7 @@ def _group_cost(shapes):
 _NS_PER_K, _SAVED_US_PER_LAYER, _LIBRARY_RATE = 2.3e-3, 5.0, 1.15
 
 
+@functools.lru_cache(maxsize=4096)
 def _group_pays(shapes, k):
     """Whether one launch over these outputs beats a library GEMM and a tail kernel per layer: what the partly filled last
     wave wastes (the library splits K there) has to stay below what the launches and the extra pass over the output
@@ -728,11 +755,16 @@ def _group_pays(shapes, k):
 
 def use_linear_group(items):
     """Whether one linear_group() launch beats separate library GEMMs and tail kernels."""
-    items = [e for it in items for e in it._entries()]
-    rows = sum(it.x.shape[0] * it.x.shape[1] for it in items)
-    return 1 <= len(items) <= _C.MAX_LINEAR_ITEMS and FUSED_LINEAR_MIN_ROWS <= rows <= FUSED_LINEAR_MAX_ROWS and \
-        all(it.epilogue not in ("gelu_tanh", "gate_residual") or it.epilogue in FUSED_LINEAR_TAILS for it in items) and \
-        _group_pays([(it.x.shape[0] * it.x.shape[1], it.weight.shape[0]) for it in items], items[0].x.shape[2])
+    shapes, rows = [], 0
+    for it in items:
+        if it.epilogue in ("gelu_tanh", "gate_residual") and it.epilogue not in FUSED_LINEAR_TAILS:
+            return False
+        B, S, k = it.x.shape
+        n = it.weight.shape[0]
+        shapes += [(B * S, n)] if it._even() else [(S, n)] * B
+        rows += B * S
+    return 1 <= len(shapes) <= _C.MAX_LINEAR_ITEMS and FUSED_LINEAR_MIN_ROWS <= rows <= FUSED_LINEAR_MAX_ROWS and \
+        _group_pays(tuple(shapes), k)
 
 
 def try_linear_tails(specs):
@@ -780,7 +812,7 @@ def cfg_euler_step(noise_pred, sample, sigmas, step_index, guidance_scale, cfg=T
     es = noise_pred.element_size()
     uncond = noise_pred.data_ptr()
     cond = uncond + n * es if cfg else None
-    with torch.cuda.device(sample.device):
+    with _on(sample.device):
         _C.check(_C.lib().hdit_cfg_euler_step(_DTYPE_CODE[sample.dtype], uncond, cond, sample.data_ptr(), out.data_ptr(),
                                               out_peer_ptr, n, float(guidance_scale), sigmas.data_ptr(), int(step_index),
                                               _stream_ptr(sample.device)))
