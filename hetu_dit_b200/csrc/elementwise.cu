@@ -50,7 +50,7 @@ __device__ __forceinline__ float2 block_sum2(float a, float b, float2* red) {
 }
 
 // The rows of up to two tensors (the image and the text stream of a block) are one list, so that the second one costs no
-// launch of its own: 4096 + 512 rows of 3072 12.1 -> 11.4 us, 2 x (1024 + 77) rows of 1536 6.8 -> 4.5 us.
+// launch of its own: 4096 + 512 rows of 3072 12.1 -> 10.6 us, 2 x (1024 + 77) rows of 1536 6.8 -> 4.7 us.
 struct LnSeg {
   const uint16_t* x;
   const uint16_t* shift;
