@@ -1,5 +1,5 @@
-// Per-head RMSNorm / LayerNorm and rotary embedding of eight consecutive elements, shared by the in-place / scatter
-// kernel (norm_rope.cu) and the linear kernel's epilogue (gemm_sm100.cu).
+// Per-head RMSNorm / LayerNorm and rotary embedding of eight consecutive elements in the linear kernel's epilogue
+// (gemm_sm100.cu), with the rounding points of norm_rope_kernel (norm_rope.cu), so that both give the same bits.
 //
 // Rounding follows the reference's eager sequence: normalise in fp32, round to the 16-bit type, multiply by the 16-bit
 // weight and round, rotate in fp32 with separately rounded products, round once more. Roundings are done two at a
