@@ -48,17 +48,24 @@ def _count(n=1):
 _NO_SWITCH = contextlib.nullcontext()
 
 
+def _cuda_index(device):
+    """Index of a CUDA device, the current one's where `device` names none. Any other kind of device is refused: the
+    addresses of its tensors are not the GPU's."""
+    if device.type != "cuda":
+        raise ValueError(f"expected a cuda device, got {device}")
+    return torch.cuda.current_device() if device.index is None else device.index
+
+
 def _on(device):
     """A context in which `device` is the current one; entering it costs nothing when it already is, as in a process
     that drives one GPU."""
-    index = torch.device(device).index
-    return _NO_SWITCH if index is None or index == torch.cuda.current_device() else torch.cuda.device(index)
+    index = _cuda_index(device)
+    return _NO_SWITCH if index == torch.cuda.current_device() else torch.cuda.device(index)
 
 
 def _stream_ptr(device):
     """The current stream of `device` as an address, without a Stream object around it (1.5 us of a 14 us call)."""
-    index = device.index
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+    return torch._C._cuda_getCurrentRawStream(_cuda_index(device))
 
 
 def _fill_seg(seg, t):
