@@ -49,8 +49,10 @@ _NO_SWITCH = contextlib.nullcontext()
 
 
 def _cuda_index(device):
-    """Index of a CUDA device, the current one's where `device` names none. Any other kind of device is refused: the
-    addresses of its tensors are not the GPU's."""
+    """Index of a CUDA device given as a torch.device, a string, an integer or None; the current one's where it names
+    none. Any other kind of device is refused: the addresses of its tensors are not the GPU's."""
+    if type(device) is not torch.device:
+        device = torch.device("cuda", device) if isinstance(device, int) else torch.device(device or "cuda")
     if device.type != "cuda":
         raise ValueError(f"expected a cuda device, got {device}")
     return torch.cuda.current_device() if device.index is None else device.index

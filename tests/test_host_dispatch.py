@@ -42,3 +42,13 @@ def test_host_tensors_never_reach_a_kernel(lib):
         with pytest.raises(ValueError, match="cuda"):
             call()
     assert lib.calls == []
+
+
+@pytest.mark.parametrize("device", ["cuda:0", "cuda", 0, -1, None, torch.device("cuda"), torch.device("cuda", 0)])
+def test_devices_are_named_as_torch_names_them(lib, device):
+    kernels.copy_pieces([BOX], device)
+    (name, args), = lib.calls
+    assert name == "hdit_copy_pieces" and args[1:] == (1, 1000)
+    with pytest.raises(ValueError):
+        kernels.copy_pieces([BOX], "cpu")
+    assert len(lib.calls) == 1
