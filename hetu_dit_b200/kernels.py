@@ -52,7 +52,9 @@ def _cuda_index(device):
     """Index of a CUDA device given as a torch.device, a string, an integer or None; the current one's where it names
     none. Any other kind of device is refused: the addresses of its tensors are not the GPU's."""
     if type(device) is not torch.device:
-        device = torch.device("cuda", device) if isinstance(device, int) else torch.device(device or "cuda")
+        if isinstance(device, int):  # -1 is the current device, as for torch.cuda.device()
+            return torch.cuda.current_device() if device < 0 else device
+        device = torch.device("cuda" if device is None else device)
     if device.type != "cuda":
         raise ValueError(f"expected a cuda device, got {device}")
     return torch.cuda.current_device() if device.index is None else device.index
