@@ -5,6 +5,7 @@ import functools
 import os
 
 import torch
+from torch.nn.modules import module as _all_modules
 
 from . import _C
 
@@ -685,6 +686,20 @@ FUSED_LINEAR_MIN_ROWS = int(os.environ.get("HDIT_FUSED_LINEAR_MIN_ROWS", "0"))
 FUSED_LINEAR_MAX_ROWS = int(os.environ.get("HDIT_FUSED_LINEAR_MAX_ROWS", str(1 << 40)))
 
 
+_PLAIN_TENSORS = (torch.nn.Parameter, torch.Tensor)
+
+
+def _is_plain_linear(linear):
+    """Whether calling `linear` is x @ weight.T + bias and nothing else, so that a kernel may be given its weight instead:
+    no other class (an adapter, a quantised layer), no forward() put on the object, no weight of a tensor class of its
+    own, and no hook, of this layer or of all modules, that waits for the call."""
+    if type(linear) is not torch.nn.Linear or linear._forward_hooks or linear._forward_pre_hooks or \
+            "forward" in linear.__dict__ or _all_modules._global_forward_hooks or _all_modules._global_forward_pre_hooks:
+        return False
+    w, b = linear.weight, linear.bias
+    return type(w) in _PLAIN_TENSORS and (b is None or type(b) in _PLAIN_TENSORS)
+
+
 def linear_tail(linear, x, epilogue, residual=None, gate=None, out=None):
     """A torch.nn.Linear followed by its elementwise tail ("gelu_tanh", or "gate_residual" = residual +
     gate[:, None] * linear(x)), as one kernel when FUSED_LINEAR is set and the layouts allow it (rows evenly
@@ -693,6 +708,7 @@ def linear_tail(linear, x, epilogue, residual=None, gate=None, out=None):
                and FUSED_LINEAR_MIN_ROWS <= x.shape[0] * x.shape[1] <= FUSED_LINEAR_MAX_ROWS
                and (out is None or _even_rows(out)) and (residual is None or _even_rows(residual))
                and (gate is None or (gate.stride(-1) == 1 and (x.shape[0] == 1 or x.shape[1] >= 32)))
+               and _is_plain_linear(linear)
                and _group_pays(((x.shape[0] * x.shape[1], linear.weight.shape[0]),), x.shape[2]))
     if fusable:
         return linear_fused(x, linear.weight, linear.bias, epilogue, residual=residual, gate=gate, out=out)
@@ -719,7 +735,7 @@ def can_group_linears(xs, linears):
         if kx != k or sk != 1 or ss % 8 or sb % 8 or x.data_ptr() % 16 or (B > 1 and S < 32):
             return False
     for l in linears:
-        if type(l) is not torch.nn.Linear or l._forward_hooks or l._forward_pre_hooks:
+        if not _is_plain_linear(l):
             return False
         w, b = l._parameters.get("weight"), l._parameters.get("bias")
         if w is None or w.dtype != dtype or w.device != dev or w.data_ptr() % 16:

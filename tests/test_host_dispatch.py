@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from hetu_dit_b200 import _C, kernels
+from tests import cpu_stand_ins
 
 
 class Recorder:
@@ -52,3 +53,97 @@ def test_devices_are_named_as_torch_names_them(lib, device):
     with pytest.raises(ValueError):
         kernels.copy_pieces([BOX], "cpu")
     assert len(lib.calls) == 1
+
+
+class OnGpu(torch.Tensor):
+    """A host tensor that says it is on the GPU."""
+    is_cuda = property(lambda self: True)
+
+
+def gpu_like(*shape, dtype=torch.bfloat16):
+    return torch.randn(*shape).to(dtype).as_subclass(OnGpu)
+
+
+@pytest.fixture
+def fused(monkeypatch):
+    """Calls of the fused linear kernels, by name; the kernels after a library GEMM are torch stand-ins."""
+    calls = []
+
+    def record(name, result):
+        def call(*args, **kw):
+            calls.append(name)
+            return result(*args, **kw)
+        return call
+
+    monkeypatch.setattr(kernels, "linear_fused", record("linear_fused", lambda x, w, *a, **kw: x.new_zeros(*x.shape[:2], w.shape[0])))
+    monkeypatch.setattr(kernels, "linear_group", record("linear_group", lambda items, *a, **kw: [
+        it.x.new_zeros(*it.x.shape[:2], it.weight.shape[0]) for it in items]))
+    for name in ("gelu_tanh", "gate_residual", "qk_norm_rope"):
+        monkeypatch.setattr(kernels, name, getattr(cpu_stand_ins, name))
+    monkeypatch.setattr(kernels, "_group_pays", lambda shapes, k: True)
+    return calls
+
+
+class Doubled(torch.nn.Linear):
+    """A layer of its own with a weight, as an adapter or a quantised layer has."""
+
+    def forward(self, x):
+        return 2 * super().forward(x)
+
+
+def _hook(linear):
+    linear.register_forward_hook(lambda m, args, y: 2 * y)
+
+
+def _pre_hook(linear):
+    linear.register_forward_pre_hook(lambda m, args: (2 * args[0],))
+
+
+def _own_forward(linear):
+    linear.forward = lambda x: 2 * torch.nn.functional.linear(x, linear.weight, linear.bias)
+
+
+def _other_module(linear):
+    linear.__class__ = Doubled
+
+
+def _other_weight(linear):
+    class Packed(OnGpu):
+        pass
+    linear.weight = torch.nn.Parameter((2 * linear.weight.detach()).as_subclass(Packed))
+
+
+def _everywhere(linear):
+    return torch.nn.modules.module.register_module_forward_hook(lambda m, args, y: 2 * y if m is linear else None)
+
+
+@pytest.mark.parametrize("rows", [64, 4608])
+@pytest.mark.parametrize("epilogue", ["gelu_tanh", "gate_residual"])
+@pytest.mark.parametrize("change", [_hook, _pre_hook, _own_forward, _other_module, _other_weight, _everywhere])
+def test_a_layer_with_a_call_of_its_own_is_called(fused, change, epilogue, rows):
+    """Whatever a program puts in the way of a linear layer's call changes the result, with fusion on."""
+    linear = torch.nn.Linear(32, 64, bias=False, dtype=torch.bfloat16)
+    x = gpu_like(1, rows, 32)
+    rest = (gpu_like(1, rows, 64), gpu_like(1, 64)) if epilogue == "gate_residual" else ()
+    with torch.no_grad():
+        y = 2 * linear(x)
+        want = cpu_stand_ins.gelu_tanh(y) if epilogue == "gelu_tanh" else cpu_stand_ins.gate_residual(rest[0], rest[1], y)
+        handle = change(linear)
+        try:
+            one = kernels.linear_tail(linear, x, epilogue, *rest)
+            plain = torch.nn.Linear(32, 64, dtype=torch.bfloat16)
+            two = kernels.linear_tails([(linear, x, epilogue, *rest), (plain, x, epilogue, *rest)])[0]
+        finally:
+            if handle is not None:
+                handle.remove()
+    assert torch.equal(one, want) and torch.equal(two, want)
+
+
+@pytest.mark.parametrize("epilogue", ["gelu_tanh", "gate_residual"])
+def test_a_plain_layer_is_fused(fused, epilogue):
+    linear, x = torch.nn.Linear(32, 64, dtype=torch.bfloat16), gpu_like(1, 64, 32)
+    rest = (gpu_like(1, 64, 64), gpu_like(1, 64)) if epilogue == "gate_residual" else ()
+    with torch.no_grad():
+        kernels.linear_tail(linear, x, epilogue, *rest)
+        kernels.linear_tails([(linear, x, epilogue, *rest)] * 2)
+    assert fused == ["linear_fused", "linear_group"]
