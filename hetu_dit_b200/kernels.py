@@ -465,9 +465,10 @@ def ln_modulate(x, shift, scale, eps=1e-6, out=None):
 
 
 def ln_modulate_pair(x, x_shift, x_scale, c, c_shift, c_scale, eps=1e-6, x_out=None, c_out=None):
-    """ln_modulate() of two tensors of one row length, in one launch where both have evenly strided rows."""
+    """ln_modulate() of two tensors of one row length, in one launch where both are on one device and have evenly strided
+    rows."""
     pair = ((x, x_shift, x_scale, x_out), (c, c_shift, c_scale, c_out))
-    if not x.is_cuda or x.shape[2] != c.shape[2] or x.dtype != c.dtype or \
+    if not x.is_cuda or c.device != x.device or x.shape[2] != c.shape[2] or x.dtype != c.dtype or \
             not all(_even_rows(t) and (out is None or _even_rows(out)) and sh.stride(-1) == 1 and sc.stride(-1) == 1 and
                     sh.stride(0) == sc.stride(0) for t, sh, sc, out in pair):
         return ln_modulate(x, x_shift, x_scale, eps, x_out), ln_modulate(c, c_shift, c_scale, eps, c_out)

@@ -29,6 +29,15 @@ def lib(monkeypatch):
     return rec
 
 
+class OnGpu(torch.Tensor):
+    """A host tensor that says it is on the GPU."""
+    is_cuda = property(lambda self: True)
+
+
+def gpu_like(*shape, dtype=torch.bfloat16):
+    return torch.randn(*shape).to(dtype).as_subclass(OnGpu)
+
+
 BOX = (16, 32, 1, 0, 0, 1, 0, 0, 8)
 
 
@@ -45,6 +54,15 @@ def test_host_tensors_never_reach_a_kernel(lib):
     assert lib.calls == []
 
 
+def test_ln_modulate_pair_refuses_a_host_tensor_beside_a_gpu_tensor(lib, monkeypatch):
+    x, mod = gpu_like(1, 8, 256), gpu_like(1, 256)
+    x_dev = type("OnGpu0", (OnGpu,), {"device": property(lambda self: torch.device("cuda", 0))})
+    monkeypatch.setattr(torch, "empty", lambda shape, **kw: torch.zeros(shape, dtype=kw["dtype"]))
+    with pytest.raises(RuntimeError, match="CUDA"):
+        kernels.ln_modulate_pair(x.as_subclass(x_dev), mod, mod, torch.zeros(1, 4, 256, dtype=torch.bfloat16), mod, mod)
+    assert "hdit_ln_modulate_items" not in [name for name, _ in lib.calls]
+
+
 @pytest.mark.parametrize("device", ["cuda:0", "cuda", 0, -1, None, torch.device("cuda"), torch.device("cuda", 0)])
 def test_devices_are_named_as_torch_names_them(lib, device):
     kernels.copy_pieces([BOX], device)
@@ -53,15 +71,6 @@ def test_devices_are_named_as_torch_names_them(lib, device):
     with pytest.raises(ValueError):
         kernels.copy_pieces([BOX], "cpu")
     assert len(lib.calls) == 1
-
-
-class OnGpu(torch.Tensor):
-    """A host tensor that says it is on the GPU."""
-    is_cuda = property(lambda self: True)
-
-
-def gpu_like(*shape, dtype=torch.bfloat16):
-    return torch.randn(*shape).to(dtype).as_subclass(OnGpu)
 
 
 @pytest.fixture
