@@ -703,13 +703,12 @@ def _is_plain_linear(linear):
 
 def linear_tail(linear, x, epilogue, residual=None, gate=None, out=None):
     """A torch.nn.Linear followed by its elementwise tail ("gelu_tanh", or "gate_residual" = residual +
-    gate[:, None] * linear(x)), as one kernel when FUSED_LINEAR is set and the layouts allow it (rows evenly
-    strided across the batch), else as the library GEMM plus hdit_gelu_tanh / hdit_gate_residual."""
-    fusable = (FUSED_LINEAR and epilogue in FUSED_LINEAR_TAILS and x.is_cuda and x.dim() == 3 and _even_rows(x) and not torch.is_grad_enabled()
+    gate[:, None] * linear(x)), as one kernel when can_group_linears() allows it, rows are evenly strided across the
+    batch and it pays, else as the call of `linear` plus hdit_gelu_tanh / hdit_gate_residual."""
+    fusable = (epilogue in FUSED_LINEAR_TAILS and can_group_linears([x], [linear]) and _even_rows(x)
                and FUSED_LINEAR_MIN_ROWS <= x.shape[0] * x.shape[1] <= FUSED_LINEAR_MAX_ROWS
-               and (out is None or _even_rows(out)) and (residual is None or _even_rows(residual))
-               and (gate is None or (gate.stride(-1) == 1 and (x.shape[0] == 1 or x.shape[1] >= 32)))
-               and _is_plain_linear(linear)
+               and (out is None or (_even_rows(out) and _aligned(out))) and (residual is None or _even_rows(residual))
+               and (gate is None or gate.stride(-1) == 1)
                and _group_pays(((x.shape[0] * x.shape[1], linear.weight.shape[0]),), x.shape[2]))
     if fusable:
         return linear_fused(x, linear.weight, linear.bias, epilogue, residual=residual, gate=gate, out=out)
@@ -721,9 +720,18 @@ def linear_tail(linear, x, epilogue, residual=None, gate=None, out=None):
     raise ValueError(epilogue)
 
 
+def _aligned(x):
+    """Whether the rows of a (B, S, Dm) tensor are contiguous, do not overlap and start on 16-byte boundaries (16-bit
+    elements)."""
+    (B, _, dim), (sb, ss, sk) = x.shape, x.stride()
+    return sk == 1 and ss >= dim and ss % 8 == 0 and (B == 1 or sb % 8 == 0) and x.data_ptr() % 16 == 0
+
+
 def can_group_linears(xs, linears):
-    """Whether these plain torch.nn.Linear layers on these (B, S, K) inputs may go through linear_group(): the switch is
-    on, no gradient is recorded, layouts and types are what the kernel takes, and no hook waits for a layer's call."""
+    """Whether these layers on these (B, S, K) inputs may go through linear_fused() / linear_group(): the switch is on, no
+    gradient is recorded, the layers are plain torch.nn.Linear that nothing waits for the call of, and layouts and types
+    are what the kernel takes. The library GEMM takes all others: inner sizes that are no multiple of 8, rows that overlap or
+    do not start on 16-byte boundaries."""
     if not FUSED_LINEAR or torch.is_grad_enabled():
         return False
     k, dtype, dev = xs[0].shape[-1], xs[0].dtype, xs[0].device
@@ -732,8 +740,7 @@ def can_group_linears(xs, linears):
     for x in xs:
         if not x.is_cuda or x.dim() != 3 or x.dtype != dtype or x.device != dev:
             return False
-        (B, S, kx), (sb, ss, sk) = x.shape, x.stride()
-        if kx != k or sk != 1 or ss % 8 or sb % 8 or x.data_ptr() % 16 or (B > 1 and S < 32):
+        if x.shape[2] != k or not _aligned(x) or (x.shape[0] > 1 and x.shape[1] < 32):
             return False
     for l in linears:
         if not _is_plain_linear(l):
@@ -742,12 +749,12 @@ def can_group_linears(xs, linears):
         if w is None or w.dtype != dtype or w.device != dev or w.data_ptr() % 16:
             return False
         (n, kw), (sn, sk) = w.shape, w.stride()
-        if kw != k or n % 8 or sk != 1 or sn % 8:
+        if kw != k or n % 8 or sk != 1 or sn < k or sn % 8:
             return False
         if b is None:
             if l.bias is not None:
                 return False
-        elif b.dtype != dtype or not b.is_contiguous() or b.data_ptr() % 16:
+        elif b.dtype != dtype or b.numel() != n or not b.is_contiguous() or b.data_ptr() % 16:
             return False
     return True
 

@@ -156,3 +156,52 @@ def test_a_plain_layer_is_fused(fused, epilogue):
         kernels.linear_tail(linear, x, epilogue, *rest)
         kernels.linear_tails([(linear, x, epilogue, *rest)] * 2)
     assert fused == ["linear_fused", "linear_group"]
+
+
+def _layer(n=64, k=32, bias=True):
+    return torch.nn.Linear(k, n, bias=bias, dtype=torch.bfloat16)
+
+
+def _odd_weight():
+    linear = _layer()
+    linear.weight = torch.nn.Parameter(torch.randn(64 * 32 + 1).to(torch.bfloat16)[1:].view(64, 32))
+    return linear
+
+
+def _odd_bias():
+    linear = _layer()
+    linear.bias = torch.nn.Parameter(torch.randn(65).to(torch.bfloat16)[1:])
+    return linear
+
+
+def _expanded_weight():
+    linear = _layer()
+    linear.weight = torch.nn.Parameter(torch.randn(1, 32).to(torch.bfloat16).expand(64, 32))
+    return linear
+
+
+# what the library GEMM takes and the fused kernel does not: (linear layer, input, out or None)
+LAYOUTS = {
+    "inner size not a multiple of 8": lambda: (_layer(k=36), gpu_like(1, 40, 36), None),
+    "input not 16-byte aligned": lambda: (_layer(), gpu_like(1, 40, 40)[..., 1:33], None),
+    "input row stride not a multiple of 8": lambda: (_layer(), gpu_like(1, 40, 36)[..., :32], None),
+    "input rows expanded": lambda: (_layer(), gpu_like(1, 1, 32).expand(1, 40, 32), None),
+    "weight rows expanded": lambda: (_expanded_weight(), gpu_like(1, 40, 32), None),
+    "input columns strided": lambda: (_layer(), gpu_like(1, 40, 64)[..., ::2], None),
+    "weight not 16-byte aligned": lambda: (_odd_weight(), gpu_like(1, 40, 32), None),
+    "bias not 16-byte aligned": lambda: (_odd_bias(), gpu_like(1, 40, 32), None),
+    "result not 16-byte aligned": lambda: (_layer(), gpu_like(1, 40, 32), gpu_like(1, 40, 72)[..., 1:65]),
+    "result row stride not a multiple of 8": lambda: (_layer(), gpu_like(1, 40, 32), gpu_like(1, 40, 68)[..., :64]),
+}
+
+
+@pytest.mark.parametrize("epilogue", ["gelu_tanh", "gate_residual"])
+@pytest.mark.parametrize("layout", LAYOUTS)
+def test_layouts_of_the_library_gemm_stay_with_it(fused, layout, epilogue):
+    linear, x, out = LAYOUTS[layout]()
+    rest = (gpu_like(1, 40, 64), gpu_like(1, 64)) if epilogue == "gate_residual" else ()
+    with torch.no_grad():
+        y = linear(x)
+        want = cpu_stand_ins.gelu_tanh(y) if epilogue == "gelu_tanh" else cpu_stand_ins.gate_residual(*rest, y)
+        got = kernels.linear_tail(linear, x, epilogue, *rest, out=out)
+    assert fused == [] and torch.equal(got, want)
