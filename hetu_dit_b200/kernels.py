@@ -542,8 +542,8 @@ def linear_fused(x, weight, bias=None, epilogue="bias", residual=None, gate=None
     if out is None:
         out = torch.empty(tuple(x.shape[:-1]) + (n,), dtype=x.dtype, device=x.device)
     rows_o, n_o, _, os_ = _rows_view(out)
-    if (rows_o, n_o) != (rows, n):
-        raise ValueError("out does not match (rows, N)")
+    if (rows_o, n_o) != (rows, n) or out.dtype != x.dtype:
+        raise ValueError("out does not match (rows, N) or x's dtype")
     a = _C.GemmArgs()
     a.dtype = _DTYPE_CODE[x.dtype]
     a.epilogue = {"bias": _C.GEMM_BIAS, "gelu_tanh": _C.GEMM_BIAS_GELU_TANH,
@@ -558,10 +558,10 @@ def linear_fused(x, weight, bias=None, epilogue="bias", residual=None, gate=None
     a.out, a.ldo = out.data_ptr(), os_
     if epilogue == "gate_residual":
         rows_r, n_r, _, rs = _rows_view(residual)
-        if (rows_r, n_r) != (rows, n):
-            raise ValueError("residual does not match (rows, N)")
-        if gate.dim() != 2 or gate.shape[1] != n or gate.stride(1) != 1 or rows % gate.shape[0] != 0:
-            raise ValueError("gate must be (B, N) with rows a multiple of B")
+        if (rows_r, n_r) != (rows, n) or residual.dtype != x.dtype:
+            raise ValueError("residual does not match (rows, N) or x's dtype")
+        if gate.dim() != 2 or gate.shape[1] != n or gate.stride(1) != 1 or rows % gate.shape[0] != 0 or gate.dtype != x.dtype:
+            raise ValueError("gate must be (B, N) of x's dtype with rows a multiple of B")
         a.residual, a.ldr = residual.data_ptr(), rs
         a.gate, a.gate_batch_stride = gate.data_ptr(), gate.stride(0)
         a.rows_per_batch = rows // gate.shape[0]
@@ -707,8 +707,8 @@ def linear_tail(linear, x, epilogue, residual=None, gate=None, out=None):
     batch and it pays, else as the call of `linear` plus hdit_gelu_tanh / hdit_gate_residual."""
     fusable = (epilogue in FUSED_LINEAR_TAILS and can_group_linears([x], [linear]) and _even_rows(x)
                and FUSED_LINEAR_MIN_ROWS <= x.shape[0] * x.shape[1] <= FUSED_LINEAR_MAX_ROWS
-               and (out is None or (_even_rows(out) and _aligned(out))) and (residual is None or _even_rows(residual))
-               and (gate is None or gate.stride(-1) == 1)
+               and _tail_fits(x, linear.weight.shape[0], residual, gate, out)
+               and all(t is None or _even_rows(t) for t in (residual, out))
                and _group_pays(((x.shape[0] * x.shape[1], linear.weight.shape[0]),), x.shape[2]))
     if fusable:
         return linear_fused(x, linear.weight, linear.bias, epilogue, residual=residual, gate=gate, out=out)
@@ -725,6 +725,17 @@ def _aligned(x):
     elements)."""
     (B, _, dim), (sb, ss, sk) = x.shape, x.stride()
     return sk == 1 and ss >= dim and ss % 8 == 0 and (B == 1 or sb % 8 == 0) and x.data_ptr() % 16 == 0
+
+
+def _tail_fits(x, n, residual, gate, out=None):
+    """Whether the kernel takes these with an (B, S, N) output for input x: residual and result of that shape and gate
+    (B, N), of x's type, on its device, aligned. What it does not take, gate_residual() takes or refuses by itself."""
+    shape = (x.shape[0], x.shape[1], n)
+    for t in (residual, out):
+        if t is not None and (tuple(t.shape) != shape or t.dtype != x.dtype or t.device != x.device or not _aligned(t)):
+            return False
+    return gate is None or (tuple(gate.shape) == (shape[0], n) and gate.dtype == x.dtype and gate.device == x.device and
+                            gate.stride(1) == 1 and gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0)
 
 
 def can_group_linears(xs, linears):
@@ -810,11 +821,8 @@ def try_linear_tails(specs):
     items = []
     for linear, x, epilogue, *rest in specs:
         residual, gate = rest if rest else (None, None)
-        if residual is not None:
-            aligned = residual.data_ptr() % 16 == 0 and gate.data_ptr() % 16 == 0 and \
-                all(v % 8 == 0 for v in (residual.stride(0), residual.stride(1), gate.stride(0)))
-            if not aligned or residual.stride(2) != 1 or gate.stride(-1) != 1 or residual.dtype != x.dtype or gate.dtype != x.dtype:
-                return None
+        if not _tail_fits(x, linear.weight.shape[0], residual, gate):
+            return None
         items.append(Lin(x, linear, epilogue, residual=residual, gate=gate))
     return linear_group(items) if use_linear_group(items) else None
 

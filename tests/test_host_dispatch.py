@@ -205,3 +205,44 @@ def test_layouts_of_the_library_gemm_stay_with_it(fused, layout, epilogue):
         want = cpu_stand_ins.gelu_tanh(y) if epilogue == "gelu_tanh" else cpu_stand_ins.gate_residual(*rest, y)
         got = kernels.linear_tail(linear, x, epilogue, *rest, out=out)
     assert fused == [] and torch.equal(got, want)
+
+
+# residuals and gates that gate_residual() takes or refuses by itself, and the fused kernel would not take or would misread
+TAILS = {
+    "residual in 32 bits": lambda: (gpu_like(2, 40, 64, dtype=torch.float32), gpu_like(2, 64)),
+    "gate in 32 bits": lambda: (gpu_like(2, 40, 64), gpu_like(2, 64, dtype=torch.float32)),
+    "residual not 16-byte aligned": lambda: (gpu_like(2, 40, 72)[..., 1:65], gpu_like(2, 64)),
+    "gate with a row between": lambda: (gpu_like(2, 40, 64), gpu_like(2, 1, 64)),
+    "residual rows expanded": lambda: (gpu_like(1, 1, 64).expand(2, 40, 64), gpu_like(2, 64)),
+    "gate of one row for two": lambda: (gpu_like(2, 40, 64), gpu_like(1, 64)),
+    "residual of another shape": lambda: (gpu_like(1, 80, 64), gpu_like(2, 64)),
+    "residual on the host": lambda: (torch.zeros(2, 40, 64, dtype=torch.bfloat16), gpu_like(2, 64)),
+}
+
+
+@pytest.mark.parametrize("tail", TAILS)
+def test_tails_of_the_separate_kernel_stay_with_it(fused, monkeypatch, tail):
+    """Residuals and gates that the separate kernel takes, or refuses, go there and not to the fused kernel."""
+    res, gate = TAILS[tail]()
+    if tail == "residual on the host":
+        monkeypatch.setattr(OnGpu, "device", property(lambda self: torch.device("cuda", 0)))
+        monkeypatch.setattr(torch.nn.Parameter, "device", property(lambda self: torch.device("cuda", 0)), raising=False)
+    seen = []
+    monkeypatch.setattr(kernels, "gate_residual", lambda r, g, y, out=None: seen.append((r, g)) or y)
+    linear, x = _layer(), gpu_like(2, 40, 32)
+    with torch.no_grad():
+        kernels.linear_tail(linear, x, "gate_residual", res, gate)
+        kernels.linear_tails([(linear, x, "gate_residual", res, gate)] * 2)
+    assert fused == [] and len(seen) == 3 and all(r is res and g is gate for r, g in seen)
+
+
+@pytest.mark.parametrize("wrong", ["residual", "gate", "out"])
+def test_fused_kernel_refuses_other_types_than_its_own(lib, wrong):
+    """The kernel reads and writes 16-bit elements: a 32-bit residual, gate or result would be misread."""
+    x = gpu_like(1, 40, 32)
+    x = x.as_subclass(type("OnGpu0", (OnGpu,), {"device": property(lambda self: torch.device("cuda", 0))}))
+    kw = {"residual": gpu_like(1, 40, 64), "gate": gpu_like(1, 64), "out": gpu_like(1, 40, 64)}
+    kw[wrong] = kw[wrong].float()
+    with pytest.raises(ValueError, match="dtype"):
+        kernels.linear_fused(x, gpu_like(64, 32), None, "gate_residual", **kw)
+    assert lib.calls == []
