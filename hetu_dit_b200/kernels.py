@@ -770,6 +770,23 @@ def can_group_linears(xs, linears):
     return True
 
 
+def norm_rope_fits(x, head_dim, norms, rope):
+    """Whether the "norm_rope" epilogue of linear_group() takes these norms, (kind, weight, bias, eps) each, and rotary
+    tables (cos, sin) or None for input x. qk_norm_rope() takes more: LayerNorm of 128-wide heads, for which the epilogue
+    has no registers left, and tables of different lengths."""
+    if head_dim not in (64, 128):
+        return False
+    for kind, w, b, _ in norms:
+        if kind not in (1, 2) or (kind == 2 and head_dim != 64):
+            return False
+        for t in (w, b):
+            if t is not None and (t.dtype != x.dtype or t.device != x.device or t.numel() != head_dim or
+                                  not t.is_contiguous() or t.data_ptr() % 16):
+                return False
+    return rope is None or (rope[0].shape == rope[1].shape and rope[0].dim() == 2 and rope[0].shape[1] == head_dim and
+                            all(t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in rope))
+
+
 def _group_cost(shapes):
     """Time of one launch over the (rows, n) output shapes in units of one SM's work on a 128 x 128 block of output: waves
     of output tiles times the time of a tile, smallest over the kernel's tile shapes (the constants are the library's

@@ -51,26 +51,33 @@ def _norm_rope(attn, q, k, wq, wk, rope, row0, rope_seq_start=0):
 def _qkv(attn, streams, rope):
     """Q, K and V of one or two streams, normalised and rotated where the layer does that. streams: list of
     (x, projections, (norm_q, norm_k), ranges): ranges are (lo, hi, rotate, row0, rope_seq_start) row ranges of x, row
-    lo + rope_seq_start of a rotated range takes table row row0. One launch computes everything when
-    kernels.use_linear_group says so, else each projection is a library GEMM and norm + RoPE run in place after them.
+    lo + rope_seq_start of a rotated range takes table row row0. One launch computes everything when the kernel takes the
+    layers, norms and tables and kernels.use_linear_group says that it pays, else each projection is a library GEMM and
+    norm + RoPE run in place after them.
     Returns one [q, k, v] of (B, S, H, D) tensors per stream."""
     H, D = attn.heads, attn.head_dim
     linears = [p for _, projs, _, _ in streams for p in projs]
     if kernels.can_group_linears([x for x, _, _, _ in streams], linears):
-        items, outs = [], []
+        items, fits = [], True
         for x, projs, norms, ranges in streams:
-            bufs = [torch.empty((x.shape[0], x.shape[1], H * D), dtype=x.dtype, device=x.device) for _ in projs]
-            outs.append([_heads(b, attn) for b in bufs])
+            norms = [None if w is None else (w.kind, w.weight, getattr(w, "bias", None), w.eps) for w in norms]
+            tables = rope if any(r[2] for r in ranges) else None
+            fits = fits and ((tables is None and norms == [None, None]) or
+                             kernels.norm_rope_fits(x, D, [n for n in norms if n is not None], tables))
             for lo, hi, rotate, row0, seq_start in ranges:
-                for p, w, buf in zip(projs, (*norms, None), bufs):
-                    is_v = buf is bufs[2]
-                    norm = None if w is None else (w.kind, w.weight, getattr(w, "bias", None), w.eps)
-                    rp = (seq_start, row0) if rotate and not is_v else None
-                    ep = "bias" if norm is None and rp is None else "norm_rope"
-                    whole = lo == 0 and hi == x.shape[1]
-                    items.append(kernels.Lin(x if whole else x[:, lo:hi], p, ep, out=buf if whole else buf[:, lo:hi],
-                                             head_dim=D, norm=norm, rope=rp))
-        if kernels.use_linear_group(items):
+                part = x if lo == 0 and hi == x.shape[1] else x[:, lo:hi]
+                turn = (seq_start, row0) if rotate else None
+                for p, norm, rp in zip(projs, (*norms, None), (turn, turn, None)):
+                    items.append(kernels.Lin(part, p, "bias" if norm is None and rp is None else "norm_rope", head_dim=D,
+                                             norm=norm, rope=rp))
+        if fits and kernels.use_linear_group(items):
+            outs, at = [], iter(items)
+            for x, projs, _, ranges in streams:
+                bufs = [torch.empty((x.shape[0], x.shape[1], H * D), dtype=x.dtype, device=x.device) for _ in projs]
+                outs.append([_heads(b, attn) for b in bufs])
+                for lo, hi, *_ in ranges:
+                    for buf in bufs:
+                        next(at).out = buf if lo == 0 and hi == x.shape[1] else buf[:, lo:hi]
             cos, sin = rope if rope is not None else (None, None)
             kernels.linear_group(items, cos, sin)
             return outs

@@ -246,3 +246,77 @@ def test_fused_kernel_refuses_other_types_than_its_own(lib, wrong):
     with pytest.raises(ValueError, match="dtype"):
         kernels.linear_fused(x, gpu_like(64, 32), None, "gate_residual", **kw)
     assert lib.calls == []
+
+
+def _linear_group(items, cos=None, sin=None, **kw):
+    """linear_group() as its documentation has it, in torch."""
+    for it in items:
+        y = torch.nn.functional.linear(it.x, it.weight, it.bias)
+        if it.epilogue == "norm_rope":
+            kind, w, b, eps = it.norm or (0, None, None, 1e-6)
+            start, row0 = it.rope or (0, 0)
+            cpu_stand_ins.qk_norm_rope([(y.view(*y.shape[:2], -1, it.head_dim), w, kind, it.rope is not None, b)], eps=eps,
+                                       cos=cos, sin=sin, rope_seq_start=start, rope_row0=row0)
+        it.out = y if it.out is None else it.out.copy_(y)
+    return [it.out for it in items]
+
+
+def _attention(kind, head_dim, **norms):
+    from hetu_dit_b200.model_executor.models.shaped_dit import Attention, DiTShape
+    shape = DiTShape("tiny", 1, 1, 256, 256 // head_dim, head_dim, 64, 128, 96, True, None, False, qk_norm_kind=kind)
+    attn = Attention(shape, joint=False).to(torch.bfloat16)
+    gen = torch.Generator().manual_seed(head_dim)
+    for p in attn.parameters():
+        p.data.copy_(torch.randn(p.shape, generator=gen) * (0.1 if p.dim() == 2 else 0.3) + (1 if p.dim() == 1 else 0))
+    return attn
+
+
+def _tables(rows, head_dim):
+    ang = torch.randn(rows, head_dim // 2).repeat_interleave(2, -1)
+    return torch.cos(ang), torch.sin(ang)
+
+
+def _both_routes(monkeypatch, attn, ranges, rope, B=1, S=50):
+    """[q, k, v] by the grouped launch where it is taken and by the separate kernels, and whether it was taken."""
+    from hetu_dit_b200.model_executor.layers import attention_processor as ap
+    taken = []
+    monkeypatch.setattr(kernels, "linear_group", lambda *a, **kw: taken.append(1) or _linear_group(*a, **kw))
+    stream = [(gpu_like(B, S, 256), (attn.to_q, attn.to_k, attn.to_v), (attn.norm_q, attn.norm_k), ranges)]
+    with torch.no_grad():
+        (got,) = ap._qkv(attn, stream, rope)
+        monkeypatch.setattr(kernels, "FUSED_LINEAR", False)
+        (want,) = ap._qkv(attn, stream, rope)
+    return got, want, bool(taken)
+
+
+def _break_nothing(attn, rope):
+    return rope
+
+
+def _fp32_weight(attn, rope):
+    attn.norm_k.weight.data = attn.norm_k.weight.data.float()
+    return rope
+
+
+def _odd_norm_weight(attn, rope):
+    attn.norm_q.weight.data = torch.ones(attn.head_dim + 1, dtype=torch.bfloat16)[1:]
+    return rope
+
+
+def _longer_sines(attn, rope):
+    return rope[0], torch.cat([rope[1], rope[1]])
+
+
+@pytest.mark.parametrize("kind,head_dim,change,grouped", [
+    ("rms", 64, _break_nothing, True), ("rms", 128, _break_nothing, True), ("layer", 64, _break_nothing, True),
+    ("layer", 128, _break_nothing, False), ("rms", 64, _fp32_weight, False), ("layer", 64, _odd_norm_weight, False),
+    ("rms", 128, _longer_sines, False)])
+@pytest.mark.parametrize("ranges", [[(0, 50, True, 0, 0)], [(0, 50, True, 3, 17)], [(0, 9, False, 0, 0), (9, 50, True, 5, 0)]])
+def test_qkv_takes_the_grouped_launch_only_where_its_epilogue_can(fused, monkeypatch, kind, head_dim, change, grouped, ranges):
+    """LayerNorm of 128-wide heads, norm weights and tables that the epilogue does not take: the separate kernels, as for
+    all other layers that are not grouped. Where it is grouped the result is the same."""
+    attn = _attention(kind, head_dim)
+    got, want, taken = _both_routes(monkeypatch, attn, ranges, change(attn, _tables(60, head_dim)))
+    assert taken is grouped
+    for g, w in zip(got, want):
+        assert torch.equal(g, w)
