@@ -60,14 +60,16 @@ def _qkv(attn, streams, rope):
     if kernels.can_group_linears([x for x, _, _, _ in streams], linears):
         items, fits = [], True
         for x, projs, norms, ranges in streams:
-            norms = [None if w is None else (w.kind, w.weight, getattr(w, "bias", None), w.eps) for w in norms]
+            eps = norms[0].eps if norms[0] is not None else 1e-6  # as _norm_rope() has it
+            norms = [None if w is None else (w.kind, w.weight, getattr(w, "bias", None), eps) for w in norms]
             tables = rope if any(r[2] for r in ranges) else None
             fits = fits and ((tables is None and norms == [None, None]) or
                              kernels.norm_rope_fits(x, D, [n for n in norms if n is not None], tables))
             for lo, hi, rotate, row0, seq_start in ranges:
                 part = x if lo == 0 and hi == x.shape[1] else x[:, lo:hi]
                 turn = (seq_start, row0) if rotate else None
-                for p, norm, rp in zip(projs, (*norms, None), (turn, turn, None)):
+                own = norms if norms[0] is not None or rotate else [None, None]
+                for p, norm, rp in zip(projs, (*own, None), (turn, turn, None)):
                     items.append(kernels.Lin(part, p, "bias" if norm is None and rp is None else "norm_rope", head_dim=D,
                                              norm=norm, rope=rp))
         if fits and kernels.use_linear_group(items):

@@ -320,3 +320,19 @@ def test_qkv_takes_the_grouped_launch_only_where_its_epilogue_can(fused, monkeyp
     assert taken is grouped
     for g, w in zip(got, want):
         assert torch.equal(g, w)
+
+
+@pytest.mark.parametrize("norms", ["own eps", "K only", "Q only"])
+@pytest.mark.parametrize("rotate", [False, True])
+def test_qkv_normalises_the_same_on_both_routes(fused, monkeypatch, norms, rotate):
+    """One eps, Q's, serves both; K alone is normalised only beside a rotation."""
+    attn = _attention("rms", 64)
+    attn.norm_q.eps, attn.norm_k.eps = 0.5, 2.0
+    if norms == "K only":
+        attn.norm_q = None
+    if norms == "Q only":
+        attn.norm_k = None
+    got, want, taken = _both_routes(monkeypatch, attn, [(0, 50, rotate, 0, 0)], _tables(50, 64) if rotate else None)
+    assert taken
+    for g, w in zip(got, want):
+        assert torch.equal(g, w)
