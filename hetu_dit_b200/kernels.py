@@ -690,12 +690,18 @@ FUSED_LINEAR_MAX_ROWS = int(os.environ.get("HDIT_FUSED_LINEAR_MAX_ROWS", str(1 <
 _PLAIN_TENSORS = (torch.nn.Parameter, torch.Tensor)
 
 
+def is_plain(module, cls):
+    """Whether calling `module` runs cls.forward and nothing else, so that what it does may be done without the call: no
+    other class (an adapter, a quantised layer), no forward() put on the object, and no hook, of this module or of all
+    modules, that waits for the call."""
+    return type(module) is cls and not (module._forward_hooks or module._forward_pre_hooks or "forward" in module.__dict__ or
+                                        _all_modules._global_forward_hooks or _all_modules._global_forward_pre_hooks)
+
+
 def _is_plain_linear(linear):
-    """Whether calling `linear` is x @ weight.T + bias and nothing else, so that a kernel may be given its weight instead:
-    no other class (an adapter, a quantised layer), no forward() put on the object, no weight of a tensor class of its
-    own, and no hook, of this layer or of all modules, that waits for the call."""
-    if type(linear) is not torch.nn.Linear or linear._forward_hooks or linear._forward_pre_hooks or \
-            "forward" in linear.__dict__ or _all_modules._global_forward_hooks or _all_modules._global_forward_pre_hooks:
+    """Whether calling `linear` is x @ weight.T + bias and nothing else, so that a kernel may be given its weight instead: a
+    plain torch.nn.Linear without a weight of a tensor class of its own."""
+    if not is_plain(linear, torch.nn.Linear):
         return False
     w, b = linear.weight, linear.bias
     return type(w) in _PLAIN_TENSORS and (b is None or type(b) in _PLAIN_TENSORS)

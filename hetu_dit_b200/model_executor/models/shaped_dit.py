@@ -141,20 +141,24 @@ class FeedForward(nn.Module):
         return kernels.linear_tail(self.net[2], x, "gate_residual", residual=residual, gate=gate)
 
 
-def _hooked(ff):
-    """Whether a hook waits for the call of a wrapped MLP or of one of the modules in it."""
-    return any(m._forward_hooks or m._forward_pre_hooks for m in ff.modules())
+def _mlp_layers(ff):
+    """The two linear layers of a wrapped MLP, or None where something waits for the call of one of its other modules or
+    has taken its place: the MLP is called then."""
+    if not (kernels.is_plain(ff, _Wrapped) and kernels.is_plain(ff.module, FeedForward)):
+        return None
+    up, between, down = (ff.module.net[i] for i in range(3))
+    return (up.proj, down) if kernels.is_plain(up, _GELUProj) and kernels.is_plain(between, nn.Identity) else None
 
 
 def feed_forward_pair(ff, x, x_res, x_gate, ff_c, c, c_res, c_gate):
     """ff(x, x_res, x_gate), ff_c(c, c_res, c_gate): the two streams' wrapped MLPs layer by layer, both streams in one
     launch where that pays (kernels.linear_tails)."""
-    if _hooked(ff) or _hooked(ff_c):
+    layers, layers_c = _mlp_layers(ff), _mlp_layers(ff_c)
+    if layers is None or layers_c is None:
         return ff(x, residual=x_res, gate=x_gate), ff_c(c, residual=c_res, gate=c_gate)
-    ff, ff_c = ff.module, ff_c.module
-    x, c = kernels.linear_tails([(ff.net[0].proj, x, "gelu_tanh"), (ff_c.net[0].proj, c, "gelu_tanh")])
-    return kernels.linear_tails([(ff.net[2], x, "gate_residual", x_res, x_gate),
-                                 (ff_c.net[2], c, "gate_residual", c_res, c_gate)])
+    x, c = kernels.linear_tails([(layers[0], x, "gelu_tanh"), (layers_c[0], c, "gelu_tanh")])
+    return kernels.linear_tails([(layers[1], x, "gate_residual", x_res, x_gate),
+                                 (layers_c[1], c, "gate_residual", c_res, c_gate)])
 
 
 class RMSNormWeight(nn.Module):
@@ -364,11 +368,11 @@ class CogVideoXBlock(nn.Module):
         a = self.attn1(x, image_rotary_emb=rope, text_len=S_txt, token_offset=token_offset)
         hidden, context = self._gated(attn.to_out[0], a, S_txt, hidden, m1[2], context, m1[5])
         kernels.ln_modulate_pair(hidden, m2[0], m2[1], context, m2[3], m2[4], x_out=x[:, S_txt:], c_out=x[:, :S_txt])
-        if _hooked(self.ff):
+        layers = _mlp_layers(self.ff)
+        if layers is None:
             f = self.ff(x)
             return kernels.gate_residual(hidden, m2[2], f[:, S_txt:]), kernels.gate_residual(context, m2[5], f[:, :S_txt])
-        ff = self.ff.module
-        return self._gated(ff.net[2], ff.net[0](x), S_txt, hidden, m2[2], context, m2[5])
+        return self._gated(layers[1], kernels.linear_tail(layers[0], x, "gelu_tanh"), S_txt, hidden, m2[2], context, m2[5])
 
     @staticmethod
     def _gated(linear, x, S_txt, hidden, h_gate, context, c_gate):

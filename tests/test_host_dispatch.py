@@ -336,3 +336,75 @@ def test_qkv_normalises_the_same_on_both_routes(fused, monkeypatch, norms, rotat
     assert taken
     for g, w in zip(got, want):
         assert torch.equal(g, w)
+
+
+@pytest.fixture
+def block_of(fused, monkeypatch):
+    """Builds a block whose kernels are torch stand-ins and runs it on tensors that say they are on the GPU."""
+    from hetu_dit_b200.core.distributed import parallel_state as ps
+    from hetu_dit_b200.core.resource_manager.cache_manager import reset_cache_manager
+    from hetu_dit_b200.model_executor.models.shaped_dit import CogVideoXBlock, DiTShape, JointBlock
+    ps.destroy_model_parallel()
+    reset_cache_manager()
+    for name in ("attn_fwd", "ln_modulate"):
+        monkeypatch.setattr(kernels, name, getattr(cpu_stand_ins, name))
+    monkeypatch.setattr(kernels, "ln_modulate_pair", lambda x, xs, xc, c, cs, cc, eps=1e-6, x_out=None, c_out=None: (
+        kernels.ln_modulate(x, xs, xc, eps, x_out), kernels.ln_modulate(c, cs, cc, eps, c_out)))
+    monkeypatch.setattr(kernels, "linear_group", _tails_group)
+    monkeypatch.setattr(kernels, "linear_fused", lambda x, w, b, epilogue, **kw: _tails_group([_item(x, w, b, epilogue, **kw)])[0])
+
+    def build(kind):
+        torch.manual_seed(5)
+        shape = DiTShape("tiny", 1, 0, 128, 2, 64, 64, 128, 96, True, None, False, block_kind=kind, temb_dim=128)
+        block = (JointBlock if kind == "mmdit" else CogVideoXBlock)(shape).to(torch.bfloat16)
+        x, c, temb = gpu_like(1, 40, 128), gpu_like(1, 33, 128), gpu_like(1, 128)
+
+        def run():
+            with torch.no_grad():
+                return block(x, c, temb, None)
+        return block, run
+    return build
+
+
+def _item(x, weight, bias, epilogue, residual=None, gate=None, out=None):
+    linear = torch.nn.Linear(8, 8)
+    linear.weight, linear.bias = weight, bias
+    return kernels.Lin(x, linear, epilogue, residual, gate, out)
+
+
+def _tails_group(items, cos=None, sin=None, **kw):
+    outs = _linear_group(items, cos, sin)
+    for i, it in enumerate(items):
+        if it.epilogue == "gelu_tanh":
+            outs[i] = cpu_stand_ins.gelu_tanh(outs[i], out=it.out)
+        if it.epilogue == "gate_residual":
+            outs[i] = cpu_stand_ins.gate_residual(it.residual, it.gate, outs[i])
+    return outs
+
+
+def _named(block, path):
+    return block.get_submodule(path) if path else block
+
+
+@pytest.mark.parametrize("kind", ["mmdit", "cogvideox"])
+@pytest.mark.parametrize("path", ["ff", "ff.module", "ff.module.net.0", "ff.module.net.1", "ff.module.net.2"])
+@pytest.mark.parametrize("how", ["hook", "class", "object"])
+def test_an_mlp_of_its_own_is_called(block_of, kind, path, how):
+    block, run = block_of(kind)
+    plain, called = run(), []
+    module = _named(block, path)
+    if how == "hook":
+        module.register_forward_hook(lambda *a: called.append(1))
+    else:
+        forward = module.forward
+
+        def own(*args, **kw):
+            called.append(1)
+            return forward(*args, **kw)
+        if how == "object":
+            module.forward = own
+        else:
+            module.__class__ = type("Own", (type(module),), {"forward": lambda self, *args, **kw: own(*args, **kw)})
+    for a, b in zip(run(), plain):
+        assert torch.allclose(a.float(), b.float(), atol=0.05, rtol=0.05)
+    assert called == [1]
