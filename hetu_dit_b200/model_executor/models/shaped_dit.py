@@ -274,8 +274,11 @@ class JointBlock(nn.Module):
         h, c = kernels.ln_modulate_pair(hidden, mod[0], mod[1], context, cmod[0], cmod[1])
         sp = (ps.get_sequence_parallel_world_size() > 1 or BRANCH_TEXT_TAIL_ALWAYS) and hidden.is_cuda
         # with fused linear layers the gated residual of the image stream rides on the attention's output
-        # projection (and the text stream's too, unless its tail runs on the branch stream below)
-        fuse = kernels.FUSED_LINEAR and "gate_residual" in kernels.FUSED_LINEAR_TAILS and hidden.is_cuda
+        # projection (and the text stream's too, unless its tail runs on the branch stream below). Only where nothing
+        # sees the attention module's result: a hook, or a processor of its own, is given the projected output alone
+        fuse = kernels.FUSED_LINEAR and "gate_residual" in kernels.FUSED_LINEAR_TAILS and hidden.is_cuda and \
+            kernels.is_plain(self.attn, _Wrapped) and kernels.is_plain(self.attn.module, Attention) and \
+            type(self.attn.module.processor) is JointAttnProcessor
         tails = ((hidden, mod[2]) if fuse else None, (context, cmod[2]) if fuse and not sp else None)
         a_img, a_txt = self.attn(h, encoder_hidden_states=c, image_rotary_emb=rope, token_offset=token_offset,
                                  text_len=text_total, text_offset=text_offset, tails=tails)

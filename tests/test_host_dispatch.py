@@ -408,3 +408,35 @@ def test_an_mlp_of_its_own_is_called(block_of, kind, path, how):
     for a, b in zip(run(), plain):
         assert torch.allclose(a.float(), b.float(), atol=0.05, rtol=0.05)
     assert called == [1]
+
+
+@pytest.mark.parametrize("path", ["attn", "attn.module"])
+def test_a_hook_on_attention_sees_the_projected_attention(block_of, monkeypatch, path):
+    """The residual is added outside the attention module, whatever the kernels fuse: a hook sees and changes the projected
+    attention output alone."""
+    block, run = block_of("mmdit")
+    plain = run()
+    seen = []
+    _named(block, path).register_forward_hook(lambda m, args, y: seen.append(y) or tuple(2 * t for t in y))
+    got = run()
+    monkeypatch.setattr(kernels, "FUSED_LINEAR", False)
+    want = run()
+    for a, b in zip(seen[0], seen[1]):
+        assert torch.equal(a, b)
+    for a, b, p in zip(got, want, plain):
+        assert torch.equal(a, b) and not torch.equal(a, p)
+
+
+def test_a_processor_of_its_own_need_not_know_the_residual(block_of, monkeypatch):
+    from hetu_dit_b200.model_executor.layers.attention_processor import JointAttnProcessor
+
+    class Own(JointAttnProcessor):
+        def __call__(self, attn, x, tails=None, **kw):
+            return tuple(2 * t for t in super().__call__(attn, x, **kw))
+
+    block, run = block_of("mmdit")
+    block.attn.module.processor = Own()
+    got = run()
+    monkeypatch.setattr(kernels, "FUSED_LINEAR", False)
+    for a, b in zip(got, run()):
+        assert torch.equal(a, b)
