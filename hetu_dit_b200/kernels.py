@@ -679,10 +679,11 @@ def linear_group(items, cos=None, sin=None, tile_m=0, tile_n=0, cta_pair=0, max_
 
 
 # Whether linear layers may run the fused tensor-core kernel (csrc/gemm_sm100.cu) instead of the library GEMM followed by
-# one-pass kernels, for which tails, and from / to how many rows on top of the rule in _group_pays(). HDIT_FUSED_LINEAR=0
-# turns the fused kernel off, HDIT_FUSED_LINEAR_TAILS=gelu_tanh fuses only that tail.
+# one-pass kernels, for which tails, and from / to how many rows (an input's rows count once, however many layers of a
+# launch read it) on top of the rule in _group_pays(). HDIT_FUSED_LINEAR=0 turns the fused kernel off,
+# HDIT_FUSED_LINEAR_TAILS=gelu_tanh fuses only that tail; "bias" and "norm_rope" are the Q, K, V projections.
 FUSED_LINEAR = os.environ.get("HDIT_FUSED_LINEAR", "1") == "1"
-FUSED_LINEAR_TAILS = set(os.environ.get("HDIT_FUSED_LINEAR_TAILS", "gelu_tanh,gate_residual").split(","))
+FUSED_LINEAR_TAILS = set(os.environ.get("HDIT_FUSED_LINEAR_TAILS", "bias,gelu_tanh,gate_residual,norm_rope").split(","))
 FUSED_LINEAR_MIN_ROWS = int(os.environ.get("HDIT_FUSED_LINEAR_MIN_ROWS", "0"))
 FUSED_LINEAR_MAX_ROWS = int(os.environ.get("HDIT_FUSED_LINEAR_MAX_ROWS", str(1 << 40)))
 
@@ -711,6 +712,8 @@ def linear_tail(linear, x, epilogue, residual=None, gate=None, out=None):
     """A torch.nn.Linear followed by its elementwise tail ("gelu_tanh", or "gate_residual" = residual +
     gate[:, None] * linear(x)), as one kernel when can_group_linears() allows it, rows are evenly strided across the
     batch and it pays, else as the call of `linear` plus hdit_gelu_tanh / hdit_gate_residual."""
+    if epilogue not in ("gelu_tanh", "gate_residual"):
+        raise ValueError(epilogue)
     fusable = (epilogue in FUSED_LINEAR_TAILS and can_group_linears([x], [linear]) and _even_rows(x)
                and FUSED_LINEAR_MIN_ROWS <= x.shape[0] * x.shape[1] <= FUSED_LINEAR_MAX_ROWS
                and _tail_fits(x, linear.weight.shape[0], residual, gate, out)
@@ -721,9 +724,7 @@ def linear_tail(linear, x, epilogue, residual=None, gate=None, out=None):
     y = linear(x)
     if epilogue == "gelu_tanh":
         return gelu_tanh(y, out=y if out is None else out)
-    if epilogue == "gate_residual":
-        return gate_residual(residual, gate, y, out=out)
-    raise ValueError(epilogue)
+    return gate_residual(residual, gate, y, out=out)
 
 
 def _aligned(x):
@@ -824,16 +825,16 @@ def _group_pays(shapes, k):
 
 def use_linear_group(items):
     """Whether one linear_group() launch beats separate library GEMMs and tail kernels."""
-    shapes, rows = [], 0
+    shapes, inputs = [], {}
     for it in items:
-        if it.epilogue in ("gelu_tanh", "gate_residual") and it.epilogue not in FUSED_LINEAR_TAILS:
+        if it.epilogue not in FUSED_LINEAR_TAILS:
             return False
         B, S, k = it.x.shape
         n = it.weight.shape[0]
         shapes += [(B * S, n)] if it._even() else [(S, n)] * B
-        rows += B * S
-    return 1 <= len(shapes) <= _C.MAX_LINEAR_ITEMS and FUSED_LINEAR_MIN_ROWS <= rows <= FUSED_LINEAR_MAX_ROWS and \
-        _group_pays(tuple(shapes), k)
+        inputs[id(it.x)] = B * S
+    return 1 <= len(shapes) <= _C.MAX_LINEAR_ITEMS and \
+        FUSED_LINEAR_MIN_ROWS <= sum(inputs.values()) <= FUSED_LINEAR_MAX_ROWS and _group_pays(tuple(shapes), k)
 
 
 def try_linear_tails(specs):

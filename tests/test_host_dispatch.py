@@ -440,3 +440,22 @@ def test_a_processor_of_its_own_need_not_know_the_residual(block_of, monkeypatch
     monkeypatch.setattr(kernels, "FUSED_LINEAR", False)
     for a, b in zip(got, run()):
         assert torch.equal(a, b)
+
+
+def test_switches_hold_for_grouped_layers_too(fused, monkeypatch):
+    """The row limits count an input's rows once, however many layers read it; a tail that is not named is not fused."""
+    attn = _attention("rms", 64)
+    for name, value in (("FUSED_LINEAR_MIN_ROWS", 51), ("FUSED_LINEAR_MAX_ROWS", 49), ("FUSED_LINEAR_TAILS", {"gelu_tanh"}),
+                        ("FUSED_LINEAR_TAILS", {"bias", "gelu_tanh", "gate_residual"})):
+        with monkeypatch.context() as m:
+            m.setattr(kernels, name, value)
+            assert not _both_routes(m, attn, [(0, 50, True, 0, 0)], _tables(50, 64))[2], (name, value)
+    monkeypatch.setattr(kernels, "FUSED_LINEAR_MIN_ROWS", 50)
+    monkeypatch.setattr(kernels, "FUSED_LINEAR_MAX_ROWS", 50)
+    with torch.no_grad():
+        kernels.linear_tails([(_layer(), gpu_like(1, n, 32), "gate_residual", gpu_like(1, n, 64), gpu_like(1, 64))
+                              for n in (17, 33)])
+        with pytest.raises(ValueError):
+            kernels.linear_tail(_layer(), gpu_like(1, 50, 32), "bias")  # a name of the switch, not a tail
+    assert fused == ["linear_group"]
+    assert _both_routes(monkeypatch, attn, [(0, 9, False, 0, 0), (9, 50, True, 0, 0)], _tables(50, 64))[2]
