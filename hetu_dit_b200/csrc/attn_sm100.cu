@@ -220,12 +220,14 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 }
 
 // 2^x for a pair of scores on the FMA pipe: x = n + f with n = round(x), f in [-0.5, 0.5]; 2^f by a degree-5
-// polynomial with constant term 1, fitted for the smallest largest relative error (9.1e-8; evaluated in fp32 at most
-// 1.7e-7, below the 2^-22 that ex2.approx is documented with), 2^n by adding n to the exponent field. Inputs below -126
-// (masked scores are -inf) clamp to 2^-126, and so does NaN: the row maximum carries NaN instead.
+// polynomial with constant term 1, fitted for a small largest relative error (1.08e-7 in exact arithmetic, at f = -0.5;
+// evaluated in fp32 at most 1.7e-7, below the 2^-22 that ex2.approx is documented with), 2^n by adding n to the exponent
+// field. Inputs below -127 (masked scores are -inf) clamp to -127, where f is 0, the polynomial exactly 1 and the
+// exponent field 0: the result is +0, the weight that ex2.approx.ftz gives such a score. Between -127 and -126 the
+// result is denormal and at most 2^-127 off. NaN clamps too: the row maximum carries it instead.
 __device__ __forceinline__ float2 ex2_poly2(float2 x) {
-  x.x = fmaxf(x.x, -126.0f);
-  x.y = fmaxf(x.y, -126.0f);
+  x.x = fmaxf(x.x, -127.0f);
+  x.y = fmaxf(x.y, -127.0f);
   const float2 magic = make_float2(12582912.0f, 12582912.0f);  // 1.5 * 2^23: the sum's low mantissa bits hold n
   const float2 t = __fadd2_rn(x, magic);
   const float2 r = __fadd2_rn(t, make_float2(-12582912.0f, -12582912.0f));

@@ -113,6 +113,21 @@ def test_special_values_reach_the_output(key, D, dtype):
 
 
 @pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("key", [0, 3, 4, 5, 6, 7, 70, 71, 127, 134, 135, 199])
+def test_a_key_far_below_the_maximum_weighs_nothing(key, D):
+    """A score more than 2^127 below the row's maximum has weight zero on every pipe that exponentiates, so that a value
+    near the type's largest does not reach the output."""
+    gen = torch.Generator().manual_seed(key + D)
+    q, k, v = (_mk((1, n, 2, D), torch.bfloat16, gen) for n in (140, 200, 200))
+    q[..., 0] = 40.0
+    k[:, key, :, 0] = -60.0
+    out, lse = _run([q], [k], [v], softmax_scale=1.0)
+    v[:, key] = 2.0 ** 127
+    got, lse2 = _run([q], [k], [v], softmax_scale=1.0)
+    assert torch.equal(got, out) and torch.equal(lse2, lse)
+
+
+@pytest.mark.parametrize("D", [64, 128])
 def test_partial_and_merge_modes(D):
     """Ring-style accumulation: PARTIAL_FIRST, PARTIAL_MERGE, MERGE_FINAL over KV blocks == one shot."""
     from hetu_dit_b200 import _C, kernels
