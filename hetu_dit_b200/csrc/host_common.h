@@ -49,7 +49,9 @@ cudaError_t launch_overlapped(void (*kernel)(KernelArgs...), dim3 grid, dim3 blo
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = cluster > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Args&&>(args)...);
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, static_cast<Args&&>(args)...);
+  if (err != cudaSuccess) (void)cudaGetLastError();  // reported here, not once more by whoever launches next
+  return err;
 }
 
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
