@@ -193,17 +193,38 @@ def test_linear_group_argument_errors():
             kernels.linear_group([kernels.Lin(x, lin)] * 9)
 
 
-def test_linear_group_on_row_slices_of_a_batch():
-    """Rows that are a slice of every batch entry (the image and text rows of one attention output): same result as on
-    contiguous copies, nothing written outside."""
-    from hetu_dit_b200 import kernels
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_linear_group_on_row_slices_of_a_batch(dtype):
+    """Rows that are a slice of every batch entry (the image and text rows of one attention output): one launch with an item
+    per entry, the bits of a call on contiguous copies, nothing written outside the slices."""
+    from hetu_dit_b200 import _C, kernels
     gen = torch.Generator().manual_seed(9)
-    x = torch.randn(2, 300, 256, generator=gen).to(torch.bfloat16).to(DEV)
-    lin = torch.nn.Linear(256, 192, device=DEV, dtype=torch.bfloat16)
-    gate = torch.randn(2, 192, generator=gen).to(torch.bfloat16).to(DEV)
-    res = [torch.randn(2, n, 192, generator=gen).to(torch.bfloat16).to(DEV) for n in (223, 77)]
+
+    def mk(*shape):
+        return torch.randn(*shape, generator=gen).to(dtype).to(DEV)
+
+    x, gate, w = mk(2, 300, 256), mk(2, 192), (1 + 0.2 * mk(64))
+    lin = torch.nn.Linear(256, 192, device=DEV, dtype=dtype)
+    cos, sin = (torch.randn(300, 64, generator=gen).to(DEV) for _ in range(2))
+    kw = dict(tile_m=128, tile_n=128)  # one tile shape on both sides: one order of sums
+    gated, normed = (torch.full((2, 320, 208), 7.0, dtype=dtype, device=DEV) for _ in range(2))
+    res = mk(2, 320, 192)
     with torch.no_grad():
-        parts = [x[:, :223], x[:, 223:]]
-        got = kernels.linear_tails([(lin, p, "gate_residual", r, gate) for p, r in zip(parts, res)])
-        for g, p, r in zip(got, parts, res):
-            _check(g, _want(p.contiguous(), lin.weight, lin.bias, "gate_residual", r, gate))
+        items, want = [], []
+        for lo, hi, rope in ((0, 223, None), (223, 300, (13, 4))):
+            xs, whole = x[:, lo:hi], x[:, lo:hi].contiguous()
+            items += [kernels.Lin(xs, lin, "gate_residual", residual=res[:, 5 + lo:5 + hi], gate=gate, out=gated[:, 5 + lo:5 + hi, 8:200]),
+                      kernels.Lin(xs, lin, "norm_rope", head_dim=64, norm=(1, w, None, 1e-6), rope=rope, out=normed[:, 5 + lo:5 + hi, 8:200])]
+            want += kernels.linear_group([
+                kernels.Lin(whole, lin, "gate_residual", residual=res[:, 5 + lo:5 + hi].contiguous(), gate=gate),
+                kernels.Lin(whole, lin, "norm_rope", head_dim=64, norm=(1, w, None, 1e-6), rope=rope)], cos, sin, **kw)
+            _check(want[-2], _want(whole, lin.weight, lin.bias, "gate_residual", res[:, 5 + lo:5 + hi], gate))
+        before = kernels.launch_count()
+        got = kernels.linear_group(items, cos, sin, **kw)
+        assert kernels.launch_count() == before + 1
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    for buf, own in ((gated, (want[0], want[2])), (normed, (want[1], want[3]))):
+        untouched = torch.full_like(buf, 7.0)
+        untouched[:, 5:305, 8:200] = torch.cat(own, dim=1)
+        assert torch.equal(buf, untouched)
+    assert _C.device_status(0, clear=True)[0] == 0

@@ -232,6 +232,43 @@ def test_graph_replay_matches_eager_bit_for_bit():
     assert _C.device_status(0, clear=True)[0] == 0
 
 
+def test_layer_norm_of_wide_heads_takes_the_separate_kernel(monkeypatch):
+    """LayerNorm over 128-wide heads is not in the linear kernel's epilogue: such a model runs, with the result it has
+    with no fused linear layers."""
+    from hetu_dit_b200 import kernels
+    from hetu_dit_b200.model_executor.models.shaped_dit import DiTShape, ShapedDiT
+    args, kw, grid = TINY["flux"]
+    shape = DiTShape(*args, **kw, qk_norm_kind="layer")
+    model = ShapedDiT(shape).to(DEV).init_weights(seed=5, std=0.05).bfloat16()
+    lat, txt, pooled, t, g = (x.to(DEV) for x in _inputs(shape, grid[0] * grid[1], 33, seed=1))
+    with torch.no_grad():
+        got = model(lat, txt, pooled, t, g, grid=grid).clone()
+        monkeypatch.setattr(kernels, "FUSED_LINEAR", False)
+        want = model(lat, txt, pooled, t, g, grid=grid)
+    cos, rel = oa.cosine_and_max_rel(got.cpu(), want.cpu())
+    assert cos >= 0.9999 and rel <= 2e-2, (cos, rel)
+
+
+@pytest.mark.parametrize("kind", ["flux", "sd3"])
+def test_text_tail_on_the_branch_stream_replays_bit_for_bit(kind, monkeypatch):
+    """The text stream's tail on the second stream, captured: kernels on both streams start early and wait for the kernel
+    before them in their stream and for the events between the streams. Replays give the eager step's bits."""
+    from hetu_dit_b200 import _C
+    from hetu_dit_b200.model_executor.models import shaped_dit
+    shape, grid = tiny_shape(kind)
+    model = shaped_dit.ShapedDiT(shape).to(DEV).init_weights(seed=5, std=0.05).bfloat16()
+    lat, txt, pooled, t, g = (x.to(DEV) for x in _inputs(shape, grid[0] * grid[1], 33, seed=1))
+    with torch.no_grad():
+        one_stream = model(lat, txt, pooled, t, g, grid=grid).clone()
+        monkeypatch.setattr(shaped_dit, "BRANCH_TEXT_TAIL_ALWAYS", True)
+        eager = model(lat, txt, pooled, t, g, grid=grid).clone()
+        for _ in range(8):
+            assert torch.equal(model.forward_graphed(lat, txt, pooled, t, g, grid=grid), eager)
+    cos, rel = oa.cosine_and_max_rel(eager.cpu(), one_stream.cpu())
+    assert cos >= 0.9999 and rel <= 2e-2, (cos, rel)
+    assert _C.device_status(0, clear=True)[0] == 0
+
+
 def test_pipeline_whole_image_steps_replay_from_a_graph():
     """The SD3-shaped pipeline without pipeline patches replays its stage forward from a CUDA graph: same latents
     as with the graph switched off, bit for bit, over several steps and two requests."""
