@@ -356,20 +356,21 @@ def test_copy_pieces_of_very_different_sizes():
 
 
 def test_a_failed_launch_leaves_no_error_behind():
-    """A launch that the runtime refuses (on the legacy stream while this thread captures another one) is reported by the
-    call that made it and by no later one: the runtime's last error, which the next launch looks at, is cleared."""
+    """A launch that the runtime refuses (on the legacy stream while a stream that waits for it is captured) is reported by
+    the call that made it and by no later one: the runtime's last error, which the next launch looks at, is cleared."""
     import ctypes
 
     from hetu_dit_b200 import _C
     x = torch.zeros(1, 8, dtype=torch.bfloat16, device="cuda:0")
-    stream, graph = torch.cuda.Stream(), ctypes.c_void_p()
     cudart = ctypes.CDLL("libcudart.so.12")
+    stream, graph = ctypes.c_void_p(), ctypes.c_void_p()
     torch.cuda.synchronize()
-    handle = ctypes.c_void_p(stream.cuda_stream)
-    assert cudart.cudaStreamBeginCapture(handle, 0) == 0
+    assert cudart.cudaStreamCreate(ctypes.byref(stream)) == 0
+    assert cudart.cudaStreamBeginCapture(stream, 0) == 0
     rc = _C.lib().hdit_gelu_tanh(_C.HDIT_BF16, x.data_ptr(), x.data_ptr(), 1, 8, 8, 8, None)
     left = cudart.cudaGetLastError()
-    cudart.cudaStreamEndCapture(handle, ctypes.byref(graph))  # the capture is void
+    cudart.cudaStreamEndCapture(stream, ctypes.byref(graph))  # the capture is void
     cudart.cudaGetLastError()
+    assert cudart.cudaStreamDestroy(stream) == 0
     assert rc == _C.HDIT_ERR_CUDA and left == 0
     assert torch.equal(x + 1, torch.ones_like(x))
