@@ -913,8 +913,8 @@ struct ScatterParams {
 // NS > 0 fixes the split count at compile time: all partial rows and LSEs of a row are then requested
 // before any of them is used (the kernel is latency-bound: 17 MB per call at the Flux shape).
 template <int D, bool FP16, int NS>
-__global__ void __launch_bounds__(256) attn_combine_kernel(const float* __restrict__ part_out,
-                                                          const float* __restrict__ part_lse, int n_split,
+__global__ void __launch_bounds__(256) attn_combine_kernel(const float* part_out,
+                                                          const float* part_lse, int n_split,
                                                           long long acc_stride, long long lse_stride, int batch,
                                                           long long sq, int heads, void* out, long long out_sb,
                                                           long long out_ss, long long out_sh, float* lse,

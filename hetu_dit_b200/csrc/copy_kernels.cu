@@ -35,6 +35,7 @@ struct PieceTable {
   Piece p[kMaxPieces];
   int n;
   unsigned ctas;
+  bool early;  // the next kernel may start before this one has finished
 };
 
 __device__ __forceinline__ void row_offsets(const Piece& pc, unsigned long long row, long long& so, long long& dof) {
@@ -90,7 +91,7 @@ __device__ __forceinline__ void copy_piece(const Piece& pc, long long tid, long 
 }
 
 __global__ void __launch_bounds__(kCopyThreads) copy_pieces_kernel(const __grid_constant__ PieceTable tab) {
-  grid_dependency_release();
+  if (tab.early) grid_dependency_release();
   grid_dependency_wait();
   int lo = 0, hi = tab.n;  // the last piece that starts at or before this CTA
   while (hi - lo > 1) {
@@ -123,11 +124,8 @@ int pick_vec(const hdit_copy_piece& d) {
   return 1;
 }
 
-}  // namespace
-}  // namespace hdit
-
-extern "C" int hdit_copy_pieces(const hdit_copy_piece* pieces, int64_t n, void* stream) {
-  using namespace hdit;
+// early: the copied bytes are activations, which no kernel reads by the read-only path (see launch_overlapped()).
+int copy_pieces(const hdit_copy_piece* pieces, int64_t n, bool early, void* stream) {
   if (n < 0 || (n > 0 && pieces == nullptr)) return set_error(HDIT_ERR_BAD_ARG, "bad piece list");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int64_t i = 0;
@@ -169,9 +167,17 @@ extern "C" int hdit_copy_pieces(const hdit_copy_piece* pieces, int64_t n, void* 
       ctas += static_cast<unsigned>((pc.n_outer * pc.rows * pc.row_bytes + per_cta - 1) / per_cta);
     }
     tab.ctas = ctas;
+    tab.early = early;
     HDIT_CUDA_OK(launch_overlapped(copy_pieces_kernel, dim3(ctas), dim3(kCopyThreads), 0, st, 1, tab));
   }
   return HDIT_OK;
+}
+
+}  // namespace
+}  // namespace hdit
+
+extern "C" int hdit_copy_pieces(const hdit_copy_piece* pieces, int64_t n, void* stream) {
+  return hdit::copy_pieces(pieces, n, false, stream);  // weights among them, when a plan switch re-slices them
 }
 
 extern "C" int hdit_kv_scatter(void* kv_cache, const void* new_k, const void* new_v, int64_t batch, int64_t cache_tokens,
@@ -194,5 +200,5 @@ extern "C" int hdit_kv_scatter(void* kv_cache, const void* new_k, const void* ne
     pc[i].dst_pitch = 2 * row_bytes;
     pc[i].row_bytes = row_bytes;
   }
-  return hdit_copy_pieces(pc, 2, stream);
+  return copy_pieces(pc, 2, true, stream);
 }

@@ -208,8 +208,8 @@ bool try_ln_warp(const LnSegs& segs, int dim, float eps, cudaStream_t st, cudaEr
 }
 
 template <bool FP16>
-__global__ void __launch_bounds__(256) gate_residual_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ gate,
-                                                           const uint16_t* __restrict__ y, uint16_t* __restrict__ out,
+__global__ void __launch_bounds__(256) gate_residual_kernel(const uint16_t* x, const uint16_t* gate,
+                                                           const uint16_t* y, uint16_t* out,
                                                            long long rows, int dim, long long rows_per_batch,
                                                            long long x_row_stride, long long y_row_stride,
                                                            long long out_row_stride, long long gate_batch_stride) {
@@ -252,7 +252,7 @@ __device__ __forceinline__ float gelu_tanh_f(float x) {
 // out[r, :] = gelu_tanh(x[r, :]); rows may be strided on both sides (e.g. the output is a column block of
 // a wider buffer). Two 16-byte loads in flight per thread.
 template <bool FP16>
-__global__ void __launch_bounds__(256) gelu_tanh_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ out,
+__global__ void __launch_bounds__(256) gelu_tanh_kernel(const uint16_t* x, uint16_t* out,
                                                        long long rows, int dim, long long x_row_stride,
                                                        long long out_row_stride) {
   grid_dependency_release();
@@ -306,11 +306,11 @@ namespace {
 // fp32 denoised = sample - product, derivative = (sample - denoised) / sigma, sample + derivative * dt, each
 // operation rounded on its own) and is rounded to the 16-bit type once.
 template <bool FP16>
-__global__ void __launch_bounds__(256) cfg_euler_step_kernel(const uint16_t* __restrict__ uncond,
-                                                            const uint16_t* __restrict__ cond,
-                                                            const uint16_t* __restrict__ sample, uint16_t* __restrict__ out,
-                                                            uint16_t* __restrict__ out2, long long n_vec, float guidance,
-                                                            const float* __restrict__ sigmas, int step) {
+__global__ void __launch_bounds__(256) cfg_euler_step_kernel(const uint16_t* uncond,
+                                                            const uint16_t* cond,
+                                                            const uint16_t* sample, uint16_t* out,
+                                                            uint16_t* out2, long long n_vec, float guidance,
+                                                            const float* sigmas, int step) {
   grid_dependency_release();
   grid_dependency_wait();
   const float sigma = sigmas[step];

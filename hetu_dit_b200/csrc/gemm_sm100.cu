@@ -39,6 +39,11 @@
 //                         the even CTA's barrier, and tcgen05.commit multicasts "stage consumed" / "accumulator
 //                         ready" to both CTAs. No TMA multicast is used.
 //
+// Biases, norm weights and rotary tables are read with __ldg(): parameters, which no kernel writes that lets another one
+// start before it has finished (host_common.h). Everything else, the gate among it, is read with plain loads. Behind plain
+// loads the bias waits for the stores to the staging buffer around it: Q, K, V of 2 x (1024 + 77) rows, hidden 1536, 32.6 ->
+// 38.0 us; eight of them in registers ahead of the stores cost the larger shapes more (2 x (4096 + 333) rows 94.3 -> 104.8).
+//
 // The fused tails remove one full read + write of the activation per layer (GELU) or a read of it plus a write
 // (gated residual) that separate elementwise kernels would spend on HBM.
 //
@@ -314,8 +319,7 @@ __device__ __forceinline__ float2 head_stats(const GemmItem& p, uint32_t taddr, 
 // part (n is a multiple of 64 here, so a piece lies inside or outside as a whole). Four rows' table entries are requested
 // before the first is used.
 template <bool FP16>
-__device__ __forceinline__ void norm_rope_rows(const GemmItem& p, const float* __restrict__ cos_tab,
-                                               const float* __restrict__ sin_tab, const uint8_t* staging, float2 stats,
+__device__ __forceinline__ void norm_rope_rows(const GemmItem& p, const float* cos_tab, const float* sin_tab, const uint8_t* staging, float2 stats,
                                                long long row0, long long batch0, long long next_batch_row, int col) {
   const int lane = threadIdx.x & 31;
   const int sub_row = lane >> 3, chunk = lane & 7;
@@ -632,9 +636,9 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
               xv[i] = (row < im.M) ? *reinterpret_cast<const uint4*>(im.residual + row * im.ldr + col) : make_uint4(0, 0, 0, 0);
             }
             // the 32 rows of this warp lie in at most two batch entries
-            const uint4 g_lo = __ldg(reinterpret_cast<const uint4*>(im.gate + batch0 * im.gate_batch_stride + col));
+            const uint4 g_lo = *reinterpret_cast<const uint4*>(im.gate + batch0 * im.gate_batch_stride + col);
             const uint4 g_hi = (row0 + 31 >= next_batch_row && next_batch_row < im.M)
-                                   ? __ldg(reinterpret_cast<const uint4*>(im.gate + (batch0 + 1) * im.gate_batch_stride + col))
+                                   ? *reinterpret_cast<const uint4*>(im.gate + (batch0 + 1) * im.gate_batch_stride + col)
                                    : g_lo;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {

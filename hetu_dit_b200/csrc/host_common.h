@@ -29,7 +29,11 @@ int32_t* device_status_ptr();
 // Launch in stream order, but let the grid start while the kernel before it in the stream drains: its CTAs are
 // scheduled, set up their barriers and tensor memory and then stand in grid_dependency_wait() until that kernel has
 // completed and its writes are visible. Every kernel launched this way calls grid_dependency_wait() in all threads before
-// its first access to global memory, and grid_dependency_release() so that the kernel after it may do the same.
+// its first access to global memory, and grid_dependency_release() so that the kernel after it may do the same. What the
+// kernel before it writes changes while this kernel already runs, so none of them reads activations by the read-only path
+// (__ldg(), const __restrict__ parameters), which promises data that is constant for the kernel's lifetime. Parameters of a
+// layer may be read by it: copy_pieces_kernel, the one kernel here that writes them, lets the next one start only when it
+// has finished.
 // Measured: PipeFusion patch (scatter + attention) 127.7 -> 119.5 us, SD3-shaped step 20.8 -> 20.3 ms, SD3-shaped request
 // 42.0 -> 41.3 ms, a 453 MB re-slice 74.3 -> 72.1 us a call.
 template <typename... KernelArgs, typename... Args>

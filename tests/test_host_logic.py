@@ -869,3 +869,24 @@ def test_adjust_pipeline_coroutine_takes_the_reference_argument_forms():
     assert c.calls[3][1]["peer_directories"] == {1: {}} and c.calls[0][1]["peer_directories"] is None
     with pytest.raises(TypeError):
         asyncio.run(c.adjust_pipeline(transformer=gpu, **ranges))
+
+
+def test_kernels_that_start_early_read_activations_by_plain_loads():
+    """A kernel that starts before its predecessor has finished writing may not promise that what the predecessor writes is
+    constant for its lifetime: no ld.global.nc and no __restrict__ pointers, __ldg() for a layer's parameters alone, which
+    only the piece copies write; those let no kernel start early. And every kernel waits once."""
+    csrc = os.path.join(ROOT, "hetu_dit_b200", "csrc")
+    code = {}
+    for name in sorted(os.listdir(csrc)):
+        if name.endswith((".cu", ".cuh")):
+            with open(os.path.join(csrc, name)) as f:
+                code[name] = re.sub(r"//[^\n]*", "", f.read())
+    for name, text in code.items():
+        assert not re.search(r"ld\.global\.nc|__restrict__", text), name
+        for operand in re.findall(r"__ldg\(reinterpret_cast<const \w+\*>\(([\w.]+)|__ldg", text):
+            assert operand in ("p.bias", "im.bias", "p.norm_weight", "p.norm_bias", "cos_tab", "sin_tab"), (name, operand)
+        if "launch_overlapped(" in text:
+            n = len(re.findall(r"__global__", text))
+            assert text.count("grid_dependency_wait();") == text.count("grid_dependency_release();") == n, name
+    assert "if (tab.early) grid_dependency_release();" in code["copy_kernels.cu"]
+    assert "hdit::copy_pieces(pieces, n, false, stream)" in code["copy_kernels.cu"]
