@@ -9,8 +9,8 @@
 //                                (one elected thread; behind elect.sync it runs a few MMAs ahead of the tensor
 //                                pipe, so its barrier polls overlap with MMAs. Behind `lane == 0` every MMA took it 61
 //                                cycles to issue, which left the pipe idle at each hand-shake and ran the 128x64
-//                                P V of head_dim 64 at half rate: 250 -> 226 us at 24 heads x 4608 tokens x 128,
-//                                40.9 -> 37.6 ms at 6 heads x 119 k)
+//                                P V of head_dim 64 at half rate: 10 % of the time at 24 heads x 4608 tokens x 128,
+//                                8 % at 6 heads x 119 k)
 //   warps 10-11 idle           : complete the third warpgroup so registers can be handed over
 //                                (setmaxnreg: 72 per thread there, 216 for the softmax threads;
 //                                72 + 2 * 216 = 3 * 168, the pool the CTA was launched with --
@@ -61,8 +61,10 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 units
 // P of a KV block is handed to the MMA thread in two parts, the first after this many of its four 32-column chunks: the
 // first half of P V runs while the second half is exponentiated, which takes those MMAs off the chain softmax -> P V ->
 // next Q K^T that bounds a tile (3294 -> 3057 cycles per KV block pair at head_dim 128, 2048 of them MMAs). Measured
-// against one hand-over: 24 heads x 4608 x 128 266 -> 240 us, 3 heads 44.9 -> 39.2 us, 29.7 k x 119 k tokens 10.06 -> 9.3
-// ms; after one or three chunks it is 251 / 241 us. Four hand-overs cost more in waits than they overlap.
+// against one hand-over, in turn on one box: 24 heads x 4608 x 128 10 % less (after one chunk 6 %, after three 9 %), 3 heads
+// 13 %, 6 heads of 29.7 k x 119 k tokens 8 %. Four hand-overs cost more in waits than they overlap. With it, in bursts of 20
+// ms / in loops of 1.5 s at the clock that the power limit leaves there: 217 / 245 us (1597 MHz), 43 / 39 us (1905 MHz), 8.2
+// / 9.3 ms (1567 MHz).
 constexpr int kPFirst = 2;
 constexpr float kLn2 = 0.69314718055994531f;
 constexpr int kSmCount = 148;
@@ -160,10 +162,11 @@ struct Cfg {
   static constexpr uint32_t kColO = 256;    // + t * D
   // Of every 8 scores, how many take the polynomial exp2 on the FMA pipe instead of ex2 on the special-function unit
   // (16 per clock and SM). At head_dim 64 a KV block has as many scores as at 128 and half the MMAs, so the
-  // special-function unit is what both softmax groups compete for: two of eight moved off it took 24 heads x 4429 tokens,
-  // batch 2, from 371 to 353 us and 48 heads x 11.4 k x 33.7 k from 6.39 to 5.93 ms; four of eight are slower (the FMA and
-  // ALU work of a pair, 25 cycles of a warp, then exceeds the 16 cycles of its two ex2). At head_dim 128 it is neutral in
-  // long runs (242 / 239 us at 24 x 4608) and slower where the SMs run at full clock (39.1 -> 40.7 us at 3 x 4608).
+  // special-function unit is what both softmax groups compete for: two of eight moved off it took 5 % off 24 heads x 4429
+  // tokens, batch 2 (now 349 us in a burst, 362 us in a loop at 1845 MHz), and 7 % off 48 heads x 11.4 k x 33.7 k (5.71 ms,
+  // 6.25 ms at 1785 MHz); four of eight are slower (the FMA and ALU work of a pair, 25 cycles of a warp, then exceeds the 16
+  // cycles of its two ex2). At head_dim 128 it is neutral in long runs (24 x 4608, 1 %) and 4 % slower where the SMs run at
+  // full clock (3 x 4608).
   static constexpr int kPoly8 = (D == 64) ? 2 : 0;
 };
 

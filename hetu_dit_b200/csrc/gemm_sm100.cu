@@ -6,7 +6,7 @@
 //   warp 0      TMA producer : A and W tiles of one 64-wide K block per ring stage
 //   warp 1      MMA issuer   : four tcgen05.mma (K = 16 each) per stage and 128-row block of the tile. The issuing
 //                              thread is picked by elect.sync, not by `lane == 0`, which costs 61 cycles of issue per
-//                              MMA (4608 x 12288 x 3072 + GELU 257 -> 241 us, 4608 x 9216 x 3072 202 -> 185 us)
+//                              MMA (6 % of the time at 4608 x 12288 x 3072 + GELU, 8 % at 4608 x 9216 x 3072)
 //   warps 2..   epilogue     : four warps per 128 x 128 or 128 x 256 (one CTA per 256-row tile) block, eight where a
 //                              128 x 256 block is all the CTA has. A thread reads its accumulator row from TMEM 64
 //                              columns at a time, adds the bias in fp32 and rounds to the storage type (the value
@@ -18,11 +18,13 @@
 //
 // A launch takes up to eight layers ("items") of one K; their tiles form one list, so that layers with few rows (the text
 // stream beside the image stream) and layers on one input (Q, K, V) share one partly filled last wave. Measured against
-// a library GEMM and a tail kernel per layer, 4096 image + 512 text rows, hidden 3072: Q, K, V with norm and rotation 352 ->
-// 199 us, output projections + gated residual 97.5 -> 68.6, MLP up + GELU 389 -> 252, MLP down + gated residual 344 -> 261.
+// a library GEMM and a tail kernel per layer, 4096 image + 512 text rows, hidden 3072, in bursts of 20 ms: Q, K, V with norm
+// and rotation 252 -> 193 us, output projections + gated residual 86 -> 67, MLP up + GELU 293 -> 246, MLP down + gated residual
+// 274 -> 253. In loops of 0.8 s both sides slow down with the clock: 278 us at 1634 MHz -> 221 us at 1207 MHz, 90 (1590) -> 76
+// (1425), 326 (1545) -> 283 (1132), 303 (1372) -> 293 (1162).
 //
 // The main loop runs at the tensor pipe's rate: 296.8 k cycles against 294.9 k of MMAs for 4608 x 12288 x 3072 on pairs. What
-// bounds it is the power limit, which holds the SM clock near 1.25-1.35 GHz in such loops (1465-1510 TFLOP/s).
+// bounds it is the power limit, which holds the SM clock at 1.1 to 1.35 GHz in such loops (1190-1510 TFLOP/s, box to box).
 //
 // Tile shapes (rows x columns of the output one CTA owns at a time):
 //   128 x 256, 128 x 128  two accumulators in TMEM: the tensor pipe starts the next tile while the previous one is

@@ -820,10 +820,10 @@ _NS_PER_K, _SAVED_US_PER_LAYER, _LIBRARY_RATE = 2.3e-3, 5.0, 1.15
 def _group_pays(shapes, k):
     """Whether one launch over these outputs beats a library GEMM and a tail kernel per layer: what the partly filled last
     wave wastes (the library splits K there) has to stay below what the launches and the extra pass over the output
-    cost. Measured, us, this kernel / library: 2 layers of 1961 + 231 rows, K = 12288: 163 / 150 (not taken); K = 3072:
-    41 / 46; 1024 + 256 rows, K = 12288: 94 / 101; 256 + 77 rows, K = 12288: 53 / 46 (not taken); 4096 + 512 rows, K =
-    12288: 266 / 318; Q, K, V of 2 x (1024 + 77) rows, K = 1536: 33 / 43, of 4096 + 512 rows, K = 3072 with norm and
-    rotation: 236 / 313."""
+    cost. Measured in bursts of 20 ms, us, this kernel / library: 2 layers of 1961 + 231 rows, K = 12288: 160 / 139 (not
+    taken); K = 3072: 42 / 46; 1024 + 256 rows, K = 12288: 83 / 93; 256 + 77 rows, K = 12288: 54 / 51 (not taken); 4096 + 512
+    rows, K = 12288: 253 / 274; 12240 + 224 rows: 671 / 660 (taken although 2 % slower alone); Q, K,
+    V of 2 x (1024 + 77) rows, K = 1536: 34 / 50, of 4096 + 512 rows, K = 3072 with norm and rotation: 193 / 252."""
     cost, ideal = _group_cost(shapes)
     return (cost - _LIBRARY_RATE * ideal) * k * _NS_PER_K <= _SAVED_US_PER_LAYER * len(shapes)
 
