@@ -693,39 +693,44 @@ FUSED_LINEAR_MIN_ROWS = int(os.environ.get("HDIT_FUSED_LINEAR_MIN_ROWS", "0"))
 FUSED_LINEAR_MAX_ROWS = int(os.environ.get("HDIT_FUSED_LINEAR_MAX_ROWS", str(1 << 40)))
 
 
-_PLAIN_TENSORS = (torch.nn.Parameter, torch.Tensor)
+_HOOKS_OF_ALL, _PRE_HOOKS_OF_ALL = _all_modules._global_forward_hooks, _all_modules._global_forward_pre_hooks
 
 
 def is_plain(module, cls):
     """Whether calling `module` runs cls.forward and nothing else, so that what it does may be done without the call: no
     other class (an adapter, a quantised layer), no forward() put on the object, and no hook, of this module or of all
     modules, that waits for the call."""
-    return type(module) is cls and not (module._forward_hooks or module._forward_pre_hooks or "forward" in module.__dict__ or
-                                        _all_modules._global_forward_hooks or _all_modules._global_forward_pre_hooks)
-
-
-def _is_plain_linear(linear):
-    """Whether calling `linear` is x @ weight.T + bias and nothing else, so that a kernel may be given its weight instead: a
-    plain torch.nn.Linear without a weight of a tensor class of its own."""
-    if not is_plain(linear, torch.nn.Linear):
+    if type(module) is not cls:
         return False
-    w, b = linear.weight, linear.bias
-    return type(w) in _PLAIN_TENSORS and (b is None or type(b) in _PLAIN_TENSORS)
+    own = module.__dict__  # what a module's attributes are read from, at a quarter of the cost
+    return not (own["_forward_hooks"] or own["_forward_pre_hooks"] or "forward" in own or _HOOKS_OF_ALL or _PRE_HOOKS_OF_ALL)
+
+
+def _plain_weights(linear):
+    """(weight, bias) where calling `linear` is x @ weight.T + bias and nothing else, so that a kernel may be given them
+    instead: a plain torch.nn.Linear without a weight of a tensor class of its own. Else None."""
+    if not is_plain(linear, torch.nn.Linear):
+        return None
+    own = linear.__dict__["_parameters"]
+    w, b = own.get("weight"), own.get("bias")
+    if type(w) is not torch.nn.Parameter or (linear.bias is not None if b is None else type(b) is not torch.nn.Parameter):
+        return None
+    return w, b
 
 
 def linear_tail(linear, x, epilogue, residual=None, gate=None, out=None):
     """A torch.nn.Linear followed by its elementwise tail ("gelu_tanh", or "gate_residual" = residual +
-    gate[:, None] * linear(x)), as one kernel when can_group_linears() allows it, rows are evenly strided across the
-    batch and it pays, else as the call of `linear` plus hdit_gelu_tanh / hdit_gate_residual."""
+    gate[:, None] * linear(x)), as one kernel when _fusable_weights() has the layer, rows are evenly strided across
+    the batch and it pays, else as the call of `linear` plus hdit_gelu_tanh / hdit_gate_residual."""
     if epilogue not in ("gelu_tanh", "gate_residual"):
         raise ValueError(epilogue)
-    fusable = (epilogue in FUSED_LINEAR_TAILS and can_group_linears([x], [linear]) and _even_rows(x)
-               and FUSED_LINEAR_MIN_ROWS <= x.shape[0] * x.shape[1] <= FUSED_LINEAR_MAX_ROWS
-               and _tail_fits(x, linear.weight.shape[0], residual, gate, out)
-               and all(t is None or _even_rows(t) for t in (residual, out))
-               and _group_pays(((x.shape[0] * x.shape[1], linear.weight.shape[0]),), x.shape[2]))
-    if fusable:
-        return linear_fused(x, linear.weight, linear.bias, epilogue, residual=residual, gate=gate, out=out)
+    weights = _fusable_weights((x,), (linear,)) if epilogue in FUSED_LINEAR_TAILS else None
+    if weights is not None:
+        (w, b), = weights
+        (B, S, k), n = x.shape, w.shape[0]
+        if _even_rows(x) and FUSED_LINEAR_MIN_ROWS <= B * S <= FUSED_LINEAR_MAX_ROWS and _tail_fits(x, n, residual, gate, out) \
+                and (residual is None or _even_rows(residual)) and (out is None or _even_rows(out)) and _group_pays(((B * S, n),), k):
+            return linear_fused(x, w, b, epilogue, residual=residual, gate=gate, out=out)
     y = linear(x)
     if epilogue == "gelu_tanh":
         return gelu_tanh(y, out=y if out is None else out)
@@ -742,44 +747,51 @@ def _aligned(x):
 def _tail_fits(x, n, residual, gate, out=None):
     """Whether the kernel takes these with an (B, S, N) output for input x: residual and result of that shape and gate
     (B, N), of x's type, on its device, aligned. What it does not take, gate_residual() takes or refuses by itself."""
-    shape = (x.shape[0], x.shape[1], n)
+    B, S, _ = x.shape
+    dtype, dev = x.dtype, x.device
     for t in (residual, out):
-        if t is not None and (tuple(t.shape) != shape or t.dtype != x.dtype or t.device != x.device or not _aligned(t)):
+        if t is not None and (t.shape != (B, S, n) or t.dtype != dtype or t.device != dev or not _aligned(t)):
             return False
-    return gate is None or (tuple(gate.shape) == (shape[0], n) and gate.dtype == x.dtype and gate.device == x.device and
-                            gate.stride(1) == 1 and gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0)
+    if gate is None:
+        return True
+    return gate.shape == (B, n) and gate.dtype == dtype and gate.device == dev and gate.stride(1) == 1 and \
+        gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0
+
+
+def _fusable_weights(xs, linears):
+    """The (weight, bias) of every layer where these layers on these (B, S, K) inputs may go through linear_fused() /
+    linear_group(): the switch is on, no gradient is recorded, the layers are plain torch.nn.Linear that nothing waits for
+    the call of, and layouts and types are what the kernel takes. Else None: the library GEMM takes inner sizes that are no
+    multiple of 8 and rows that overlap or do not start on 16-byte boundaries."""
+    if not FUSED_LINEAR or torch.is_grad_enabled():
+        return None
+    k, dtype, dev = xs[0].shape[-1], xs[0].dtype, xs[0].device
+    if dtype not in _DTYPE_CODE or k % 8:
+        return None
+    for x in xs:
+        if not x.is_cuda or x.dim() != 3 or x.dtype != dtype or x.device != dev:
+            return None
+        B, S, kx = x.shape
+        if kx != k or (B > 1 and S < 32) or not _aligned(x):
+            return None
+    weights = []
+    for linear in linears:
+        plain = _plain_weights(linear)
+        if plain is None:
+            return None
+        w, b = plain
+        (n, kw), (sn, sk) = w.shape, w.stride()
+        if kw != k or n % 8 or sk != 1 or sn < k or sn % 8 or w.dtype != dtype or w.device != dev or w.data_ptr() % 16:
+            return None
+        if b is not None and (b.dtype != dtype or b.numel() != n or not b.is_contiguous() or b.data_ptr() % 16):
+            return None
+        weights.append(plain)
+    return weights
 
 
 def can_group_linears(xs, linears):
-    """Whether these layers on these (B, S, K) inputs may go through linear_fused() / linear_group(): the switch is on, no
-    gradient is recorded, the layers are plain torch.nn.Linear that nothing waits for the call of, and layouts and types
-    are what the kernel takes. The library GEMM takes all others: inner sizes that are no multiple of 8, rows that overlap or
-    do not start on 16-byte boundaries."""
-    if not FUSED_LINEAR or torch.is_grad_enabled():
-        return False
-    k, dtype, dev = xs[0].shape[-1], xs[0].dtype, xs[0].device
-    if dtype not in _DTYPE_CODE or k % 8:
-        return False
-    for x in xs:
-        if not x.is_cuda or x.dim() != 3 or x.dtype != dtype or x.device != dev:
-            return False
-        if x.shape[2] != k or not _aligned(x) or (x.shape[0] > 1 and x.shape[1] < 32):
-            return False
-    for l in linears:
-        if not _is_plain_linear(l):
-            return False
-        w, b = l._parameters.get("weight"), l._parameters.get("bias")
-        if w is None or w.dtype != dtype or w.device != dev or w.data_ptr() % 16:
-            return False
-        (n, kw), (sn, sk) = w.shape, w.stride()
-        if kw != k or n % 8 or sk != 1 or sn < k or sn % 8:
-            return False
-        if b is None:
-            if l.bias is not None:
-                return False
-        elif b.dtype != dtype or b.numel() != n or not b.is_contiguous() or b.data_ptr() % 16:
-            return False
-    return True
+    """Whether these layers on these inputs may go through linear_group(), see _fusable_weights()."""
+    return _fusable_weights(xs, linears) is not None
 
 
 def norm_rope_fits(x, head_dim, norms, rope):
@@ -844,13 +856,13 @@ def use_linear_group(items):
 
 def try_linear_tails(specs):
     """The layers of linear_tails() in one launch, or None where that is not possible or does not pay."""
-    xs, linears = [sp[1] for sp in specs], [sp[0] for sp in specs]
-    if not can_group_linears(xs, linears):
+    weights = _fusable_weights([sp[1] for sp in specs], [sp[0] for sp in specs])
+    if weights is None:
         return None
     items = []
-    for linear, x, epilogue, *rest in specs:
+    for (linear, x, epilogue, *rest), (w, _) in zip(specs, weights):
         residual, gate = rest if rest else (None, None)
-        if not _tail_fits(x, linear.weight.shape[0], residual, gate):
+        if not _tail_fits(x, w.shape[0], residual, gate):
             return None
         items.append(Lin(x, linear, epilogue, residual=residual, gate=gate))
     return linear_group(items) if use_linear_group(items) else None
