@@ -481,6 +481,11 @@ HDIT_API int hdit_linear_fused(const hdit_gemm_args* args);
  *                                  fp32 each.
  * Alignment and ragged sizes as for hdit_linear_fused.
  *
+ * Kernels of this library start while the kernel before them in the stream drains, and wait for it before they read. The bias
+ * (here and in hdit_linear_fused), norm weights and tables are parameters, read by the read-only path: their writer has to have
+ * finished when this kernel starts, as torch's kernels and hdit_copy_pieces have; no other kernel here may be their writer
+ * with nothing in between.
+ *
  * In the reference Q, K, V and the added text projections are torch.nn.Linear calls of their own, followed by eager norm
  * and rotary kernels (layers/attention_processor.py:68-120, 632-793, 797-987).
  */
