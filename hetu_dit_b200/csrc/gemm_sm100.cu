@@ -40,6 +40,13 @@
 //                         partner's barrier), the odd CTA's epilogue warps hand accumulators back by arriving on
 //                         the even CTA's barrier, and tcgen05.commit multicasts "stage consumed" / "accumulator
 //                         ready" to both CTAs. No TMA multicast is used.
+//   pair, 256 x 192 and 256 x 128   the same with narrower tiles (each CTA loads 96 or 64 rows of W), for launches whose
+//                         256 x 256 tiles would leave much of the last wave idle. They ask L2 for 73 and 96 bytes per clock
+//                         and SM instead of 64; a wave of them takes 0.78 and 0.55 of a wave of 256 x 256 tiles. Against the
+//                         best of the other shapes (256 x 256 pair / 128 x 128), us in bursts of 20 ms: 1961 + 231 rows,
+//                         K = 12288, N = 3072 (108 tiles on 74 pairs) 175 -> 138 with 192 columns; 2192 rows, K = 15360
+//                         217 -> 168; 11056 rows, K = 15360 920 -> 766; 2 x (1024 + 77) rows, K = 6144 48 -> 40; Q, K, V of
+//                         1024 + 256 rows, K = 3072, 75 -> 70 with 128 columns; 2 x (600 + 120) rows, K = 6144 29 -> 26.
 //
 // Biases, norm weights and rotary tables are read with __ldg(): parameters, which no kernel writes that lets another one
 // start before it has finished (host_common.h). Everything else, the gate among it, is read with plain loads. Behind plain
@@ -74,8 +81,11 @@ constexpr uint32_t kSpinLimit = 8u * 1000u * 1000u;
 constexpr int kMaxSmem = 232448;  // 227 KiB opt-in limit per CTA
 // Relative time per 128 x 128 of output for each work-unit shape, from measurement; used only to choose a shape. 256 x 256
 // pair : 128 x 256 : 128 x 128, us per wave: 10.6 : 11.8 : 6.8 per (2 : 2 : 1) blocks at K = 1536, 20.8 : 25 : 15.5 at 12464
-// rows and K = 3072, 30 : 31 : 15.2 at 1280 rows, where the clock is not held down.
-constexpr double kCost128x256 = 1.18, kCost128x128 = 1.25, kCost256x256 = 1.3, kCostPair = 1.05;
+// rows and K = 3072, 30 : 31 : 15.2 at 1280 rows, where the clock is not held down. Pairs of 192 and 128 columns against
+// 256, us per wave: 69 : 48 : 87.5 and 18 : 12.5 : 23 at 2192 rows (K = 12288, 3072), 33.4 : 23.8 : 46 at 8858 rows and
+// K = 6144, 63 : 47 : 86 at 11056 rows and K = 12288.
+constexpr double kCost128x256 = 1.18, kCost128x128 = 1.25, kCost256x256 = 1.3, kCostPair = 1.05,
+                 kCostPair192 = 1.09, kCostPair128 = 1.18;
 
 #ifdef HDIT_GEMM_TRACE
 // per CTA: MMA thread {total, waiting for operands, waiting for a free accumulator, tiles}, epilogue warp 2
@@ -92,13 +102,15 @@ enum GemmWait : int {
 
 template <int BM, int BN, bool PAIR>
 struct GemmCfg {
-  static_assert(!PAIR || (BM == 128 && BN == 256), "a CTA of a pair owns 128 x 256 of the pair's 256 x 256 tile");
+  static_assert(!PAIR || BM == 128, "a CTA of a pair owns 128 of the tile's 256 rows");
   static constexpr int kHalves = BM / 128;                 // 128-row MMA blocks per CTA tile
   static constexpr int kAccBufs = (kHalves == 1) ? 2 : 1;  // accumulator tiles resident in TMEM
-  // Four warps reach all 128 lanes of an accumulator block; a 256-column accumulator has two such teams, each with half
-  // of the columns. With one team the norm + rotation tail took 28.6 k cycles per 128 x 256 accumulator, longer than the
+  // Four warps reach all 128 lanes of an accumulator block; the accumulators of a pair and those of 256 columns have two
+  // such teams, each with half of the columns (128 and 64 of 192). With one team the norm + rotation tail took 28.6 k cycles per 128 x 256 accumulator, longer than the
   // 24.6 k of the main loop at K = 3072 that it hides behind.
-  static constexpr int kColTeams = (kHalves == 1 && BN == 256) ? 2 : 1;
+  static constexpr int kColTeams = (kHalves == 1 && (PAIR || BN == 256)) ? 2 : 1;
+  static constexpr int kPieces = BN / 64;                                    // 64-column pieces of the accumulator
+  static constexpr int kTeamPieces = (kPieces + kColTeams - 1) / kColTeams;  // the last team may have fewer
   static constexpr int kEpiWarps = 4 * kHalves * kColTeams;
   static constexpr int kThreads = 64 + 32 * kEpiWarps;
   static constexpr int kTileRows = PAIR ? 2 * BM : BM;     // rows of the scheduling unit's tile
@@ -110,7 +122,8 @@ struct GemmCfg {
   static constexpr int kBarBytes = 256;
   static constexpr int kStagesFit = (kMaxSmem - 1024 - kBarBytes - kStagingBytes) / kStageBytes;
   static constexpr int kStages = kStagesFit > 8 ? 8 : kStagesFit;
-  static constexpr int kTmemCols = kHalves * kAccBufs * BN;
+  static constexpr int kAccCols = (BN == 192) ? 256 : BN;  // TMEM columns from one accumulator to the next
+  static constexpr int kTmemCols = kHalves * kAccBufs * kAccCols;
   static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kStagingBytes + kBarBytes;
   static_assert(kTmemCols == 256 || kTmemCols == 512, "TMEM allocation must be a power of two");
   static_assert(kStages >= 3, "ring too short");
@@ -501,7 +514,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
 #ifdef HDIT_GEMM_TRACE
         tr_wait_acc += clock64() - tr_a0;
 #endif
-        const uint32_t d_tmem = tmem_base + acc * C::kHalves * BN;
+        const uint32_t d_tmem = tmem_base + acc * C::kHalves * C::kAccCols;
         for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
           const uint32_t s = it % C::kStages, round = it / C::kStages;
 #ifdef HDIT_GEMM_TRACE
@@ -527,7 +540,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
               if constexpr (PAIR)
                 umma_ss_pair(d_tmem, a_desc + off, b_desc + off, idesc, (kb | kk) != 0 ? 1u : 0u);
               else
-                umma_ss(d_tmem + h * BN, a_desc + off, b_desc + off, idesc, (kb | kk) != 0 ? 1u : 0u);
+                umma_ss(d_tmem + h * C::kAccCols, a_desc + off, b_desc + off, idesc, (kb | kk) != 0 ? 1u : 0u);
             }
           }
           if constexpr (PAIR) tc_commit_pair(&empty[s]);
@@ -557,8 +570,9 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
     const int quarter = warp & 3;  // the TMEM lanes this warp may read: [32 * quarter, 32 * quarter + 32)
     const int team = (warp - 2) >> 2;
     const int half = C::kColTeams == 1 ? team : 0;  // which 128-row block of the tile
-    constexpr int kPieces = BN / 64 / C::kColTeams;   // 64-column pieces of this warp
-    const int c0 = C::kColTeams == 1 ? 0 : team * kPieces;
+    // 64-column pieces of this warp
+    const int c0 = C::kColTeams == 1 ? 0 : team * C::kTeamPieces;
+    const int c1 = C::kColTeams == 1 ? C::kPieces : min(C::kPieces, c0 + C::kTeamPieces);
     uint8_t* staging = staging_base + (warp - 2) * 4096;
     const int sub_row = lane >> 3, chunk = lane & 7;  // store phase: 4 rows per instruction, 8 lanes per row
     uint32_t local = 0;
@@ -583,7 +597,7 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
       // first of the 32 rows this warp owns
       const long long row0 = static_cast<long long>(m_t) * C::kTileRows + static_cast<long long>(rank) * BM + half * 128 +
                              quarter * 32;
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + (acc * C::kHalves + half) * BN;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + (acc * C::kHalves + half) * C::kAccCols;
       long long batch0 = 0, next_batch_row = im.M;
       if (im.epilogue >= HDIT_GEMM_BIAS_GATE_RESIDUAL && row0 < im.M) {
         batch0 = static_cast<long long>(static_cast<unsigned>(row0) / static_cast<unsigned>(im.rows_per_batch));
@@ -591,14 +605,15 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
       }
       float2 stats = make_float2(0.f, 0.f);
 #pragma unroll 1
-      for (int c = c0; c < c0 + kPieces; ++c) {
-        if (im.epilogue == HDIT_GEMM_BIAS_NORM_ROPE && im.norm != 0 && ((c * 64) & (im.head_dim - 1)) == 0)
-          stats = head_stats<FP16>(im, taddr + c * 64, n_t * BN + c * 64);
+      for (int c = c0; c < c1; ++c) {
+        const int head0 = (c * 64) & ~(im.head_dim - 1);  // a team may begin in the middle of a head
+        if (im.epilogue == HDIT_GEMM_BIAS_NORM_ROPE && im.norm != 0 && (c == c0 || head0 == c * 64))
+          stats = head_stats<FP16>(im, taddr + head0, n_t * BN + head0);
         uint32_t r[64];
         tmem_ld32(taddr + c * 64, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
         tmem_ld32(taddr + c * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
         tc_wait_ld();
-        if (c == c0 + kPieces - 1) {
+        if (c == c1 - 1) {
           // the accumulator is in registers: hand it back to the MMA warp before the rest of the last piece
           tc_fence_before();
           __syncwarp();
@@ -902,7 +917,8 @@ extern "C" int hdit_linear_group(const hdit_linear_group_args* a) {
   kp.status = device_status_ptr();
   if (kp.status == nullptr) return HDIT_ERR_CUDA;
 
-  // Shape of the work unit: 0 = 128 x 256, 1 = 128 x 128, 2 = 256 x 256 in one CTA, 3 = 256 x 256 on a CTA pair.
+  // Shape of the work unit: 0 = 128 x 256, 1 = 128 x 128, 2 = 256 x 256 in one CTA, 3 = 256 x 256, 4 = 256 x 192, 5 =
+  // 256 x 128 on a CTA pair.
   int shape;
   if (a->cta_pair == 2) {
     shape = 3;
@@ -916,14 +932,20 @@ extern "C" int hdit_linear_group(const hdit_linear_group_args* a) {
     // write-out (256 x 256 in one CTA).
     const long long sms = a->max_ctas > 0 ? a->max_ctas : sm_count();
     struct Cand { int shape, rows, cols, units_div; double per_tile; };
-    const Cand cand[4] = {{0, 128, 256, 1, 2.0 * kCost128x256}, {1, 128, 128, 1, 1.0 * kCost128x128},
-                          {2, 256, 256, 1, 4.0 * kCost256x256}, {3, 256, 256, 2, 2.0 * kCostPair}};
+    const Cand cand[6] = {{0, 128, 256, 1, 2.0 * kCost128x256}, {1, 128, 128, 1, 1.0 * kCost128x128},
+                          {2, 256, 256, 1, 4.0 * kCost256x256}, {3, 256, 256, 2, 2.0 * kCostPair},
+                          {4, 256, 192, 2, 1.5 * kCostPair192}, {5, 256, 128, 2, 1.0 * kCostPair128}};
+    bool wide_heads = false;  // heads of 128 columns do not divide a 192-column tile
+    for (int i = 0; i < live.n_items; ++i)
+      wide_heads |= live.item[i].epilogue == HDIT_GEMM_BIAS_NORM_ROPE && live.item[i].head_dim == 128;
     double best = -1.0;
     shape = 0;
     for (const Cand& c : cand) {
       if (a->tile_m != 0 && a->tile_m != c.rows) continue;
       if (a->tile_n != 0 && a->tile_n != c.cols) continue;
-      if (c.shape == 3 && a->cta_pair == 1) continue;
+      if (c.shape >= 3 && a->cta_pair == 1) continue;
+      if (c.shape >= 4 && (a->tile_m != 0 || a->tile_n != 0)) continue;  // not among the shapes that can be asked for
+      if (c.shape == 4 && wide_heads) continue;
       if (c.shape == 2 && a->tile_m != 256) continue;  // one CTA per 256 x 256 tile only on request
       const long long units = sms / c.units_div > 0 ? sms / c.units_div : 1;
       long long tiles = 0;
@@ -935,6 +957,8 @@ extern "C" int hdit_linear_group(const hdit_linear_group_args* a) {
   }
   const bool fp16 = a->dtype == HDIT_FP16;
   switch (shape) {
+    case 5: return fp16 ? launch_gemm<128, 128, true, true>(kp, &live) : launch_gemm<128, 128, true, false>(kp, &live);
+    case 4: return fp16 ? launch_gemm<128, 192, true, true>(kp, &live) : launch_gemm<128, 192, true, false>(kp, &live);
     case 3: return fp16 ? launch_gemm<128, 256, true, true>(kp, &live) : launch_gemm<128, 256, true, false>(kp, &live);
     case 2: return fp16 ? launch_gemm<256, 256, false, true>(kp, &live) : launch_gemm<256, 256, false, false>(kp, &live);
     case 1: return fp16 ? launch_gemm<128, 128, false, true>(kp, &live) : launch_gemm<128, 128, false, false>(kp, &live);

@@ -816,7 +816,8 @@ def _group_cost(shapes):
     of output tiles times the time of a tile, smallest over the kernel's tile shapes (the constants are the library's
     own, csrc/gemm_sm100.cu). Second result: the same if every SM always had work."""
     best = None
-    for tm, tn, units, per_tile in ((128, 256, _SM_COUNT, 2.36), (128, 128, _SM_COUNT, 1.25), (256, 256, _SM_COUNT // 2, 2.1)):
+    for tm, tn, units, per_tile in ((128, 256, _SM_COUNT, 2.36), (128, 128, _SM_COUNT, 1.25), (256, 256, _SM_COUNT // 2, 2.1),
+                                    (256, 192, _SM_COUNT // 2, 1.635), (256, 128, _SM_COUNT // 2, 1.18)):
         tiles = sum(-(-m // tm) * -(-n // tn) for m, n in shapes)
         cost = -(-tiles // units) * per_tile
         best = cost if best is None else min(best, cost)
@@ -832,8 +833,8 @@ _NS_PER_K, _SAVED_US_PER_LAYER, _LIBRARY_RATE = 2.3e-3, 5.0, 1.15
 def _group_pays(shapes, k):
     """Whether one launch over these outputs beats a library GEMM and a tail kernel per layer: what the partly filled last
     wave wastes (the library splits K there) has to stay below what the launches and the extra pass over the output
-    cost. Measured in bursts of 20 ms, us, this kernel / library: 2 layers of 1961 + 231 rows, K = 12288: 160 / 139 (not
-    taken); K = 3072: 42 / 46; 1024 + 256 rows, K = 12288: 83 / 93; 256 + 77 rows, K = 12288: 54 / 51 (not taken); 4096 + 512
+    cost. Measured in bursts of 20 ms, us, this kernel / library: 2 layers of 1961 + 231 rows, K = 12288: 138 / 162
+    (192-column tiles); K = 3072: 38 / 47; 1024 + 256 rows, K = 12288: 83 / 93; 256 + 77 rows, K = 12288: 47 / 46 (not taken); 4096 + 512
     rows, K = 12288: 253 / 274; 12240 + 224 rows: 671 / 660 (taken although 2 % slower alone); Q, K,
     V of 2 x (1024 + 77) rows, K = 1536: 34 / 50, of 4096 + 512 rows, K = 3072 with norm and rotation: 193 / 252."""
     cost, ideal = _group_cost(shapes)
