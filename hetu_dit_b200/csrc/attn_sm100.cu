@@ -1,7 +1,8 @@
 // Joint flash-attention forward for sm_100a.
 //
 // One CTA owns two 128-row Q tiles of one (batch, head) and walks the KV
-// sequence in 128-row blocks:
+// sequence in 128-row blocks (at head_dim 64 also three tiles and 96-row
+// blocks, see below; the warp numbers are those of two tiles):
 //
 //   warp 8      TMA producer   : Q tiles once, then K/V blocks through two rings
 //   warp 9      MMA issuer     : S = Q K^T (tcgen05.mma, smem x smem -> TMEM)
@@ -20,6 +21,14 @@
 //
 // The two softmax groups ping-pong against the tensor pipe: while group 0
 // exponentiates S0 the tensor pipe runs P1 V and the next Q1 K^T, and vice versa.
+//
+// At head_dim 64 a pair leaves every unit idle for half of the time: a KV block of a tile goes S -> load -> maximum ->
+// exponentials -> P V -> next Q K^T, and with two tiles that chain sets the pace (2880 cycles per 128 x 128 block of both, 770
+// of them waiting for S; 1536 of exponentials, 768 of MMAs). The tensor memory that the narrower O leaves holds a third
+// tile once the KV block has 96 rows (3 * 96 + 3 * 64 columns), with 152 registers per softmax thread: 2 x 24 heads x 4429
+// tokens 349 -> 318 us, 48 heads x 12464 2.45 -> 2.36 ms, 2 x 24 heads x 1101 38.6 -> 26 us (144 CTAs instead of 240). Taken
+// by the wave rule in attn_fwd_impl(). Two CTAs per SM of two tiles and 64-row blocks each were no faster than the pair
+// (349 us), one CTA with two S buffers per tile slower (382; head_dim 128: 220 -> 268 us at 24 heads x 4608).
 //
 // Small grids (fewer tile pairs than SMs, e.g. the head-sharded calls after a Ulysses exchange) run in
 // "interleaved" mode instead: a CTA owns ONE Q tile, its two halves (softmax group + MMA issuer each)
@@ -53,19 +62,8 @@ namespace hdit {
 namespace {
 
 constexpr int kBlockM = 128;
-constexpr int kBlockN = 128;
-constexpr int kNumThreads = 384;  // 2 softmax warpgroups + 1 warpgroup holding the TMA and MMA warps
-constexpr int kPanelBytes = 128 * 128;  // 128 rows x 64 16-bit elements, 128B-swizzled
 constexpr uint32_t kSpinLimit = 8u * 1000u * 1000u;
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
-// P of a KV block is handed to the MMA thread in two parts, the first after this many of its four 32-column chunks: the
-// first half of P V runs while the second half is exponentiated, which takes those MMAs off the chain softmax -> P V ->
-// next Q K^T that bounds a tile (3294 -> 3057 cycles per KV block pair at head_dim 128, 2048 of them MMAs). Measured
-// against one hand-over, in turn on one box: 24 heads x 4608 x 128 10 % less (after one chunk 6 %, after three 9 %), 3 heads
-// 13 %, 6 heads of 29.7 k x 119 k tokens 8 %. Four hand-overs cost more in waits than they overlap. With it, in bursts of 20
-// ms / in loops of 1.5 s at the clock that the power limit leaves there: 217 / 245 us (1597 MHz), 43 / 39 us (1905 MHz), 8.2
-// / 9.3 ms (1567 MHz).
-constexpr int kPFirst = 2;
 constexpr float kLn2 = 0.69314718055994531f;
 constexpr int kSmCount = 148;
 
@@ -117,7 +115,7 @@ struct alignas(64) AttnKernelParams {
   unsigned char v_swap[HDIT_MAX_KV_SEG];
   int n_q_seg, n_kv_seg;
   int batch, heads;
-  int n_tiles_seg0, n_tiles, n_pairs;
+  int n_tiles_seg0, n_tiles, n_groups;
   int n_kv_blocks;
   int mode;
   float scale_log2;
@@ -146,20 +144,44 @@ struct alignas(64) AttnKernelParams {
   unsigned wait_spins;
 };
 
-template <int D>
+// L lanes: softmax warpgroups, each with an S / P and an O tile of its own in tensor memory.
+template <int D, int L>
 struct Cfg {
+  static_assert(L == 2 || (L == 3 && D == 64), "three lanes need the tensor memory that a head of 64 leaves");
+  static constexpr int kBN = (L == 2) ? 128 : 96;   // rows of a KV block
+  static constexpr int kThreads = 128 * (L + 1);    // + 1 warpgroup holding the TMA and MMA warps
   static constexpr int kPanels = D / 64;
+  static constexpr int kQPanelBytes = kBlockM * 128;  // 64 16-bit elements of every row, 128B-swizzled
+  static constexpr int kPanelBytes = kBN * 128;
+  static constexpr int kQBytes = kPanels * kQPanelBytes;
   static constexpr int kTileBytes = kPanels * kPanelBytes;
   static constexpr int kStagesK = (D == 128) ? 2 : 4;
   static constexpr int kStagesV = (D == 128) ? 2 : 4;
-  static constexpr int kSmemQ = 2 * kTileBytes;
+  static constexpr int kSmemQ = L * kQBytes;
   static constexpr int kSmemK = kStagesK * kTileBytes;
   static constexpr int kSmemV = kStagesV * kTileBytes;
   static constexpr int kSmemBytes = kSmemQ + kSmemK + kSmemV + 1024 /*align*/ + 512 /*barriers etc.*/;
   static_assert(kSmemBytes <= 232448, "exceeds the 227 KB a CTA may use");
   static constexpr uint32_t kTmemCols = 512;
-  static constexpr uint32_t kColS = 0;      // + t * 128
-  static constexpr uint32_t kColO = 256;    // + t * D
+  static constexpr uint32_t kColS = 0;          // + t * kBN
+  static constexpr uint32_t kColO = L * kBN;    // + t * D
+  static_assert(L * (kBN + D) <= 512, "exceeds the tensor memory of an SM");
+  // registers per thread of the softmax warps and of the others, out of the pool that the CTA was launched with
+  static constexpr int kRegsLaunch = (L == 2) ? 168 : 128;
+  static constexpr int kRegsSoftmax = (L == 2) ? 216 : 152;
+  static constexpr int kRegsOther = (L == 2) ? 72 : 56;
+  static_assert(L * kRegsSoftmax + kRegsOther <= (L + 1) * kRegsLaunch, "setmaxnreg.inc would wait for ever");
+  static constexpr int kRescaleCols = (L == 2) ? 32 : 16;  // columns of O in registers at a time, beside a row of S
+  static constexpr int kChunks = kBN / 32;
+  // P of a KV block is handed to the MMA thread in two parts, the first after this many of its 32-column chunks: the first
+  // part of P V runs while the rest is exponentiated, which takes those MMAs off the chain softmax -> P V -> next Q K^T
+  // that bounds a tile (3294 -> 3057 cycles per KV block pair at head_dim 128, 2048 of them MMAs). Measured against one
+  // hand-over, in turn on one box, with two lanes: 24 heads x 4608 x 128 10 % less (after one chunk 6 %, after three 9 %), 3
+  // heads 13 %, 6 heads of 29.7 k x 119 k tokens 8 %. Four hand-overs cost more in waits than they overlap. With it, in
+  // bursts of 20 ms / in loops of 1.5 s at the clock that the power limit leaves there: 217 / 245 us (1597 MHz), 43 / 39 us
+  // (1905 MHz), 8.2 / 9.3 ms (1567 MHz). With three lanes after one chunk / two / no first part: 2 x 24 heads x 4429
+  // 318 / 322 / 318 us, 48 heads x 12464 2.36 / 2.38 / 2.40 ms.
+  static constexpr int kPFirst = (L == 2) ? 2 : 1;
   // Of every 8 scores, how many take the polynomial exp2 on the FMA pipe instead of ex2 on the special-function unit
   // (16 per clock and SM). At head_dim 64 a KV block has as many scores as at 128 and half the MMAs, so the
   // special-function unit is what both softmax groups compete for: two of eight moved off it took 5 % off 24 heads x 4429
@@ -173,8 +195,8 @@ struct Cfg {
 struct KvCursor {
   int seg;
   int row0;
-  __device__ __forceinline__ void advance(const AttnKernelParams& p) {
-    row0 += kBlockN;
+  __device__ __forceinline__ void advance(const AttnKernelParams& p, int block) {
+    row0 += block;
     if (row0 >= p.kv_len[seg]) {
       ++seg;
       row0 = 0;
@@ -195,12 +217,12 @@ __device__ __forceinline__ void tile_coords(const AttnKernelParams& p, int tile,
 }
 
 __device__ __forceinline__ void load_tile(const CUtensorMap* map, bool swapped, char* smem, uint64_t* bar, int panels,
-                                          int h, int row0, int b) {
+                                          int panel_bytes, int h, int row0, int b) {
   for (int pn = 0; pn < panels; ++pn) {
     if (swapped)
-      tma_load_4d(smem + pn * kPanelBytes, map, bar, pn * 64, row0, h, b);
+      tma_load_4d(smem + pn * panel_bytes, map, bar, pn * 64, row0, h, b);
     else
-      tma_load_4d(smem + pn * kPanelBytes, map, bar, pn * 64, h, row0, b);
+      tma_load_4d(smem + pn * panel_bytes, map, bar, pn * 64, h, row0, b);
   }
 }
 
@@ -246,26 +268,28 @@ __device__ __forceinline__ float2 ex2_poly2(float2 x) {
   return out;
 }
 
-template <int D, bool FP16, bool IL>
-__global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_constant__ AttnKernelParams p) {
-  using C = Cfg<D>;
+template <int D, int L, bool FP16, bool IL>
+__global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const __grid_constant__ AttnKernelParams p) {
+  static_assert(!IL || L == 2, "interleaved mode has two halves");
+  using C = Cfg<D, L>;
+  constexpr int kBlockN = C::kBN;
   extern __shared__ char smem_raw[];
   char* smem = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   char* smem_q = smem;
   char* smem_k = smem_q + C::kSmemQ;
   char* smem_v = smem_k + C::kSmemK;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_v + C::kSmemV);
-  uint64_t* q_full = bars;                       // [2]
-  uint64_t* k_full = q_full + 2;                 // [K stages]
+  uint64_t* q_full = bars;                       // [L]
+  uint64_t* k_full = q_full + L;                 // [K stages]
   uint64_t* k_empty = k_full + C::kStagesK;      // [K stages]
   uint64_t* v_full = k_empty + C::kStagesK;      // [V stages]
   uint64_t* v_empty = v_full + C::kStagesV;      // [V stages]
-  uint64_t* s_full = v_empty + C::kStagesV;      // [2]
-  uint64_t* p_ready = s_full + 2;                // [2]
-  uint64_t* o_done = p_ready + 2;                // [2]
-  uint64_t* merge_bar = o_done + 2;              // [1] interleaved mode: half 1's partial result is in smem
-  uint64_t* p_rest = merge_bar + 1;              // [2] the second part of P is in TMEM (p_ready: the first)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_rest + 2);
+  uint64_t* s_full = v_empty + C::kStagesV;      // [L]
+  uint64_t* p_ready = s_full + L;                // [L]
+  uint64_t* o_done = p_ready + L;                // [L]
+  uint64_t* merge_bar = o_done + L;              // [1] interleaved mode: half 1's partial result is in smem
+  uint64_t* p_rest = merge_bar + 1;              // [L] the second part of P is in TMEM (p_ready: the first)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_rest + L);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -273,20 +297,20 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
 
   // ---- work item -------------------------------------------------------
   int idx = blockIdx.x;
-  const int pair = idx % p.n_pairs;
-  idx /= p.n_pairs;
+  const int group = idx % p.n_groups;
+  idx /= p.n_groups;
   const int h = idx % p.heads;
   const int b = idx / p.heads;
   constexpr bool il = IL;  // interleaved mode is its own instantiation: the paired loop carries none of its branches
-  const int tile0 = il ? pair : pair * 2;
+  const int tile0 = il ? group : group * L;
   int j_begin = 0;
   int nblk = p.n_kv_blocks;
   if (p.kv_split_blocks > 0) {
     j_begin = static_cast<int>(blockIdx.y) * p.kv_split_blocks;
     nblk = min(p.n_kv_blocks - j_begin, p.kv_split_blocks);
   }
-  // half t (softmax group t + MMA issuer t): its Q tile, and which KV blocks it walks
-  const bool half1_active = il ? (nblk >= 2) : ((tile0 + 1) < p.n_tiles);
+  // lane t (softmax group t): its Q tile, and which KV blocks it walks
+  const int n_active = min(L, il ? nblk : p.n_tiles - tile0);
   const int blk_step = il ? 2 : 1;
   float* const acc_out = p.acc_out + static_cast<long long>(blockIdx.y) * p.split_acc_stride;
   float* const acc_lse = p.acc_lse + static_cast<long long>(blockIdx.y) * p.split_lse_stride;
@@ -297,7 +321,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
   // ---- set-up ----------------------------------------------------------
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < L; ++i) {
       mbar_init(&q_full[i], 1);
       mbar_init(&s_full[i], 1);
       mbar_init(&p_ready[i], 4);  // one arrival per softmax warp
@@ -316,7 +340,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
     fence_mbar_init();
     fence_proxy_async_smem();
   }
-  if (warp == 9) {
+  if (warp == 4 * L + 1) {
     tmem_alloc(tmem_slot, C::kTmemCols);
     tmem_relinquish();
   }
@@ -330,9 +354,9 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
   // Register hand-over between warpgroups: a softmax thread keeps a whole 128-column row of S.
   // Each warpgroup changes its budget at the top of its own branch so the allocation of the code
   // below it is known.
-  if (warp >= 8) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-    if (warp == 8) {
+  if (warp >= 4 * L) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegsOther));
+    if (warp == 4 * L) {
       // =========================== TMA producer ===========================
       bool inputs_ready = true;
       if (p.n_wait > 0) {
@@ -363,15 +387,15 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
           tma_prefetch_desc(&p.k_map[s]);
           tma_prefetch_desc(&p.v_map[s]);
         }
-        for (int t = 0; t < 2; ++t) {
-          if (t == 1 && (il || !half1_active)) break;  // interleaved: both halves share the tile in slot 0
+        for (int t = 0; t < (il ? 1 : n_active); ++t) {  // interleaved: both halves share the tile in slot 0
           int seg, row0, orow;
           tile_coords(p, tile0 + t, seg, row0, orow);
-          mbar_expect_tx(&q_full[t], C::kTileBytes);
-          load_tile(&p.q_map[seg], p.q_swap[seg], smem_q + t * C::kTileBytes, &q_full[t], C::kPanels, h, row0, b);
+          mbar_expect_tx(&q_full[t], C::kQBytes);
+          load_tile(&p.q_map[seg], p.q_swap[seg], smem_q + t * C::kQBytes, &q_full[t], C::kPanels, C::kQPanelBytes, h,
+                    row0, b);
         }
         KvCursor cur{0, 0};
-        for (int i = 0; i < j_begin; ++i) cur.advance(p);
+        for (int i = 0; i < j_begin; ++i) cur.advance(p, kBlockN);
         bool ok = true;
         for (int j = 0; j < nblk && ok; ++j) {
           const int sk = j % C::kStagesK, sv = j % C::kStagesV;
@@ -384,8 +408,8 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
             }
           }
           mbar_expect_tx(&k_full[sk], C::kTileBytes);
-          load_tile(&p.k_map[cur.seg], p.k_swap[cur.seg], smem_k + sk * C::kTileBytes, &k_full[sk], C::kPanels, h,
-                    cur.row0, b);
+          load_tile(&p.k_map[cur.seg], p.k_swap[cur.seg], smem_k + sk * C::kTileBytes, &k_full[sk], C::kPanels,
+                    C::kPanelBytes, h, cur.row0, b);
           if (j >= C::kStagesV) {
             if (!mbar_wait_bounded(&v_empty[sv], (nv - 1) & 1, abort_flag, kSpinLimit)) {
               report_failure(p.status, abort_flag, HDIT_ERR_PEER_TIMEOUT, W_PROD_VEMPTY, j);
@@ -394,40 +418,40 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
             }
           }
           mbar_expect_tx(&v_full[sv], C::kTileBytes);
-          load_tile(&p.v_map[cur.seg], p.v_swap[cur.seg], smem_v + sv * C::kTileBytes, &v_full[sv], C::kPanels, h,
-                    cur.row0, b);
-          cur.advance(p);
+          load_tile(&p.v_map[cur.seg], p.v_swap[cur.seg], smem_v + sv * C::kTileBytes, &v_full[sv], C::kPanels,
+                    C::kPanelBytes, h, cur.row0, b);
+          cur.advance(p, kBlockN);
         }
       }
-    } else if (warp == 9) {
+    } else if (warp == 4 * L + 1) {
       // ============================ MMA issuer ============================
-      // One thread issues for both halves.
+      // One thread issues for all lanes.
       if (elect_one()) {
         constexpr uint32_t kFmt = FP16 ? 0u : 1u;
         constexpr uint32_t idesc_qk = make_idesc_f16(kBlockM, kBlockN, kFmt, 0);
         constexpr uint32_t idesc_pv = make_idesc_f16(kBlockM, D, kFmt, 1);
         bool ok = true;
-        const int last_t = half1_active ? 1 : 0;
         const int n_iter = il ? (nblk + 1) / 2 : nblk;
 
         // Descriptors differ from a per-tile base only in the start-address field (low word, units of
         // 16 bytes), so a k-step costs one 32-bit add instead of a rebuilt 64-bit descriptor.
         const uint64_t q_desc0 = make_smem_desc_sw128(smem_u32(smem_q), 16, 1024);
         const uint64_t k_desc0 = make_smem_desc_sw128(smem_u32(smem_k), 16, 1024);
-        const uint64_t v_desc0 = make_smem_desc_sw128(smem_u32(smem_v), kPanelBytes, 1024);
+        const uint64_t v_desc0 = make_smem_desc_sw128(smem_u32(smem_v), C::kPanelBytes, 1024);
         auto issue_qk = [&](int t, int stage) {
-          const uint32_t d_tmem = tmem_base + C::kColS + t * 128;
-          const uint64_t a0 = q_desc0 + static_cast<uint32_t>(((il ? 0 : t) * C::kTileBytes) >> 4);
+          const uint32_t d_tmem = tmem_base + C::kColS + t * kBlockN;
+          const uint64_t a0 = q_desc0 + static_cast<uint32_t>(((il ? 0 : t) * C::kQBytes) >> 4);
           const uint64_t b0 = k_desc0 + static_cast<uint32_t>((stage * C::kTileBytes) >> 4);
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
-            const uint32_t off = ((kk >> 2) * kPanelBytes + (kk & 3) * 32) >> 4;
-            umma_ss(d_tmem, a0 + off, b0 + off, idesc_qk, kk > 0 ? 1u : 0u);
+            const uint32_t a_off = ((kk >> 2) * C::kQPanelBytes + (kk & 3) * 32) >> 4;
+            const uint32_t b_off = ((kk >> 2) * C::kPanelBytes + (kk & 3) * 32) >> 4;
+            umma_ss(d_tmem, a0 + a_off, b0 + b_off, idesc_qk, kk > 0 ? 1u : 0u);
           }
         };
         auto issue_pv = [&](int t, int stage, bool accumulate, int kk0, int kk1) {
           const uint32_t d_tmem = tmem_base + C::kColO + t * D;
-          const uint32_t a_tmem = tmem_base + C::kColS + t * 128;
+          const uint32_t a_tmem = tmem_base + C::kColS + t * kBlockN;
           const uint64_t b0 = v_desc0 + static_cast<uint32_t>((stage * C::kTileBytes) >> 4);
 #pragma unroll
           for (int kk = kk0; kk < kk1; ++kk) {
@@ -447,27 +471,17 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
         auto v_stage = [](int j) { return j % C::kStagesV; };
         auto v_phase = [](int j) { return static_cast<uint32_t>(j / C::kStagesV) & 1; };
 
-        // prologue: S of each half's first block (block 0 for both when paired; blocks 0 and 1 when interleaved)
-        wait(&q_full[0], 0, W_MMA_QFULL, 0);
-        wait(&k_full[0], 0, W_MMA_KFULL, 0);
-        if (ok) {
+        // prologue: S of each lane's first block (block 0 for all, or block t of half t when interleaved)
+        for (int t = 0; t < n_active; ++t) {
+          const int j = il ? t : 0;
+          if (!il || t == 0) wait(&q_full[t], 0, W_MMA_QFULL, t);
+          if (il || t == 0) wait(&k_full[k_stage(j)], k_phase(j), W_MMA_KFULL, j);
+          if (!ok) break;
           tc_fence_after();
-          issue_qk(0, 0);
-          tc_commit(&s_full[0]);
-          if (il) tc_commit(&k_empty[0]);
+          issue_qk(t, k_stage(j));
+          tc_commit(&s_full[t]);
+          if (il || t == n_active - 1) tc_commit(&k_empty[k_stage(j)]);
         }
-        if (half1_active) {
-          const int j1 = il ? 1 : 0;
-          if (!il) wait(&q_full[1], 0, W_MMA_QFULL, 1);
-          if (il) wait(&k_full[k_stage(1)], k_phase(1), W_MMA_KFULL, 1);
-          if (ok) {
-            tc_fence_after();
-            issue_qk(1, k_stage(j1));
-            tc_commit(&s_full[1]);
-            if (il) tc_commit(&k_empty[k_stage(1)]);
-          }
-        }
-        if (ok && !il) tc_commit(&k_empty[0]);
 
 #ifdef HDIT_ATTN_TRACE
         if (trace_on) {
@@ -478,26 +492,26 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
         }
 #endif
         for (int i = 0; i < n_iter && ok; ++i) {
-          for (int t = 0; t <= last_t && ok; ++t) {
-            // half t's i-th KV block and the one after it
+          for (int t = 0; t < n_active && ok; ++t) {
+            // lane t's i-th KV block and the one after it
             const int j = il ? 2 * i + t : i;
             if (j >= nblk) break;  // interleaved, odd block count: half 1 has one block fewer
             const int jn = j + blk_step;
             const bool has_next = jn < nblk;
-            const bool releases = il || t == last_t;  // the last reader of a stage hands it back
+            const bool releases = il || t == n_active - 1;  // the last reader of a stage hands it back
             if (il || t == 0) {
               wait(&v_full[v_stage(j)], v_phase(j), W_MMA_VFULL, j);
             }
             HDIT_TRACE_MMA(t, i, 0);
-            wait(&p_ready[t], i & 1, W_MMA_PREADY, i * 2 + t);
+            wait(&p_ready[t], i & 1, W_MMA_PREADY, i * L + t);
             HDIT_TRACE_MMA(t, i, 1);
             if (!ok) break;
             tc_fence_after();
-            issue_pv(t, v_stage(j), i > 0, 0, 2 * kPFirst);
-            wait(&p_rest[t], i & 1, W_MMA_PREST, i * 2 + t);
+            issue_pv(t, v_stage(j), i > 0, 0, 2 * C::kPFirst);
+            wait(&p_rest[t], i & 1, W_MMA_PREST, i * L + t);
             if (!ok) break;
             tc_fence_after();
-            issue_pv(t, v_stage(j), true, 2 * kPFirst, kBlockN / 16);
+            issue_pv(t, v_stage(j), true, 2 * C::kPFirst, kBlockN / 16);
             if (releases) tc_commit(&v_empty[v_stage(j)]);  // at once: the V ring is only two deep at head_dim 128
             if (has_next) {
               if (il || t == 0) wait(&k_full[k_stage(jn)], k_phase(jn), W_MMA_KFULL, jn);
@@ -522,16 +536,14 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
       }
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kRegsSoftmax));
     // ========================= softmax / epilogue =========================
     const int t = warp >> 2;           // which half (Q tile, or KV parity when interleaved) this warpgroup owns
     const int quarter = warp & 3;      // TMEM lane quarter this warp may touch
     const int row = quarter * 32 + lane;
-    const bool active = (t == 0) || half1_active;
-    if (active) {
+    if (t < n_active) {
       const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-      const uint32_t tm_s = tmem_base + lane_base + C::kColS + t * 128;
-      const uint32_t tm_p = tmem_base + lane_base + C::kColS + t * 128;
+      const uint32_t tm_s = tmem_base + lane_base + C::kColS + t * kBlockN;  // P overwrites S
       const uint32_t tm_o = tmem_base + lane_base + C::kColO + t * D;
       const float scale_log2 = p.scale_log2;
       float m_run = -INFINITY;   // maximum the stored P and O are scaled against (log2 units)
@@ -540,28 +552,28 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
       const int first = il ? t : 0;
       const int n_mine = il ? (nblk - t + 1) / 2 : nblk;
       KvCursor cur{0, 0};
-      for (int i = 0; i < j_begin + first; ++i) cur.advance(p);
+      for (int i = 0; i < j_begin + first; ++i) cur.advance(p, kBlockN);
 
       for (int j = 0; j < n_mine; ++j) {  // j counts this half's blocks
         HDIT_TRACE_SM(0);
         // warp-uniform outcome: the tcgen05.ld/st below need the whole warp converged
         if (!__all_sync(0xffffffffu, mbar_wait_bounded(&s_full[t], j & 1, abort_flag, kSpinLimit))) {
-          report_failure(p.status, abort_flag, HDIT_ERR_PEER_TIMEOUT, W_SM_SFULL, j * 2 + t);
+          report_failure(p.status, abort_flag, HDIT_ERR_PEER_TIMEOUT, W_SM_SFULL, j * L + t);
           ok = false;
           break;
         }
         tc_fence_after();
         HDIT_TRACE_SM(1);
         const int valid = min(kBlockN, p.kv_len[cur.seg] - cur.row0);
-        for (int i = 0; i < blk_step; ++i) cur.advance(p);
-        uint32_t s[4][32];
+        for (int i = 0; i < blk_step; ++i) cur.advance(p, kBlockN);
+        uint32_t s[C::kChunks][32];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld32(tm_s + c * 32, s[c]);
+        for (int c = 0; c < C::kChunks; ++c) tmem_ld32(tm_s + c * 32, s[c]);
         tc_wait_ld();
         HDIT_TRACE_SM(2);
         if (valid < kBlockN) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
+          for (int c = 0; c < C::kChunks; ++c)
 #pragma unroll
             for (int i = 0; i < 32; ++i)
               if (c * 32 + i >= valid) s[c][i] = 0xff800000u;  // -inf
@@ -575,13 +587,15 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
           if (j > 0) {
             // O(t) is stable here: the commit that raised s_full covered the previous P V
 #pragma unroll
-            for (int c = 0; c < D / 32; ++c) {
-              uint32_t o[32];
-              tmem_ld32(tm_o + c * 32, o);
+            for (int c = 0; c < D / C::kRescaleCols; ++c) {
+              uint32_t o[C::kRescaleCols];
+              if constexpr (C::kRescaleCols == 32) tmem_ld32(tm_o + c * 32, o);
+              else tmem_ld16(tm_o + c * 16, o);
               tc_wait_ld();
 #pragma unroll
-              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-              tmem_st32(tm_o + c * 32, o);
+              for (int i = 0; i < C::kRescaleCols; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+              if constexpr (C::kRescaleCols == 32) tmem_st32(tm_o + c * 32, o);
+              else tmem_st16(tm_o + c * 16, o);
             }
           }
         };
@@ -593,7 +607,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
           const float2 neg_m2 = make_float2(-m_run, -m_run);
           float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < C::kChunks; ++c) {
             uint32_t pk[16];
 #pragma unroll
             for (int i = 0; i < 32; i += 4) {
@@ -613,8 +627,8 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
               pk[i >> 1] = pack2<FP16>(p0.x, p0.y);
               pk[(i >> 1) + 1] = pack2<FP16>(p1.x, p1.y);
             }
-            tmem_st16(tm_p + c * 16, pk);
-            if (c == kPFirst - 1) {
+            tmem_st16(tm_s + c * 16, pk);
+            if (c == C::kPFirst - 1) {
               tc_wait_st();
               tc_fence_before();
               __syncwarp();
@@ -627,7 +641,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
         {
           float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
+          for (int c = 0; c < C::kChunks; ++c)
 #pragma unroll
             for (int i = 0; i < 32; i += 8) {
               mx0 = max3(mx0, __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
@@ -685,7 +699,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
           __syncwarp();
           if (lane == 0) mbar_arrive(merge_bar);
         }
-      } else if (il && half1_active) {
+      } else if (il && n_active > 1) {
         if (ok && !__all_sync(0xffffffffu, mbar_wait_bounded(merge_bar, 0, abort_flag, kSpinLimit))) {
           report_failure(p.status, abort_flag, HDIT_ERR_PEER_TIMEOUT, W_SM_ODONE, 3);
           ok = false;
@@ -754,7 +768,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
             float f[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(o[i]) * w0;
-            if (il && half1_active) {
+            if (il && n_active > 1) {
 #pragma unroll
               for (int i = 0; i < 32; ++i) f[i] = fmaf(xo[(c * 32 + i) * 128 + row], w1, f[i]);
             }
@@ -806,7 +820,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) attn_fwd_kernel(const __grid_c
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     __syncthreads();
   }
-  if (warp == 9) {
+  if (warp == 4 * L + 1) {
     __syncwarp();
     tc_fence_after();
     tmem_dealloc(tmem_base, C::kTmemCols);
@@ -831,8 +845,8 @@ EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// Descriptor over a (B, S, H, D) tensor, box = 64 elements x 128 rows of one head.
-int encode_seg(CUtensorMap* map, unsigned char* swapped, const hdit_seg& seg, int dtype, int B, int H, int D) {
+// Descriptor over a (B, S, H, D) tensor, box = 64 elements x `rows` rows of one head.
+int encode_seg(CUtensorMap* map, unsigned char* swapped, const hdit_seg& seg, int dtype, int B, int H, int D, int rows) {
   EncodeTiledFn enc = get_encode_fn();
   if (enc == nullptr) return set_error(HDIT_ERR_CUDA, "cuTensorMapEncodeTiled entry point unavailable");
   if (seg.ptr == nullptr || seg.len <= 0) return set_error(HDIT_ERR_BAD_ARG, "segment with null pointer or len <= 0");
@@ -863,13 +877,13 @@ int encode_seg(CUtensorMap* map, unsigned char* swapped, const hdit_seg& seg, in
     strides[0] = static_cast<cuuint64_t>(sh) * 2;
     strides[1] = static_cast<cuuint64_t>(seg.stride_s) * 2;
     box[1] = 1;
-    box[2] = kBlockN;
+    box[2] = static_cast<cuuint32_t>(rows);
   } else {
     dims[1] = static_cast<cuuint64_t>(seg.len);
     dims[2] = static_cast<cuuint64_t>(H);
     strides[0] = static_cast<cuuint64_t>(seg.stride_s) * 2;
     strides[1] = static_cast<cuuint64_t>(sh) * 2;
-    box[1] = kBlockN;
+    box[1] = static_cast<cuuint32_t>(rows);
     box[2] = 1;
   }
   dims[3] = static_cast<cuuint64_t>(B);
@@ -887,18 +901,18 @@ int encode_seg(CUtensorMap* map, unsigned char* swapped, const hdit_seg& seg, in
   return HDIT_OK;
 }
 
-template <int D, bool FP16, bool IL>
+template <int D, int L, bool FP16, bool IL>
 int launch(const AttnKernelParams& kp, int grid, int grid_y, cudaStream_t stream) {
-  auto kernel = attn_fwd_kernel<D, FP16, IL>;
+  auto kernel = attn_fwd_kernel<D, L, FP16, IL>;
   // The attribute is per device: set it whenever this thread meets a new device.
   static thread_local int last_dev = -1;
   int dev = 0;
   HDIT_CUDA_OK(cudaGetDevice(&dev));
   if (dev != last_dev) {
-    HDIT_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<D>::kSmemBytes));
+    HDIT_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<D, L>::kSmemBytes));
     last_dev = dev;
   }
-  HDIT_CUDA_OK(launch_overlapped(kernel, dim3(grid, grid_y), dim3(kNumThreads), Cfg<D>::kSmemBytes, stream, 1, kp));
+  HDIT_CUDA_OK(launch_overlapped(kernel, dim3(grid, grid_y), dim3(Cfg<D, L>::kThreads), Cfg<D, L>::kSmemBytes, stream, 1, kp));
   return HDIT_OK;
 }
 
@@ -1079,35 +1093,70 @@ int attn_fwd_impl(const hdit_attn_args* a, int n_split, float* split_out, float*
     if (a->q[i].len < 0) return set_error(HDIT_ERR_BAD_ARG, "negative q segment length");
     if (a->q[i].len == 0) continue;
     if (a->q[i].len > 0x7fffff00LL) return set_error(HDIT_ERR_TOO_LARGE, "q segment too long");
-    const int rc = encode_seg(&kp.q_map[nq], &kp.q_swap[nq], a->q[i], a->dtype, a->batch, a->heads, a->head_dim);
+    const int rc = encode_seg(&kp.q_map[nq], &kp.q_swap[nq], a->q[i], a->dtype, a->batch, a->heads, a->head_dim, kBlockM);
     if (rc != HDIT_OK) return rc;
     kp.q_len[nq] = static_cast<int>(a->q[i].len);
     sq += a->q[i].len;
     ++nq;
   }
   if (nq == 0) return HDIT_OK;  // nothing to compute
+  kp.n_q_seg = nq;
+  kp.n_tiles_seg0 = (kp.q_len[0] + kBlockM - 1) / kBlockM;
+  kp.n_tiles = kp.n_tiles_seg0 + (nq > 1 ? (kp.q_len[1] + kBlockM - 1) / kBlockM : 0);
   int nkv = 0;
-  int nblk = 0;
+  int nblk2 = 0, nblk3 = 0;  // KV blocks of two lanes (128 rows) and of three (96)
   for (int i = 0; i < a->n_kv_seg; ++i) {
     if (a->k[i].len != a->v[i].len) return set_error(HDIT_ERR_SHAPE, "k and v segment lengths differ");
     if (a->k[i].len < 0) return set_error(HDIT_ERR_BAD_ARG, "negative kv segment length");
     if (a->k[i].len == 0) continue;
     if (a->k[i].len > 0x7fffff00LL) return set_error(HDIT_ERR_TOO_LARGE, "kv segment too long");
-    int rc = encode_seg(&kp.k_map[nkv], &kp.k_swap[nkv], a->k[i], a->dtype, a->batch, a->heads, a->head_dim);
-    if (rc != HDIT_OK) return rc;
-    rc = encode_seg(&kp.v_map[nkv], &kp.v_swap[nkv], a->v[i], a->dtype, a->batch, a->heads, a->head_dim);
-    if (rc != HDIT_OK) return rc;
-    kp.kv_len[nkv] = static_cast<int>(a->k[i].len);
-    nblk += static_cast<int>((a->k[i].len + kBlockN - 1) / kBlockN);
+    nblk2 += static_cast<int>((a->k[i].len + Cfg<64, 2>::kBN - 1) / Cfg<64, 2>::kBN);
+    nblk3 += static_cast<int>((a->k[i].len + Cfg<64, 3>::kBN - 1) / Cfg<64, 3>::kBN);
     ++nkv;
   }
   if (nkv == 0) return set_error(HDIT_ERR_SHAPE, "attention over an empty key/value sequence");
-  kp.n_q_seg = nq;
-  kp.n_kv_seg = nkv;
+
+  // How a CTA works: a pair of query tiles; interleaved (one tile, its two halves on the even and odd KV blocks); three
+  // tiles, head_dim 64. Fewest waves of CTAs, each weighted by its length in KV blocks of 128 rows that a pair walks.
+  // Measured at 3 heads x 4608 tokens, head_dim 128: an interleaved iteration (two KV blocks, each ring effectively half as
+  // deep) costs 1.12 paired blocks; about 6 blocks' worth of fixed cost per CTA. A block of 96 rows of three tiles costs
+  // 1.08: pair -> three tiles 349 -> 318 us at 2 x 24 heads x 4429 (6 waves of 41 blocks -> 4 of 53), 38.6 -> 26 us at 2 x 24
+  // heads x 1101 (2 waves -> 1), 112 -> 150 us at 2 x 24 heads x 1178 x 4250 (2 waves either way: the pair stays).
+  int lanes = 2;
+  if (n_split <= 1) {
+    auto waves = [&](int tiles_per_cta) {
+      const long long ctas = static_cast<long long>((kp.n_tiles + tiles_per_cta - 1) / tiles_per_cta) * a->heads * a->batch;
+      return static_cast<double>((ctas + kSmCount - 1) / kSmCount);
+    };
+    double best = waves(2) * (nblk2 + 6.0);
+    if (a->kv_interleave != 1 && nblk2 >= 2) {
+      const double t_il = waves(1) * ((nblk2 + 1) / 2 * 1.12 + 6.0);
+      if (a->kv_interleave == 2 || t_il * 1.05 < best) {
+        kp.interleave = 1;
+        best = t_il;
+      }
+    }
+    if (a->head_dim == 64 && a->kv_interleave != 2 && waves(3) * (nblk3 + 6.0) * 1.08 < best) {
+      kp.interleave = 0;
+      lanes = 3;
+    }
+  }
+  const int tiles_per_cta = kp.interleave ? 1 : lanes;
+  kp.n_groups = (kp.n_tiles + tiles_per_cta - 1) / tiles_per_cta;
+  const int nblk = lanes == 3 ? nblk3 : nblk2;
+  const int block_n = lanes == 3 ? Cfg<64, 3>::kBN : Cfg<64, 2>::kBN;
   kp.n_kv_blocks = nblk;
-  kp.n_tiles_seg0 = (kp.q_len[0] + kBlockM - 1) / kBlockM;
-  kp.n_tiles = kp.n_tiles_seg0 + (nq > 1 ? (kp.q_len[1] + kBlockM - 1) / kBlockM : 0);
-  kp.n_pairs = (kp.n_tiles + 1) / 2;
+  nkv = 0;
+  for (int i = 0; i < a->n_kv_seg; ++i) {
+    if (a->k[i].len == 0) continue;
+    int rc = encode_seg(&kp.k_map[nkv], &kp.k_swap[nkv], a->k[i], a->dtype, a->batch, a->heads, a->head_dim, block_n);
+    if (rc != HDIT_OK) return rc;
+    rc = encode_seg(&kp.v_map[nkv], &kp.v_swap[nkv], a->v[i], a->dtype, a->batch, a->heads, a->head_dim, block_n);
+    if (rc != HDIT_OK) return rc;
+    kp.kv_len[nkv] = static_cast<int>(a->k[i].len);
+    ++nkv;
+  }
+  kp.n_kv_seg = nkv;
   kp.sq_total = sq;
   const float scale = a->softmax_scale > 0.f ? a->softmax_scale : 1.0f / sqrtf(static_cast<float>(a->head_dim));
   kp.scale_log2 = scale * 1.4426950408889634f;
@@ -1153,22 +1202,7 @@ int attn_fwd_impl(const hdit_attn_args* a, int n_split, float* split_out, float*
     kp.wait_spins = static_cast<unsigned>(spins > 0xffffffffLL ? 0xffffffffLL : spins);
   }
 
-  // Interleaved mode (one Q tile per CTA, its two halves on the even and odd KV blocks): taken when it cuts
-  // the number of CTA waves, i.e. for grids smaller than the GPU. Costs are in KV blocks of one CTA.
-  if (n_split <= 1 && a->kv_interleave != 1 && nblk >= 2) {
-    const long long ctas_pair = static_cast<long long>(kp.n_pairs) * a->heads * a->batch;
-    const long long ctas_il = static_cast<long long>(kp.n_tiles) * a->heads * a->batch;
-    // measured at 3 heads x 4608 tokens, head_dim 128: an interleaved iteration (two KV blocks, each ring
-    // effectively half as deep) costs 1.12 paired blocks; about 6 blocks' worth of fixed cost per CTA
-    const double t_pair = static_cast<double>((ctas_pair + kSmCount - 1) / kSmCount) * (nblk + 6.0);
-    const double t_il = static_cast<double>((ctas_il + kSmCount - 1) / kSmCount) * ((nblk + 1) / 2 * 1.12 + 6.0);
-    if (a->kv_interleave == 2 || t_il * 1.05 < t_pair) {
-      kp.interleave = 1;
-      kp.n_pairs = kp.n_tiles;
-    }
-  }
-
-  const long long grid = static_cast<long long>(kp.n_pairs) * a->heads * a->batch;
+  const long long grid = static_cast<long long>(kp.n_groups) * a->heads * a->batch;
   if (grid > 0x7fffffffLL) return set_error(HDIT_ERR_TOO_LARGE, "grid too large");
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(a->stream);
   const bool fp16 = a->dtype == HDIT_FP16;
@@ -1186,16 +1220,17 @@ int attn_fwd_impl(const hdit_attn_args* a, int n_split, float* split_out, float*
   }
   int rc;
   const int g = static_cast<int>(grid);
-  if (kp.interleave) {
-    if (a->head_dim == 128)
-      rc = fp16 ? launch<128, true, true>(kp, g, grid_y, stream) : launch<128, false, true>(kp, g, grid_y, stream);
+  if (a->head_dim == 128) {
+    if (kp.interleave)
+      rc = fp16 ? launch<128, 2, true, true>(kp, g, grid_y, stream) : launch<128, 2, false, true>(kp, g, grid_y, stream);
     else
-      rc = fp16 ? launch<64, true, true>(kp, g, grid_y, stream) : launch<64, false, true>(kp, g, grid_y, stream);
+      rc = fp16 ? launch<128, 2, true, false>(kp, g, grid_y, stream) : launch<128, 2, false, false>(kp, g, grid_y, stream);
+  } else if (lanes == 3) {
+    rc = fp16 ? launch<64, 3, true, false>(kp, g, grid_y, stream) : launch<64, 3, false, false>(kp, g, grid_y, stream);
+  } else if (kp.interleave) {
+    rc = fp16 ? launch<64, 2, true, true>(kp, g, grid_y, stream) : launch<64, 2, false, true>(kp, g, grid_y, stream);
   } else {
-    if (a->head_dim == 128)
-      rc = fp16 ? launch<128, true, false>(kp, g, grid_y, stream) : launch<128, false, false>(kp, g, grid_y, stream);
-    else
-      rc = fp16 ? launch<64, true, false>(kp, g, grid_y, stream) : launch<64, false, false>(kp, g, grid_y, stream);
+    rc = fp16 ? launch<64, 2, true, false>(kp, g, grid_y, stream) : launch<64, 2, false, false>(kp, g, grid_y, stream);
   }
   if (rc != HDIT_OK || grid_y == 1) return rc;
   const long long n_rows = static_cast<long long>(a->batch) * sq * a->heads;

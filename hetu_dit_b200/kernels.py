@@ -228,6 +228,12 @@ def _interleave_cost(q_tiles, kv_blocks, batch, heads):
     return -(-ctas_il // _SM_COUNT) * ((kv_blocks + 1) // 2 * 1.12 + 6.0)
 
 
+def _three_tile_cost(q_tiles, kv_lens, batch, heads):
+    """The same for three query tiles per CTA over KV blocks of 96 rows (head_dim 64)."""
+    ctas = -(-q_tiles // 3) * heads * batch
+    return -(-ctas // _SM_COUNT) * (sum([-(-n // 96) for n in kv_lens]) + 6.0) * 1.08
+
+
 def _pick_kv_split(q_segs, k_segs, batch, heads, kv_interleave=0):
     """How many ways to split the KV range. One CTA per SM runs a pair of 128-row query tiles over all KV
     blocks, so the launch takes ceil(ctas / SMs) waves; splitting the KV range s ways makes waves of 1/s the
@@ -250,9 +256,11 @@ def _pick_kv_split(q_segs, k_segs, batch, heads, kv_interleave=0):
         return c if s == 1 else c + 5.0 + part_bytes * s / 1e7
 
     best, best_cost = 1, cost(1) * 0.9
+    # without a split the library itself may interleave or take three tiles per CTA; a split has to beat that too
     if kv_interleave == 0 and kv_blocks >= 2:
-        # without a split the library itself may interleave; a split has to beat that too
         best_cost = min(best_cost, _interleave_cost(q_tiles, kv_blocks, batch, heads) * 0.95)
+    if q_segs[0].shape[3] == 64:
+        best_cost = min(best_cost, _three_tile_cost(q_tiles, kv_lens, batch, heads) * 0.95)
     for s in (2, 3, 4):
         if kv_blocks // s >= 4 and cost(s) < best_cost:
             best, best_cost = s, cost(s)

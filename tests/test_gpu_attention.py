@@ -344,3 +344,51 @@ def test_ulysses_only_operator_on_one_rank(strategy):
     with pytest.raises(ValueError):
         layer(None, q.to(dev), k.to(dev), v.to(dev), joint_tensor_query=jq.to(dev), joint_tensor_key=jk.to(dev),
               joint_tensor_value=jv.to(dev), joint_strategy="none")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("sq,lens", [((300,), (1,)), ((384,), (95,)), ((257, 256), (96,)), ((290,), (97, 191)),
+                                     ((650,), (192, 193, 33)), ((600, 77), (600, 77))])
+def test_three_query_tiles_per_cta(sq, lens, dtype):
+    """Head size 64 with more heads than SMs, where a CTA takes three query tiles over 96-row KV blocks: one to three tiles
+    in the last group, tiles of both query segments in one group, one block, ragged blocks, scores that grow from block to
+    block (every lane rescales its result on the way). The oracle is given every fifth head."""
+    from torch.profiler import ProfilerActivity, profile
+    H = 160
+    gen = torch.Generator().manual_seed(sum(sq) + sum(lens))
+    qs = [_mk((1, n, H, 64), dtype, gen) * 2 for n in sq]
+    ks, vs = ([_mk((1, n, H, 64), dtype, gen) for n in lens] for _ in range(2))
+    for k in ks:
+        k *= (1 + torch.arange(k.shape[1]) // 48).view(1, -1, 1, 1).to(dtype)
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        out, lse = _run(qs, ks, vs)
+    names = {e.name for e in prof.events() if "attn_fwd_kernel" in e.name}
+    assert names and all("<64, 3," in n for n in names), names
+    hs = list(range(0, H, 5))
+    _check(out[:, :, hs], None, *([t[:, :, hs] for t in seg] for seg in (qs, ks, vs)))
+    want_lse = oa.attention_with_lse(*(torch.cat([t[:, :, hs] for t in seg], 1) for seg in (qs, ks, vs)), None)[1]
+    # 32-bit sums of 16-bit products: an error of a few 2^-24 of the largest |score|
+    assert ((lse[:, hs].cpu() - want_lse).abs() <= LSE_ATOL + 1e-5 * want_lse.abs()).all()
+
+
+def test_three_query_tiles_merge_and_scatter():
+    """The same kernel under PARTIAL_FIRST -> MERGE_FINAL and with the row scatter of its epilogue equals one shot."""
+    from hetu_dit_b200 import _C, kernels
+    dev, H = torch.device("cuda:0"), 160
+    gen = torch.Generator().manual_seed(41)
+    q = _mk((1, 300, H, 64), torch.bfloat16, gen).to(dev)
+    k1, v1, k2, v2 = (_mk((1, n, H, 64), torch.bfloat16, gen).to(dev) for n in (200, 200, 130, 130))
+    acc = torch.empty(1, 300, H, 64, device=dev)
+    acc_lse = torch.empty(1, H, 300, device=dev)
+    kernels.attn_fwd([q], [k1], [v1], mode=_C.ATTN_PARTIAL_FIRST, acc_out=acc, acc_lse=acc_lse)
+    out, lse = kernels.attn_fwd([q], [k2], [v2], mode=_C.ATTN_MERGE_FINAL, acc_out=acc, acc_lse=acc_lse, return_lse=True)
+    bufs = [torch.zeros(1, 150, H, 64, dtype=torch.bfloat16, device=dev) for _ in range(2)]
+    kernels.attn_fwd([q], [k1, k2], [v1, v2], q_rows_per_dst=[150], q_dst_row0=[0],
+                     out_dsts=kernels.RawDst([b.data_ptr() for b in bufs], bufs[0].stride()[:3]))
+    whole = kernels.attn_fwd([q], [k1, k2], [v1, v2])
+    torch.cuda.synchronize()
+    assert _C.device_status(0, clear=True)[0] == 0
+    assert torch.equal(torch.cat(bufs, 1), whole)
+    hs = list(range(0, H, 8))
+    pick = lambda *ts: [t[:, :, hs].cpu() for t in ts]
+    _check(out[:, :, hs], lse[:, hs], pick(q), pick(k1, k2), pick(v1, v2))
