@@ -310,7 +310,9 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
     nblk = min(p.n_kv_blocks - j_begin, p.kv_split_blocks);
   }
   // lane t (softmax group t): its Q tile, and which KV blocks it walks
-  const int n_active = min(L, il ? nblk : p.n_tiles - tile0);
+  const bool half1_active = il ? (nblk >= 2) : ((tile0 + 1) < p.n_tiles);
+  const bool lane2_active = L == 3 && (tile0 + 2) < p.n_tiles;
+  const int last_t = lane2_active ? 2 : half1_active ? 1 : 0;
   const int blk_step = il ? 2 : 1;
   float* const acc_out = p.acc_out + static_cast<long long>(blockIdx.y) * p.split_acc_stride;
   float* const acc_lse = p.acc_lse + static_cast<long long>(blockIdx.y) * p.split_lse_stride;
@@ -387,7 +389,8 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
           tma_prefetch_desc(&p.k_map[s]);
           tma_prefetch_desc(&p.v_map[s]);
         }
-        for (int t = 0; t < (il ? 1 : n_active); ++t) {  // interleaved: both halves share the tile in slot 0
+        for (int t = 0; t < L; ++t) {
+          if ((t == 1 && (il || !half1_active)) || (t == 2 && !lane2_active)) break;
           int seg, row0, orow;
           tile_coords(p, tile0 + t, seg, row0, orow);
           mbar_expect_tx(&q_full[t], C::kQBytes);
@@ -471,17 +474,27 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
         auto v_stage = [](int j) { return j % C::kStagesV; };
         auto v_phase = [](int j) { return static_cast<uint32_t>(j / C::kStagesV) & 1; };
 
-        // prologue: S of each lane's first block (block 0 for all, or block t of half t when interleaved)
-        for (int t = 0; t < n_active; ++t) {
-          const int j = il ? t : 0;
-          if (!il || t == 0) wait(&q_full[t], 0, W_MMA_QFULL, t);
-          if (il || t == 0) wait(&k_full[k_stage(j)], k_phase(j), W_MMA_KFULL, j);
-          if (!ok) break;
+        // prologue
+        wait(&q_full[0], 0, W_MMA_QFULL, 0);
+        wait(&k_full[0], 0, W_MMA_KFULL, 0);
+        if (ok) {
           tc_fence_after();
-          issue_qk(t, k_stage(j));
-          tc_commit(&s_full[t]);
-          if (il || t == n_active - 1) tc_commit(&k_empty[k_stage(j)]);
+          issue_qk(0, 0);
+          tc_commit(&s_full[0]);
+          if (il) tc_commit(&k_empty[0]);
         }
+        for (int t = 1; t <= last_t; ++t) {
+          const int j1 = il ? 1 : 0;
+          if (!il) wait(&q_full[t], 0, W_MMA_QFULL, t);
+          if (il) wait(&k_full[k_stage(1)], k_phase(1), W_MMA_KFULL, 1);
+          if (ok) {
+            tc_fence_after();
+            issue_qk(t, k_stage(j1));
+            tc_commit(&s_full[t]);
+            if (il) tc_commit(&k_empty[k_stage(1)]);
+          }
+        }
+        if (ok && !il) tc_commit(&k_empty[0]);
 
 #ifdef HDIT_ATTN_TRACE
         if (trace_on) {
@@ -492,13 +505,13 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
         }
 #endif
         for (int i = 0; i < n_iter && ok; ++i) {
-          for (int t = 0; t < n_active && ok; ++t) {
+          for (int t = 0; t <= last_t && ok; ++t) {
             // lane t's i-th KV block and the one after it
             const int j = il ? 2 * i + t : i;
             if (j >= nblk) break;  // interleaved, odd block count: half 1 has one block fewer
             const int jn = j + blk_step;
             const bool has_next = jn < nblk;
-            const bool releases = il || t == n_active - 1;  // the last reader of a stage hands it back
+            const bool releases = il || t == last_t;  // the last reader of a stage hands it back
             if (il || t == 0) {
               wait(&v_full[v_stage(j)], v_phase(j), W_MMA_VFULL, j);
             }
@@ -541,7 +554,8 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
     const int t = warp >> 2;           // which half (Q tile, or KV parity when interleaved) this warpgroup owns
     const int quarter = warp & 3;      // TMEM lane quarter this warp may touch
     const int row = quarter * 32 + lane;
-    if (t < n_active) {
+    const bool active = t == 0 || (t == 1 ? half1_active : lane2_active);
+    if (active) {
       const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
       const uint32_t tm_s = tmem_base + lane_base + C::kColS + t * kBlockN;  // P overwrites S
       const uint32_t tm_o = tmem_base + lane_base + C::kColO + t * D;
@@ -699,7 +713,7 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
           __syncwarp();
           if (lane == 0) mbar_arrive(merge_bar);
         }
-      } else if (il && n_active > 1) {
+      } else if (il && half1_active) {
         if (ok && !__all_sync(0xffffffffu, mbar_wait_bounded(merge_bar, 0, abort_flag, kSpinLimit))) {
           report_failure(p.status, abort_flag, HDIT_ERR_PEER_TIMEOUT, W_SM_ODONE, 3);
           ok = false;
@@ -768,7 +782,7 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
             float f[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(o[i]) * w0;
-            if (il && n_active > 1) {
+            if (il && half1_active) {
 #pragma unroll
               for (int i = 0; i < 32; ++i) f[i] = fmaf(xo[(c * 32 + i) * 128 + row], w1, f[i]);
             }

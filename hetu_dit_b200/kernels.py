@@ -835,6 +835,10 @@ def _group_cost(shapes):
 # An SM takes 4 cycles per unit of the inner dimension for a 128 x 128 block: 2.3 ns. What a separate library GEMM plus
 # tail kernel costs beyond its arithmetic, and how far the library is from the kernel's best rate.
 _NS_PER_K, _SAVED_US_PER_LAYER, _LIBRARY_RATE = 2.3e-3, 5.0, 1.15
+# One layer with a long inner dimension is what the library is best at: at the power limit its larger tiles need less energy
+# per flop than narrow ones here. 2192 rows, K = 15360, N = 3072 in a Flux-shaped step: 142 us + 9 for the tail kernel,
+# against about 180 with 192-column tiles (168 in a burst).
+_LIBRARY_RATE_LONG = 1.06
 
 
 @functools.lru_cache(maxsize=4096)
@@ -846,7 +850,8 @@ def _group_pays(shapes, k):
     rows, K = 12288: 253 / 274; 12240 + 224 rows: 671 / 660 (taken although 2 % slower alone); Q, K,
     V of 2 x (1024 + 77) rows, K = 1536: 34 / 50, of 4096 + 512 rows, K = 3072 with norm and rotation: 193 / 252."""
     cost, ideal = _group_cost(shapes)
-    return (cost - _LIBRARY_RATE * ideal) * k * _NS_PER_K <= _SAVED_US_PER_LAYER * len(shapes)
+    rate = _LIBRARY_RATE_LONG if len(shapes) == 1 and k >= 8192 else _LIBRARY_RATE
+    return (cost - rate * ideal) * k * _NS_PER_K <= _SAVED_US_PER_LAYER * len(shapes)
 
 
 def use_linear_group(items):
