@@ -312,7 +312,6 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
   // lane t (softmax group t): its Q tile, and which KV blocks it walks
   const bool half1_active = il ? (nblk >= 2) : ((tile0 + 1) < p.n_tiles);
   const bool lane2_active = L == 3 && (tile0 + 2) < p.n_tiles;
-  const int last_t = lane2_active ? 2 : half1_active ? 1 : 0;
   const int blk_step = il ? 2 : 1;
   float* const acc_out = p.acc_out + static_cast<long long>(blockIdx.y) * p.split_acc_stride;
   float* const acc_lse = p.acc_lse + static_cast<long long>(blockIdx.y) * p.split_lse_stride;
@@ -434,6 +433,7 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
         constexpr uint32_t idesc_qk = make_idesc_f16(kBlockM, kBlockN, kFmt, 0);
         constexpr uint32_t idesc_pv = make_idesc_f16(kBlockM, D, kFmt, 1);
         bool ok = true;
+        const int last_t = lane2_active ? 2 : half1_active ? 1 : 0;
         const int n_iter = il ? (nblk + 1) / 2 : nblk;
 
         // Descriptors differ from a per-tile base only in the start-address field (low word, units of
@@ -474,7 +474,9 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
         auto v_stage = [](int j) { return j % C::kStagesV; };
         auto v_phase = [](int j) { return static_cast<uint32_t>(j / C::kStagesV) & 1; };
 
-        // prologue
+        // prologue: S of each lane's first block (block 0 for all when they have tiles of their own; blocks 0 and 1 when
+        // interleaved). Written out and not as a loop over lanes, which made a pair of head_dim 64 3 % slower (112 -> 115 us
+        // at 2 x 24 heads x 1178 x 4250).
         wait(&q_full[0], 0, W_MMA_QFULL, 0);
         wait(&k_full[0], 0, W_MMA_KFULL, 0);
         if (ok) {
@@ -483,18 +485,27 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
           tc_commit(&s_full[0]);
           if (il) tc_commit(&k_empty[0]);
         }
-        for (int t = 1; t <= last_t; ++t) {
+        if (half1_active) {
           const int j1 = il ? 1 : 0;
-          if (!il) wait(&q_full[t], 0, W_MMA_QFULL, t);
+          if (!il) wait(&q_full[1], 0, W_MMA_QFULL, 1);
           if (il) wait(&k_full[k_stage(1)], k_phase(1), W_MMA_KFULL, 1);
           if (ok) {
             tc_fence_after();
-            issue_qk(t, k_stage(j1));
-            tc_commit(&s_full[t]);
+            issue_qk(1, k_stage(j1));
+            tc_commit(&s_full[1]);
             if (il) tc_commit(&k_empty[k_stage(1)]);
           }
         }
-        if (ok && !il) tc_commit(&k_empty[0]);
+        if constexpr (L == 3) {
+          if (lane2_active) {
+            wait(&q_full[2], 0, W_MMA_QFULL, 2);
+            if (ok) {
+              tc_fence_after();
+              issue_qk(2, 0);
+              tc_commit(&s_full[2]);
+            }
+          }
+        }
 
 #ifdef HDIT_ATTN_TRACE
         if (trace_on) {
@@ -511,7 +522,6 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
             if (j >= nblk) break;  // interleaved, odd block count: half 1 has one block fewer
             const int jn = j + blk_step;
             const bool has_next = jn < nblk;
-            const bool releases = il || t == last_t;  // the last reader of a stage hands it back
             if (il || t == 0) {
               wait(&v_full[v_stage(j)], v_phase(j), W_MMA_VFULL, j);
             }
@@ -525,13 +535,13 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
             if (!ok) break;
             tc_fence_after();
             issue_pv(t, v_stage(j), true, 2 * C::kPFirst, kBlockN / 16);
-            if (releases) tc_commit(&v_empty[v_stage(j)]);  // at once: the V ring is only two deep at head_dim 128
+            if (il) tc_commit(&v_empty[v_stage(j)]);  // at once: each half sees only every second block of the ring
             if (has_next) {
               if (il || t == 0) wait(&k_full[k_stage(jn)], k_phase(jn), W_MMA_KFULL, jn);
               if (!ok) break;
               issue_qk(t, k_stage(jn));
               tc_commit(&s_full[t]);
-              if (releases) tc_commit(&k_empty[k_stage(jn)]);
+              if (il) tc_commit(&k_empty[k_stage(jn)]);
             } else {
               tc_commit(&o_done[t]);
             }
@@ -554,7 +564,7 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
     const int t = warp >> 2;           // which half (Q tile, or KV parity when interleaved) this warpgroup owns
     const int quarter = warp & 3;      // TMEM lane quarter this warp may touch
     const int row = quarter * 32 + lane;
-    const bool active = t == 0 || (t == 1 ? half1_active : lane2_active);
+    const bool active = (t == 0) || (L == 3 && t == 2 ? lane2_active : half1_active);
     if (active) {
       const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
       const uint32_t tm_s = tmem_base + lane_base + C::kColS + t * kBlockN;  // P overwrites S
@@ -563,6 +573,7 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
       float m_run = -INFINITY;   // maximum the stored P and O are scaled against (log2 units)
       float l_run = 0.f;
       bool ok = true;
+      const bool last_lane = t == (lane2_active ? 2 : half1_active ? 1 : 0);
       const int first = il ? t : 0;
       const int n_mine = il ? (nblk - t + 1) / 2 : nblk;
       KvCursor cur{0, 0};
@@ -578,6 +589,14 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
         }
         tc_fence_after();
         HDIT_TRACE_SM(1);
+        // S of this block stands, so every lane's Q K^T of it and P V of the block before are done (one thread issues them in
+        // order): the last lane hands their ring stages back. Two commits fewer per block for the issuing thread, 1 to 3 % of
+        // the time at 24 heads x 4608 x 128 and 24 heads x 11056 x 128, 1 % at 2 x 24 heads x 4429 x 64. Interleaved halves
+        // commit for themselves: V held a block longer made 3 heads x 4608 x 128 33 % slower.
+        if (!il && last_lane && threadIdx.x % 128 == 0) {
+          mbar_arrive(&k_empty[j % C::kStagesK]);
+          if (j > 0) mbar_arrive(&v_empty[(j - 1) % C::kStagesV]);
+        }
         const int valid = min(kBlockN, p.kv_len[cur.seg] - cur.row0);
         for (int i = 0; i < blk_step; ++i) cur.advance(p, kBlockN);
         uint32_t s[C::kChunks][32];
