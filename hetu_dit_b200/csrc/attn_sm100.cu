@@ -506,6 +506,7 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
             }
           }
         }
+        if (ok && !il) tc_commit(&k_empty[0]);
 
 #ifdef HDIT_ATTN_TRACE
         if (trace_on) {
@@ -522,6 +523,7 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
             if (j >= nblk) break;  // interleaved, odd block count: half 1 has one block fewer
             const int jn = j + blk_step;
             const bool has_next = jn < nblk;
+            const bool releases = il || t == last_t;  // the last reader of a stage hands it back
             if (il || t == 0) {
               wait(&v_full[v_stage(j)], v_phase(j), W_MMA_VFULL, j);
             }
@@ -535,13 +537,13 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
             if (!ok) break;
             tc_fence_after();
             issue_pv(t, v_stage(j), true, 2 * C::kPFirst, kBlockN / 16);
-            if (il) tc_commit(&v_empty[v_stage(j)]);  // at once: each half sees only every second block of the ring
+            if (releases) tc_commit(&v_empty[v_stage(j)]);  // at once: the V ring is only two deep at head_dim 128
             if (has_next) {
               if (il || t == 0) wait(&k_full[k_stage(jn)], k_phase(jn), W_MMA_KFULL, jn);
               if (!ok) break;
               issue_qk(t, k_stage(jn));
               tc_commit(&s_full[t]);
-              if (il) tc_commit(&k_empty[k_stage(jn)]);
+              if (releases) tc_commit(&k_empty[k_stage(jn)]);
             } else {
               tc_commit(&o_done[t]);
             }
@@ -573,7 +575,6 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
       float m_run = -INFINITY;   // maximum the stored P and O are scaled against (log2 units)
       float l_run = 0.f;
       bool ok = true;
-      const bool last_lane = t == (lane2_active ? 2 : half1_active ? 1 : 0);
       const int first = il ? t : 0;
       const int n_mine = il ? (nblk - t + 1) / 2 : nblk;
       KvCursor cur{0, 0};
@@ -589,14 +590,6 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
         }
         tc_fence_after();
         HDIT_TRACE_SM(1);
-        // S of this block stands, so every lane's Q K^T of it and P V of the block before are done (one thread issues them in
-        // order): the last lane hands their ring stages back. Two commits fewer per block for the issuing thread, 1 to 3 % of
-        // the time at 24 heads x 4608 x 128 and 24 heads x 11056 x 128, 1 % at 2 x 24 heads x 4429 x 64. Interleaved halves
-        // commit for themselves: V held a block longer made 3 heads x 4608 x 128 33 % slower.
-        if (!il && last_lane && threadIdx.x % 128 == 0) {
-          mbar_arrive(&k_empty[j % C::kStagesK]);
-          if (j > 0) mbar_arrive(&v_empty[(j - 1) % C::kStagesV]);
-        }
         const int valid = min(kBlockN, p.kv_len[cur.seg] - cur.row0);
         for (int i = 0; i < blk_step; ++i) cur.advance(p, kBlockN);
         uint32_t s[C::kChunks][32];
