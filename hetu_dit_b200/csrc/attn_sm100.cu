@@ -24,7 +24,7 @@
 //
 // At head_dim 64 a pair leaves every unit idle for half of the time: a KV block of a tile goes S -> load -> maximum ->
 // exponentials -> P V -> next Q K^T, and with two tiles that chain sets the pace (2880 cycles per 128 x 128 block of both, 770
-// of them waiting for S; 1536 of exponentials, 768 of MMAs). The tensor memory that the narrower O leaves holds a third
+// of them waiting for S; 1536 of exponentials, 1024 of MMAs). The tensor memory that the narrower O leaves holds a third
 // tile once the KV block has 96 rows (3 * 96 + 3 * 64 columns), with 152 registers per softmax thread: 2 x 24 heads x 4429
 // tokens 349 -> 318 us, 48 heads x 12464 2.45 -> 2.36 ms, 2 x 24 heads x 1101 38.6 -> 26 us (144 CTAs instead of 240). Taken
 // by the wave rule in attn_fwd_impl(). Two CTAs per SM of two tiles and 64-row blocks each were no faster than the pair
@@ -38,7 +38,8 @@
 // The running maximum is updated lazily (only when it grows by more than 2^8),
 // so O is rescaled in TMEM rarely.
 //
-// TMEM columns: S0/P0 [0,128)  S1/P1 [128,256)  O0 [256,256+D)  O1 [256+D,256+2D).
+// TMEM columns: S0/P0 [0,128)  S1/P1 [128,256)  O0 [256,256+D)  O1 [256+D,256+2D); with three tiles S/P of tile t
+// [96t,96t+96), O [288+64t,352+64t).
 //
 // Q and K/V are lists of segments (image tokens, text tokens, ring blocks), each
 // with its own TMA descriptor, so no concatenated copy exists; a tile or block
@@ -427,7 +428,8 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
       }
     } else if (warp == 4 * L + 1) {
       // ============================ MMA issuer ============================
-      // One thread issues for all lanes.
+      // One thread issues for all lanes, in turn, which keeps their softmax groups out of phase at the special-function unit.
+      // A thread per lane lets them fall into phase: 24 heads x 4608 x 128 221 -> 284 us, 2 x 24 heads x 4429 x 64 332 -> 346.
       if (elect_one()) {
         constexpr uint32_t kFmt = FP16 ? 0u : 1u;
         constexpr uint32_t idesc_qk = make_idesc_f16(kBlockM, kBlockN, kFmt, 0);
