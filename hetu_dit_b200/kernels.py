@@ -825,7 +825,7 @@ def _group_cost(shapes):
     own, csrc/gemm_sm100.cu). Second result: the same if every SM always had work."""
     best = None
     for tm, tn, units, per_tile in ((128, 256, _SM_COUNT, 2.36), (128, 128, _SM_COUNT, 1.25), (256, 256, _SM_COUNT // 2, 2.1),
-                                    (256, 192, _SM_COUNT // 2, 1.635), (256, 128, _SM_COUNT // 2, 1.18)):
+                                    (256, 192, _SM_COUNT // 2, 1.725), (256, 128, _SM_COUNT // 2, 1.2)):
         tiles = sum(-(-m // tm) * -(-n // tn) for m, n in shapes)
         cost = -(-tiles // units) * per_tile
         best = cost if best is None else min(best, cost)
@@ -838,7 +838,7 @@ _NS_PER_K, _SAVED_US_PER_LAYER, _LIBRARY_RATE = 2.3e-3, 5.0, 1.15
 # One layer with a long inner dimension is what the library is best at: at the power limit its larger tiles need less energy
 # per flop than narrow ones here. 2192 rows, K = 15360, N = 3072 in a Flux-shaped step: 142 us + 9 for the tail kernel,
 # against about 180 with 192-column tiles (168 in a burst).
-_LIBRARY_RATE_LONG = 1.06
+_LIBRARY_RATE_LONG = 1.07
 
 
 @functools.lru_cache(maxsize=4096)
