@@ -84,8 +84,8 @@ constexpr int kMaxSmem = 232448;  // 227 KiB opt-in limit per CTA
 // rows and K = 3072, 30 : 31 : 15.2 at 1280 rows, where the clock is not held down. Pairs of 192 and 128 columns against
 // 256, us per wave: 69 : 48 : 87.5 and 18 : 12.5 : 23 at 2192 rows (K = 12288, 3072), 33.4 : 23.8 : 46 at 8858 rows and
 // K = 6144, 63 : 47 : 86 at 11056 rows and K = 12288, i.e. 1.09 and 1.16. The narrow ones count 5 % more than that: they move
-// more operand bytes per flop, which at the power limit is time. A HunyuanVideo-shaped step (10800 + 256 rows), where 192 columns
-// promise 3 % for half of the layers, took 206.2 ms with 256 and 207.1 with 192.
+// more operand bytes per flop, which at the power limit is time. In a HunyuanVideo-shaped step (10800 + 256 rows), where the waves
+// promise 3 % for half of the layers, 192 columns gave nothing (207.1 ms against 206.2 with 256, within what runs differ by).
 constexpr double kCost128x256 = 1.18, kCost128x128 = 1.25, kCost256x256 = 1.3, kCostPair = 1.05,
                  kCostPair192 = 1.15, kCostPair128 = 1.2;
 
