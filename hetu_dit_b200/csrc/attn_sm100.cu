@@ -51,6 +51,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
+#include <float.h>
 #include <math.h>
 
 #include <mutex>
@@ -574,7 +575,9 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
       const uint32_t tm_s = tmem_base + lane_base + C::kColS + t * kBlockN;  // P overwrites S
       const uint32_t tm_o = tmem_base + lane_base + C::kColO + t * D;
       const float scale_log2 = p.scale_log2;
-      float m_run = -INFINITY;   // maximum the stored P and O are scaled against (log2 units)
+      // Maximum the stored P and O are scaled against (log2 units). It starts finite: against -inf, a first block of a row
+      // with nothing but -inf in it would give NaN weights, and how far that block reaches depends on the number of tiles.
+      float m_run = -FLT_MAX;
       float l_run = 0.f;
       bool ok = true;
       const int first = il ? t : 0;
@@ -679,9 +682,9 @@ __global__ void __launch_bounds__(Cfg<D, L>::kThreads, 1) attn_fwd_kernel(const 
             }
           const float m_blk = max3(max3(mx0, mx1, mx2), mx3, mx3) * scale_log2;
           const float m_new = max3(m_run, m_blk, m_blk);
-          const bool grow = (m_new - m_run) > kRescaleThreshold;  // true on the first block (m_run = -inf)
+          const bool grow = (m_new - m_run) > kRescaleThreshold;  // true on the first block with a finite score
           if (__any_sync(0xffffffffu, grow)) rescale_to(grow, m_new);
-          l_run += m_new - m_new;  // 0, or NaN for a row with a NaN score or without a finite maximum
+          l_run += m_new - m_new;  // 0, or NaN for a row with a score of NaN or +inf
           HDIT_TRACE_SM(3);
           l_run += exp_pass();
         }

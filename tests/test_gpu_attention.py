@@ -392,3 +392,24 @@ def test_three_query_tiles_merge_and_scatter():
     hs = list(range(0, H, 8))
     pick = lambda *ts: [t[:, :, hs].cpu() for t in ts]
     _check(out[:, :, hs], lse[:, hs], pick(q), pick(k1, k2), pick(v1, v2))
+
+
+@pytest.mark.parametrize("D,H,interleave", [(64, 160, 0), (64, 8, 1), (64, 8, 2), (128, 8, 1), (128, 8, 2)])
+@pytest.mark.parametrize("n_inf", [33, 96, 127, 128, 200, 330])
+def test_leading_keys_at_minus_infinity_weigh_nothing(D, H, interleave, n_inf):
+    """Scores of -inf in front: the rows' result is that over the other keys, whether the first KV block holds only such
+    scores (96 rows where a CTA takes three query tiles, 128 elsewhere) or some. No finite score at all gives NaN, and a
+    NaN query only its own row."""
+    gen = torch.Generator().manual_seed(D + n_inf)
+    q = _mk((1, 300, H, D), torch.bfloat16, gen).abs() + 0.125
+    k, v = (_mk((1, 331, H, D), torch.bfloat16, gen) for _ in range(2))
+    k[:, :n_inf] = float("-inf")
+    kw = dict(kv_interleave=interleave, kv_split=1)
+    out, lse = _run([q], [k], [v], **kw)
+    hs = list(range(0, H, 5))
+    _check(out[:, :, hs], lse[:, hs], *([t[:, :, hs]] for t in (q, k[:, n_inf:], v[:, n_inf:])))
+    q[:, 7] = float("nan")
+    got, _ = _run([q], [k], [v], **kw)
+    assert torch.isnan(got[:, 7]).all() and torch.equal(got[:, 8:], out[:, 8:]) and torch.equal(got[:, :7], out[:, :7])
+    k[:] = float("-inf")
+    assert torch.isnan(_run([q], [k], [v], **kw)[0]).all()
