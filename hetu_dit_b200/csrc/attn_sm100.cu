@@ -68,12 +68,13 @@ constexpr uint32_t kSpinLimit = 8u * 1000u * 1000u;
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 constexpr float kLn2 = 0.69314718055994531f;
 constexpr int kSmCount = 148;
+constexpr int kMaxLanes = 3;  // softmax warpgroups of a CTA
 
 // Development aid (off in the shipped library): -DHDIT_ATTN_TRACE records SM cycle stamps of one CTA's
 // softmax and MMA phases for the first 64 KV blocks; hdit_attn_trace_read() copies them out.
 #ifdef HDIT_ATTN_TRACE
-__device__ long long g_attn_trace[2][64][8];      // [tile][block][event]
-__device__ long long g_attn_trace_mma[2][64][4];  // [tile][block][event]
+__device__ long long g_attn_trace[kMaxLanes][64][8];      // [lane][block][event]
+__device__ long long g_attn_trace_mma[kMaxLanes][64][4];  // [lane][block][event]; [0][63] the loop's start and end
 #if HDIT_ATTN_TRACE == 2  // only the loop-start / loop-end stamps of the MMA warp
 #define HDIT_TRACE_SM(ev) do {} while (0)
 #define HDIT_TRACE_MMA(tt, jj, ev) do {} while (0)
@@ -149,7 +150,7 @@ struct alignas(64) AttnKernelParams {
 // L lanes: softmax warpgroups, each with an S / P and an O tile of its own in tensor memory.
 template <int D, int L>
 struct Cfg {
-  static_assert(L == 2 || (L == 3 && D == 64), "three lanes need the tensor memory that a head of 64 leaves");
+  static_assert(L <= kMaxLanes && (L == 2 || (L == 3 && D == 64)), "three lanes need the tensor memory that a head of 64 leaves");
   static constexpr int kBN = (L == 2) ? 128 : 96;   // rows of a KV block
   static constexpr int kThreads = 128 * (L + 1);    // + 1 warpgroup holding the TMA and MMA warps
   static constexpr int kPanels = D / 64;
@@ -1060,8 +1061,8 @@ int attn_fwd_impl(const hdit_attn_args* a, int n_split, float* split_out, float*
 #ifdef HDIT_ATTN_TRACE
 extern "C" __attribute__((visibility("default"))) int hdit_attn_trace_read(long long* softmax_out, long long* mma_out) {
   using namespace hdit;
-  HDIT_CUDA_OK(cudaMemcpyFromSymbol(softmax_out, g_attn_trace, sizeof(long long) * 2 * 64 * 8));
-  HDIT_CUDA_OK(cudaMemcpyFromSymbol(mma_out, g_attn_trace_mma, sizeof(long long) * 2 * 64 * 4));
+  HDIT_CUDA_OK(cudaMemcpyFromSymbol(softmax_out, g_attn_trace, sizeof(g_attn_trace)));
+  HDIT_CUDA_OK(cudaMemcpyFromSymbol(mma_out, g_attn_trace_mma, sizeof(g_attn_trace_mma)));
   return HDIT_OK;
 }
 #endif

@@ -890,3 +890,19 @@ def test_kernels_that_start_early_read_activations_by_plain_loads():
             assert text.count("grid_dependency_wait();") == text.count("grid_dependency_release();") == n, name
     assert "if (tab.early) grid_dependency_release();" in code["copy_kernels.cu"]
     assert "hdit::copy_pieces(pieces, n, false, stream)" in code["copy_kernels.cu"]
+
+
+def test_trace_build_has_a_record_per_lane(tmp_path):
+    """-DHDIT_ATTN_TRACE: the stamps of three lanes (softmax groups) fit the arrays that the kernel stores them into."""
+    import shutil
+    import subprocess
+    if shutil.which("nvcc") is None:
+        pytest.skip("needs nvcc")
+    src = tmp_path / "trace.cu"
+    src.write_text('#include "attn_sm100.cu"\n'
+                   "static_assert(sizeof(hdit::g_attn_trace) / sizeof(hdit::g_attn_trace[0]) >= 3, \"softmax\");\n"
+                   "static_assert(sizeof(hdit::g_attn_trace_mma) / sizeof(hdit::g_attn_trace_mma[0]) >= 3, \"mma\");\n")
+    p = subprocess.run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "--expt-relaxed-constexpr",
+                        "-Xcicc", "-O0", "-DHDIT_ATTN_TRACE", "-I", os.path.join(ROOT, "hetu_dit_b200", "csrc"), "-ptx",
+                        "-o", os.devnull, str(src)], capture_output=True, text=True)
+    assert p.returncode == 0, p.stderr
