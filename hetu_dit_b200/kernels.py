@@ -819,13 +819,16 @@ def norm_rope_fits(x, head_dim, norms, rope):
                             all(t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in rope))
 
 
-def _group_cost(shapes):
+_WIDE_TILES = ((128, 256, _SM_COUNT, 2.36), (128, 128, _SM_COUNT, 1.25), (256, 256, _SM_COUNT // 2, 2.1))
+_TILES = _WIDE_TILES + ((256, 192, _SM_COUNT // 2, 1.725), (256, 128, _SM_COUNT // 2, 1.2))
+
+
+def _group_cost(shapes, tile_shapes=_TILES):
     """Time of one launch over the (rows, n) output shapes in units of one SM's work on a 128 x 128 block of output: waves
-    of output tiles times the time of a tile, smallest over the kernel's tile shapes (the constants are the library's
-    own, csrc/gemm_sm100.cu). Second result: the same if every SM always had work."""
+    of output tiles times the time of a tile, smallest over the tile shapes (rows, columns, how many at a time, time; the
+    library's own, csrc/gemm_sm100.cu). Second result: the same if every SM always had work."""
     best = None
-    for tm, tn, units, per_tile in ((128, 256, _SM_COUNT, 2.36), (128, 128, _SM_COUNT, 1.25), (256, 256, _SM_COUNT // 2, 2.1),
-                                    (256, 192, _SM_COUNT // 2, 1.725), (256, 128, _SM_COUNT // 2, 1.2)):
+    for tm, tn, units, per_tile in tile_shapes:
         tiles = sum(-(-m // tm) * -(-n // tn) for m, n in shapes)
         cost = -(-tiles // units) * per_tile
         best = cost if best is None else min(best, cost)
@@ -835,10 +838,6 @@ def _group_cost(shapes):
 # An SM takes 4 cycles per unit of the inner dimension for a 128 x 128 block: 2.3 ns. What a separate library GEMM plus
 # tail kernel costs beyond its arithmetic, and how far the library is from the kernel's best rate.
 _NS_PER_K, _SAVED_US_PER_LAYER, _LIBRARY_RATE = 2.3e-3, 5.0, 1.15
-# One layer with a long inner dimension is what the library is best at: at the power limit its larger tiles need less energy
-# per flop than narrow ones here. 2192 rows, K = 15360, N = 3072 in a Flux-shaped step: 142 us + 9 for the tail kernel,
-# against about 180 with 192-column tiles (168 in a burst).
-_LIBRARY_RATE_LONG = 1.07
 
 
 @functools.lru_cache(maxsize=4096)
@@ -848,10 +847,16 @@ def _group_pays(shapes, k):
     cost. Measured in bursts of 20 ms, us, this kernel / library: 2 layers of 1961 + 231 rows, K = 12288: 138 / 162
     (192-column tiles); K = 3072: 38 / 47; 1024 + 256 rows, K = 12288: 83 / 93; 256 + 77 rows, K = 12288: 47 / 46 (not taken); 4096 + 512
     rows, K = 12288: 253 / 274; 12240 + 224 rows: 671 / 660 (taken although 2 % slower alone); Q, K,
-    V of 2 x (1024 + 77) rows, K = 1536: 34 / 50, of 4096 + 512 rows, K = 3072 with norm and rotation: 193 / 252."""
-    cost, ideal = _group_cost(shapes)
-    rate = _LIBRARY_RATE_LONG if len(shapes) == 1 and k >= 8192 else _LIBRARY_RATE
-    return (cost - rate * ideal) * k * _NS_PER_K <= _SAVED_US_PER_LAYER * len(shapes)
+    V of 2 x (1024 + 77) rows, K = 1536: 34 / 50, of 4096 + 512 rows, K = 3072 with norm and rotation: 193 / 252.
+
+    The narrow tiles of a pair count for several layers only: for one the library has narrow tiles and split K as well.
+    One layer that they alone would bring here, kernel / library, us in bursts | in loops at the power limit: 2290 rows,
+    K = 15360, N = 3072: 150 / 141 | 179 / 169; K = 12288: 124 / 117 | 146 / 139; 2265 rows, K = 6144, N = 1536: 35 / 34;
+    498 rows, K = 3072, N = 12288: 37 / 35. One layer that 256-column tiles bring here is about even: K = 15360, N = 3072,
+    2816 rows 183 / 180 | 217 / 209; 4352: 272 / 276 | 324 / 326; 5696: 368 / 383 | 435 / 426; 7456: 480 / 489 | 556 / 566;
+    8900: 563 / 554 | 661 / 645; 14656: 925 / 924 | 1091 / 1060; 16896: 1025 / 1082 | 1236 / 1236."""
+    cost, ideal = _group_cost(shapes, _TILES if len(shapes) > 1 else _WIDE_TILES)
+    return (cost - _LIBRARY_RATE * ideal) * k * _NS_PER_K <= _SAVED_US_PER_LAYER * len(shapes)
 
 
 def use_linear_group(items):

@@ -906,3 +906,17 @@ def test_trace_build_has_a_record_per_lane(tmp_path):
                         "-Xcicc", "-O0", "-DHDIT_ATTN_TRACE", "-I", os.path.join(ROOT, "hetu_dit_b200", "csrc"), "-ptx",
                         "-o", os.devnull, str(src)], capture_output=True, text=True)
     assert p.returncode == 0, p.stderr
+
+
+@pytest.mark.parametrize("k", [12288, 15360])
+def test_one_linear_layer_takes_the_kernel_by_its_wide_tiles(k):
+    """One layer goes to the kernel where tiles of one CTA or 256 x 256 ones of a pair fill their waves, whatever its inner
+    dimension, and not for the sake of narrower tiles of a pair; several layers may."""
+    from hetu_dit_b200.kernels import _group_pays
+    for rows in (1390, 2816, 2900, 4352, 4500, 5696, 6000, 7456, 8900, 10400, 14656, 16896):
+        assert _group_pays(((rows, 3072),), k), rows
+    for rows in (720, 1969, 2192, 2290, 2304, 3340, 8192, 11056):
+        assert not _group_pays(((rows, 3072),), k), rows
+    assert not _group_pays(((498, 12288),), 3072) and not _group_pays(((2265, 1536),), 6144)
+    assert _group_pays(((1961, 3072), (231, 3072)), 12288) and _group_pays(((494, 3072), (512, 3072)), 12288)
+    assert _group_pays(((2631, 3072), (512, 3072)), 3072)
