@@ -113,6 +113,8 @@ struct GemmCfg {
   static constexpr int kColTeams = (kHalves == 1 && (PAIR || BN == 256)) ? 2 : 1;
   static constexpr int kPieces = BN / 64;                                    // 64-column pieces of the accumulator
   static constexpr int kTeamPieces = (kPieces + kColTeams - 1) / kColTeams;  // the last team may have fewer
+  static constexpr bool kEvenTeams = kPieces % kColTeams == 0;
+  static constexpr bool kMidHead = kTeamPieces == 1;  // a team may begin in the middle of a head of 128
   static constexpr int kEpiWarps = 4 * kHalves * kColTeams;
   static constexpr int kThreads = 64 + 32 * kEpiWarps;
   static constexpr int kTileRows = PAIR ? 2 * BM : BM;     // rows of the scheduling unit's tile
@@ -572,9 +574,15 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
     const int quarter = warp & 3;  // the TMEM lanes this warp may read: [32 * quarter, 32 * quarter + 32)
     const int team = (warp - 2) >> 2;
     const int half = C::kColTeams == 1 ? team : 0;  // which 128-row block of the tile
-    // 64-column pieces of this warp
+    // 64-column pieces of this warp. How the compiler gets on with the loop over them depends on the type: with a bound that
+    // is not a constant and the form of head_stats() for teams that begin inside a head, fp16 kernels spill (Q, K, V of 8300 +
+    // 333 rows, K = 1536: 141.3 us against 137.0; 5532 x 6144 + GELU 83.4 / 82.5), bf16 ones of 256 columns spill less than
+    // without (136.0 / 138.3; 83.3 / 84.6) and narrow ones more (1024 + 256 rows, K = 3072: 70.7 / 69.7).
+    constexpr bool kGeneralLoop = BN == 256 && !FP16;
     const int c0 = C::kColTeams == 1 ? 0 : team * C::kTeamPieces;
-    const int c1 = C::kColTeams == 1 ? C::kPieces : min(C::kPieces, c0 + C::kTeamPieces);
+    const int c1 = C::kColTeams == 1               ? C::kPieces
+                   : C::kEvenTeams && !kGeneralLoop ? c0 + C::kTeamPieces
+                                                    : min(C::kPieces, c0 + C::kTeamPieces);
     uint8_t* staging = staging_base + (warp - 2) * 4096;
     const int sub_row = lane >> 3, chunk = lane & 7;  // store phase: 4 rows per instruction, 8 lanes per row
     uint32_t local = 0;
@@ -608,9 +616,13 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, PAIR>::kThreads, 1)
       float2 stats = make_float2(0.f, 0.f);
 #pragma unroll 1
       for (int c = c0; c < c1; ++c) {
-        const int head0 = (c * 64) & ~(im.head_dim - 1);  // a team may begin in the middle of a head
-        if (im.epilogue == HDIT_GEMM_BIAS_NORM_ROPE && im.norm != 0 && (c == c0 || head0 == c * 64))
-          stats = head_stats<FP16>(im, taddr + head0, n_t * BN + head0);
+        if constexpr (C::kMidHead || kGeneralLoop) {
+          const int head0 = (c * 64) & ~(im.head_dim - 1);
+          if (im.epilogue == HDIT_GEMM_BIAS_NORM_ROPE && im.norm != 0 && (c == c0 || head0 == c * 64))
+            stats = head_stats<FP16>(im, taddr + head0, n_t * BN + head0);
+        } else if (im.epilogue == HDIT_GEMM_BIAS_NORM_ROPE && im.norm != 0 && ((c * 64) & (im.head_dim - 1)) == 0) {
+          stats = head_stats<FP16>(im, taddr + c * 64, n_t * BN + c * 64);
+        }
         uint32_t r[64];
         tmem_ld32(taddr + c * 64, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
         tmem_ld32(taddr + c * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
