@@ -820,19 +820,20 @@ def norm_rope_fits(x, head_dim, norms, rope):
 
 
 _WIDE_TILES = ((128, 256, _SM_COUNT, 2.36), (128, 128, _SM_COUNT, 1.25), (256, 256, _SM_COUNT // 2, 2.1))
-_TILES = _WIDE_TILES + ((256, 192, _SM_COUNT // 2, 1.725), (256, 128, _SM_COUNT // 2, 1.2))
+_TILES_WIDE_HEADS = _WIDE_TILES + ((256, 128, _SM_COUNT // 2, 1.2),)  # 192 columns do not hold whole heads of 128
+_TILES = _TILES_WIDE_HEADS + ((256, 192, _SM_COUNT // 2, 1.725),)
 
 
 def _group_cost(shapes, tile_shapes=_TILES):
-    """Time of one launch over the (rows, n) output shapes in units of one SM's work on a 128 x 128 block of output: waves
-    of output tiles times the time of a tile, smallest over the tile shapes (rows, columns, how many at a time, time; the
-    library's own, csrc/gemm_sm100.cu). Second result: the same if every SM always had work."""
+    """Time of one launch over the (rows, n, ...) output shapes in units of one SM's work on a 128 x 128 block of output:
+    waves of output tiles times the time of a tile, smallest over the tile shapes (rows, columns, how many at a time, time;
+    the library's own, csrc/gemm_sm100.cu). Second result: the same if every SM always had work."""
     best = None
     for tm, tn, units, per_tile in tile_shapes:
-        tiles = sum(-(-m // tm) * -(-n // tn) for m, n in shapes)
+        tiles = sum(-(-m // tm) * -(-n // tn) for m, n, *_ in shapes)
         cost = -(-tiles // units) * per_tile
         best = cost if best is None else min(best, cost)
-    return best, sum(m * n for m, n in shapes) / 16384.0 / _SM_COUNT
+    return best, sum(m * n for m, n, *_ in shapes) / 16384.0 / _SM_COUNT
 
 
 # An SM takes 4 cycles per unit of the inner dimension for a 128 x 128 block: 2.3 ns. What a separate library GEMM plus
@@ -842,12 +843,13 @@ _NS_PER_K, _SAVED_US_PER_LAYER, _LIBRARY_RATE = 2.3e-3, 5.0, 1.15
 
 @functools.lru_cache(maxsize=4096)
 def _group_pays(shapes, k):
-    """Whether one launch over these outputs beats a library GEMM and a tail kernel per layer: what the partly filled last
-    wave wastes (the library splits K there) has to stay below what the launches and the extra pass over the output
-    cost. Measured in bursts of 20 ms, us, this kernel / library: 2 layers of 1961 + 231 rows, K = 12288: 138 / 162
-    (192-column tiles); K = 3072: 38 / 47; 1024 + 256 rows, K = 12288: 83 / 93; 256 + 77 rows, K = 12288: 47 / 46 (not taken); 4096 + 512
-    rows, K = 12288: 253 / 274; 12240 + 224 rows: 671 / 660 (taken although 2 % slower alone); Q, K,
-    V of 2 x (1024 + 77) rows, K = 1536: 34 / 50, of 4096 + 512 rows, K = 3072 with norm and rotation: 193 / 252.
+    """Whether one launch over these outputs, (rows, n) each or (rows, n, 128) with a norm + rotation tail over heads of
+    128, beats a library GEMM and a tail kernel per layer: what the partly filled last wave wastes (the library splits K
+    there) has to stay below what the launches and the extra pass over the output cost. Measured in bursts of 20 ms, us,
+    this kernel / library: 2 layers of 1961 + 231 rows, K = 12288: 138 / 162 (192-column tiles); K = 3072: 38 / 47; 1024 +
+    256 rows, K = 12288: 83 / 93; 256 + 77 rows, K = 12288: 47 / 46 (not taken); 4096 + 512 rows, K = 12288: 253 / 274;
+    12240 + 224 rows: 671 / 660 (taken although 2 % slower alone); Q, K, V of 2 x (1024 + 77) rows, K = 1536: 34 / 50, of
+    4096 + 512 rows, K = 3072 with norm and rotation: 193 / 252.
 
     The narrow tiles of a pair count for several layers only: for one the library has narrow tiles and split K as well.
     One layer that they alone would bring here, kernel / library, us in bursts | in loops at the power limit: 2290 rows,
@@ -855,7 +857,8 @@ def _group_pays(shapes, k):
     498 rows, K = 3072, N = 12288: 37 / 35. One layer that 256-column tiles bring here is about even: K = 15360, N = 3072,
     2816 rows 183 / 180 | 217 / 209; 4352: 272 / 276 | 324 / 326; 5696: 368 / 383 | 435 / 426; 7456: 480 / 489 | 556 / 566;
     8900: 563 / 554 | 661 / 645; 14656: 925 / 924 | 1091 / 1060; 16896: 1025 / 1082 | 1236 / 1236."""
-    cost, ideal = _group_cost(shapes, _TILES if len(shapes) > 1 else _WIDE_TILES)
+    wide_heads = any([len(s) == 3 for s in shapes])
+    cost, ideal = _group_cost(shapes, _WIDE_TILES if len(shapes) == 1 else _TILES_WIDE_HEADS if wide_heads else _TILES)
     return (cost - _LIBRARY_RATE * ideal) * k * _NS_PER_K <= _SAVED_US_PER_LAYER * len(shapes)
 
 
@@ -867,7 +870,8 @@ def use_linear_group(items):
             return False
         B, S, k = it.x.shape
         n = it.weight.shape[0]
-        shapes += [(B * S, n)] if it._even() else [(S, n)] * B
+        tail = (128,) if it.epilogue == "norm_rope" and it.head_dim == 128 else ()
+        shapes += [(B * S, n, *tail)] if it._even() else [(S, n, *tail)] * B
         inputs[id(it.x)] = B * S
     return 1 <= len(shapes) <= _C.MAX_LINEAR_ITEMS and \
         FUSED_LINEAR_MIN_ROWS <= sum(inputs.values()) <= FUSED_LINEAR_MAX_ROWS and _group_pays(tuple(shapes), k)

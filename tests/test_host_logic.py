@@ -937,3 +937,62 @@ def test_fp16_linear_kernels_keep_their_registers(tmp_path):
                              p.stdout + p.stderr))
     fp16 = {name: int(n) for name, n in spills.items() if name.endswith("Lb1E")}
     assert len(fp16) == 6 and not any(fp16.values()), spills
+
+
+def _source(name):
+    with open(os.path.join(ROOT, "hetu_dit_b200", "csrc", name)) as f:
+        return f.read()
+
+
+def test_wave_rules_are_the_librarys():
+    """The costs that the wrappers count waves with are the ones that the library chooses by."""
+    from hetu_dit_b200 import kernels
+    gemm, attn = _source("gemm_sm100.cu"), _source("attn_sm100.cu")
+    per_block = {n: float(x) for n, x in re.findall(r"\b(kCost\w+) = ([\d.]+)", gemm)}
+    table = re.search(r"const Cand cand\[\d\] = \{(.*?)\};", gemm, re.S).group(1)
+    cand = [(int(r), int(c), int(u), float(f) * per_block[n])
+            for s, r, c, u, f, n in re.findall(r"\{(\d), (\d+), (\d+), (\d), ([\d.]+) \* (\w+)\}", table) if s != "2"]
+    assert len(cand) == 5  # the library takes 256 x 256 tiles of one CTA only on request
+    for shapes in [((m, n),) for m in (1, 130, 333, 1101, 2192, 4608, 11056) for n in (1536, 3072, 12288)] + \
+            [((4096, 3072),) * 3 + ((512, 3072),) * 3, ((1961, 3072), (231, 3072)), ((600, 1536),) * 5]:
+        for wide in (False, True):
+            best = min(-(-sum(-(-m // r) * -(-n // c) for m, n in shapes) // (148 // u)) * t
+                       for r, c, u, t in cand if not (wide and c == 192))
+            mine = kernels._TILES_WIDE_HEADS if wide else kernels._TILES
+            assert kernels._group_cost(shapes, mine)[0] == pytest.approx(best, rel=1e-12)
+    fixed, factor = map(float, re.search(r"waves\(3\) \* \(nblk3 \+ ([\d.]+)\) \* ([\d.]+) < best", attn).groups())
+    assert kernels._three_tile_cost(35, [4096, 333], 2, 24) == pytest.approx(-(-12 * 48 // 148) * (43 + 4 + fixed) * factor)
+    step, fixed = map(float, re.search(r"waves\(1\) \* \(\(nblk2 \+ 1\) / 2 \* ([\d.]+) \+ ([\d.]+)\)", attn).groups())
+    assert kernels._interleave_cost(36, 37, 1, 12) == pytest.approx(3 * (19 * step + fixed))
+
+
+def test_three_tiles_compete_with_a_kv_split():
+    """Heads of 64: a split of the KV range has to beat three query tiles per CTA as well."""
+    from hetu_dit_b200.kernels import _pick_kv_split
+
+    class T:
+        def __init__(self, s, d):
+            self.shape = (1, s, 1, d)
+
+    # 3 query tiles: 160 pairs in two waves that a split by 3 or more would balance; 80 CTAs of three tiles are one wave
+    for d, split in ((64, 1), (128, 3)):
+        assert _pick_kv_split([T(384, d)], [T(8192, d)], 1, 80, kv_interleave=1) == split, d
+
+
+def test_wide_heads_do_not_count_192_columns():
+    """Q, K, V of 1247 rows, hidden size 5120: 192-column tiles would pay, which heads of 128 cannot take."""
+    from hetu_dit_b200 import kernels
+
+    class X:
+        shape = (1, 1247, 5120)
+
+        def stride(self, i=None):
+            return (1247 * 5120, 5120, 1) if i is None else (1247 * 5120, 5120, 1)[i]
+
+    class Layer:
+        weight, bias = torch.empty(5120, 1), None
+
+    x = X()
+    for head_dim, pays in ((64, True), (128, False)):
+        items = [kernels.Lin(x, Layer, "norm_rope", head_dim=head_dim) for _ in range(3)]
+        assert kernels.use_linear_group(items) is pays
