@@ -346,6 +346,15 @@ def test_ulysses_only_operator_on_one_rank(strategy):
               joint_tensor_value=jv.to(dev), joint_strategy="none")
 
 
+def _attn_kernels(call):
+    """What call() returns and the names of the attention kernels that it launched."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        result = call()
+        torch.cuda.synchronize()
+    return result, {e.name for e in prof.events() if "attn_fwd_kernel" in e.name}
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("sq,lens", [((300,), (1,)), ((384,), (95,)), ((257, 256), (96,)), ((290,), (97, 191)),
                                      ((650,), (192, 193, 33)), ((600, 77), (600, 77))])
@@ -353,21 +362,19 @@ def test_three_query_tiles_per_cta(sq, lens, dtype):
     """Head size 64 with more heads than SMs, where a CTA takes three query tiles over 96-row KV blocks: one to three tiles
     in the last group, tiles of both query segments in one group, one block, ragged blocks, scores that grow from block to
     block (every lane rescales its result on the way). The oracle is given every fifth head."""
-    from torch.profiler import ProfilerActivity, profile
     H = 160
     gen = torch.Generator().manual_seed(sum(sq) + sum(lens))
     qs = [_mk((1, n, H, 64), dtype, gen) * 2 for n in sq]
     ks, vs = ([_mk((1, n, H, 64), dtype, gen) for n in lens] for _ in range(2))
     for k in ks:
         k *= (1 + torch.arange(k.shape[1]) // 48).view(1, -1, 1, 1).to(dtype)
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        out, lse = _run(qs, ks, vs)
-    names = {e.name for e in prof.events() if "attn_fwd_kernel" in e.name}
+    (out, lse), names = _attn_kernels(lambda: _run(qs, ks, vs))
     assert names and all("<64, 3," in n for n in names), names
     hs = list(range(0, H, 5))
     _check(out[:, :, hs], None, *([t[:, :, hs] for t in seg] for seg in (qs, ks, vs)))
     want_lse = oa.attention_with_lse(*(torch.cat([t[:, :, hs] for t in seg], 1) for seg in (qs, ks, vs)), None)[1]
-    # 32-bit sums of 16-bit products: an error of a few 2^-24 of the largest |score|
+    # the kernel's and the oracle's 32-bit sums of 64 products: up to 2 * 64 * 2^-24 = 7.6e-6 of |score|, and the roundings of
+    # scale and logarithm
     assert ((lse[:, hs].cpu() - want_lse).abs() <= LSE_ATOL + 1e-5 * want_lse.abs()).all()
 
 
@@ -380,18 +387,44 @@ def test_three_query_tiles_merge_and_scatter():
     k1, v1, k2, v2 = (_mk((1, n, H, 64), torch.bfloat16, gen).to(dev) for n in (200, 200, 130, 130))
     acc = torch.empty(1, 300, H, 64, device=dev)
     acc_lse = torch.empty(1, H, 300, device=dev)
-    kernels.attn_fwd([q], [k1], [v1], mode=_C.ATTN_PARTIAL_FIRST, acc_out=acc, acc_lse=acc_lse)
-    out, lse = kernels.attn_fwd([q], [k2], [v2], mode=_C.ATTN_MERGE_FINAL, acc_out=acc, acc_lse=acc_lse, return_lse=True)
     bufs = [torch.zeros(1, 150, H, 64, dtype=torch.bfloat16, device=dev) for _ in range(2)]
-    kernels.attn_fwd([q], [k1, k2], [v1, v2], q_rows_per_dst=[150], q_dst_row0=[0],
-                     out_dsts=kernels.RawDst([b.data_ptr() for b in bufs], bufs[0].stride()[:3]))
-    whole = kernels.attn_fwd([q], [k1, k2], [v1, v2])
-    torch.cuda.synchronize()
+
+    def run():
+        kernels.attn_fwd([q], [k1], [v1], mode=_C.ATTN_PARTIAL_FIRST, acc_out=acc, acc_lse=acc_lse)
+        merged = kernels.attn_fwd([q], [k2], [v2], mode=_C.ATTN_MERGE_FINAL, acc_out=acc, acc_lse=acc_lse, return_lse=True)
+        kernels.attn_fwd([q], [k1, k2], [v1, v2], q_rows_per_dst=[150], q_dst_row0=[0],
+                         out_dsts=kernels.RawDst([b.data_ptr() for b in bufs], bufs[0].stride()[:3]))
+        return merged, kernels.attn_fwd([q], [k1, k2], [v1, v2])
+
+    ((out, lse), whole), names = _attn_kernels(run)
+    assert names and all("<64, 3," in n for n in names), names
     assert _C.device_status(0, clear=True)[0] == 0
     assert torch.equal(torch.cat(bufs, 1), whole)
     hs = list(range(0, H, 8))
     pick = lambda *ts: [t[:, :, hs].cpu() for t in ts]
     _check(out[:, :, hs], lse[:, hs], pick(q), pick(k1, k2), pick(v1, v2))
+
+
+@pytest.mark.parametrize("which", ["q", "k", "v", "qkv"])
+def test_three_query_tiles_layouts(which):
+    """Head-major tensors (descriptors with sequence and head swapped), two batch entries and a result in the middle of a
+    wider buffer: the bits of contiguous tensors, and the oracle's values."""
+    from hetu_dit_b200 import kernels
+    dev, H = torch.device("cuda:0"), 80
+    gen = torch.Generator().manual_seed(43)
+    qs = [_mk((2, n, H, 64), torch.bfloat16, gen) for n in (250, 77)]
+    ks, vs = ([_mk((2, n, H, 64), torch.bfloat16, gen) for n in (200, 130)] for _ in range(2))
+    (out, lse), names = _attn_kernels(lambda: _run(qs, ks, vs))
+    swap = lambda ts, name: [t.to(dev).transpose(1, 2).contiguous().transpose(1, 2) if name in which else t.to(dev) for t in ts]
+    wide = torch.full((2, 340, H + 2, 64), 3.0, dtype=torch.bfloat16, device=dev)
+    got, more = _attn_kernels(lambda: kernels.attn_fwd(swap(qs, "q"), swap(ks, "k"), swap(vs, "v"), out=wide[:, 5:332, 1:H + 1]))
+    assert names and more and all("<64, 3," in n for n in names | more), names | more
+    assert torch.equal(got, out)
+    want = torch.full_like(wide, 3.0)
+    want[:, 5:332, 1:H + 1] = out
+    assert torch.equal(wide, want)
+    hs = list(range(0, H, 8))
+    _check(out[:, :, hs], lse[:, hs], *([t[:, :, hs] for t in seg] for seg in (qs, ks, vs)))
 
 
 @pytest.mark.parametrize("D,H,interleave", [(64, 160, 0), (64, 8, 1), (64, 8, 2), (128, 8, 1), (128, 8, 2)])

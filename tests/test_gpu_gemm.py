@@ -230,6 +230,15 @@ def test_linear_group_on_row_slices_of_a_batch(dtype):
     assert _C.device_status(0, clear=True)[0] == 0
 
 
+def _linear_kernels(call):
+    """What call() returns and the names of the linear kernels that it launched."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        result = call()
+        torch.cuda.synchronize()
+    return result, {e.name for e in prof.events() if "linear_fused_kernel" in e.name}
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("width,B,S,K,N", [(192, 1, 256, 64, 384), (192, 1, 250, 200, 376), (192, 1, 129, 1160, 328),
                                            (192, 2, 250, 3072, 1152), (128, 1, 256, 64, 256), (128, 1, 140, 200, 136),
@@ -238,14 +247,11 @@ def test_narrow_tiles_of_a_cta_pair(width, B, S, K, N, dtype):
     """Sizes for which a launch on four SMs takes 256 x 192 or 256 x 128 tiles of a CTA pair: every tail, ragged rows and
     columns, and (more tiles than pairs) both accumulators in turn. The order of sums is that of 256 x 256 tiles, so the
     bits are too."""
-    from torch.profiler import ProfilerActivity, profile
     from hetu_dit_b200 import _C, kernels
     x, w, b, res, gate = _inputs(B, S, K, N, dtype, K + N)
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        got = {ep: kernels.linear_fused(x, w, b, epilogue=ep, residual=res, gate=gate, max_ctas=4)
-               for ep in ("bias", "gelu_tanh", "gate_residual")}
-        torch.cuda.synchronize()
-    names = {e.name for e in prof.events() if "linear_fused_kernel" in e.name}
+    got, names = _linear_kernels(lambda: {
+        ep: kernels.linear_fused(x, w, b, epilogue=ep, residual=res, gate=gate, max_ctas=4)
+        for ep in ("bias", "gelu_tanh", "gate_residual")})
     assert names and all(f"<128, {width}, true" in n for n in names), names
     for ep, y in got.items():
         _check(y, _want(x, w, b, ep, res, gate))
@@ -258,7 +264,8 @@ def test_narrow_tiles_of_a_cta_pair(width, B, S, K, N, dtype):
 @pytest.mark.parametrize("S", [130, 250, 520])
 def test_norm_rope_tail_on_narrow_tiles(D, norm, rope, S):
     """The norm and rotation tail where a tile is 192 columns (heads of 64) or 128 columns wide (either head size; a warp
-    team may begin in the middle of a head): the bits of 256-column tiles."""
+    team may begin in the middle of a head): the bits of 256-column tiles. Each width runs for some number of SMs, by the
+    kernels' names, except 128 columns at heads of 64 and three rows of tiles."""
     from hetu_dit_b200 import _C, kernels
     lin, x, nrm, rp = _group_case(D, norm, rope, S, 1, torch.bfloat16, 7 * D + S)
     gen = torch.Generator().manual_seed(4)
@@ -266,8 +273,11 @@ def test_norm_rope_tail_on_narrow_tiles(D, norm, rope, S):
     with torch.no_grad():
         items = lambda: [kernels.Lin(x, lin, "norm_rope", head_dim=D, norm=nrm, rope=rp)]
         want, = kernels.linear_group(items(), cos, sin, cta_pair=2)
+        seen = set()
         for ctas in (4, 6, 8, 12):
-            got, = kernels.linear_group(items(), cos, sin, max_ctas=ctas)
+            (got,), names = _linear_kernels(lambda: kernels.linear_group(items(), cos, sin, max_ctas=ctas))
             assert torch.equal(got, want), ctas
+            seen |= {w for w in (128, 192) if any(f"<128, {w}, true" in n for n in names)}
+    assert seen == ({128} if D == 128 else {192} if S == 520 else {128, 192})
     torch.cuda.synchronize()
     assert _C.device_status(0, clear=True)[0] == 0
