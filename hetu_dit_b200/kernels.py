@@ -248,7 +248,8 @@ def _pick_kv_split(q_segs, k_segs, batch, heads, kv_interleave=0):
         return 1
     if kv_interleave == 2:
         return 1
-    part_bytes = batch * sum(q_lens) * heads * q_segs[0].shape[3] * 4
+    head_dim = q_segs[0].shape[3]
+    part_bytes = batch * sum(q_lens) * heads * head_dim * 4
 
     def cost(s):
         waves = -(-ctas * s // _SM_COUNT)
@@ -256,14 +257,15 @@ def _pick_kv_split(q_segs, k_segs, batch, heads, kv_interleave=0):
         return c if s == 1 else c + 5.0 + part_bytes * s / 1e7
 
     best, best_cost = 1, cost(1) * 0.9
-    # without a split the library itself may interleave or take three tiles per CTA; a split has to beat that too
     if kv_interleave == 0 and kv_blocks >= 2:
+        # without a split the library itself may interleave; a split has to beat that too
         best_cost = min(best_cost, _interleave_cost(q_tiles, kv_blocks, batch, heads) * 0.95)
-    if q_segs[0].shape[3] == 64:
-        best_cost = min(best_cost, _three_tile_cost(q_tiles, kv_lens, batch, heads) * 0.95)
     for s in (2, 3, 4):
         if kv_blocks // s >= 4 and cost(s) < best_cost:
             best, best_cost = s, cost(s)
+    # or take three tiles per CTA: asked last, since most calls of a few microseconds have no split to weigh it against
+    if best > 1 and head_dim == 64 and best_cost >= _three_tile_cost(q_tiles, kv_lens, batch, heads) * 0.95:
+        return 1
     return best
 
 

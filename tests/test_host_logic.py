@@ -966,8 +966,10 @@ def test_wave_rules_are_the_librarys():
     assert kernels._interleave_cost(36, 37, 1, 12) == pytest.approx(3 * (19 * step + fixed))
 
 
-def test_three_tiles_compete_with_a_kv_split():
-    """Heads of 64: a split of the KV range has to beat three query tiles per CTA as well."""
+def test_three_tiles_compete_with_a_kv_split(monkeypatch):
+    """Heads of 64: a split of the KV range has to beat three query tiles per CTA as well, whose cost a call without a
+    split to choose does not pay for."""
+    from hetu_dit_b200 import kernels
     from hetu_dit_b200.kernels import _pick_kv_split
 
     class T:
@@ -977,6 +979,10 @@ def test_three_tiles_compete_with_a_kv_split():
     # 3 query tiles: 160 pairs in two waves that a split by 3 or more would balance; 80 CTAs of three tiles are one wave
     for d, split in ((64, 1), (128, 3)):
         assert _pick_kv_split([T(384, d)], [T(8192, d)], 1, 80, kv_interleave=1) == split, d
+    asked = []
+    monkeypatch.setattr(kernels, "_three_tile_cost", lambda *args: asked.append(args) or 0.0)
+    assert _pick_kv_split([T(1178, 64)], [T(4250, 64)], 2, 24) == 1 and _pick_kv_split([T(4608, 64)], [T(4608, 64)], 1, 24) == 1
+    assert asked == []
 
 
 def test_wide_heads_do_not_count_192_columns():
