@@ -25,8 +25,10 @@
 // At head_dim 64 a pair leaves every unit idle for half of the time: a KV block of a tile goes S -> load -> maximum ->
 // exponentials -> P V -> next Q K^T, and with two tiles that chain sets the pace (2880 cycles per 128 x 128 block of both, 770
 // of them waiting for S; 1536 of exponentials, 1024 of MMAs). The tensor memory that the narrower O leaves holds a third
-// tile once the KV block has 96 rows (3 * 96 + 3 * 64 columns), with 152 registers per softmax thread: 2 x 24 heads x 4429
-// tokens 349 -> 318 us, 48 heads x 12464 2.45 -> 2.36 ms, 2 x 24 heads x 1101 38.6 -> 26 us (144 CTAs instead of 240). Taken
+// tile once the KV block has 96 rows (3 * 96 + 3 * 64 columns), with 152 registers per softmax thread. In bursts of 20 ms | in
+// loops at the power limit: 2 x 24 heads x 4429 tokens 344 -> 317 us | 364 -> 342, 48 heads x 12464 2.33 -> 2.24 ms | 2.56 ->
+// 2.49, 2 x 24 heads x 1101 41 -> 29 us (144 CTAs instead of 240). A block of all three takes 2900 cycles, which the issuing
+// thread fills: 436 waiting for P, 1436 in the lanes' turns, 1027 between them; a softmax group waits 890 to 1170 for S. Taken
 // by the wave rule in attn_fwd_impl(). Two CTAs per SM of two tiles and 64-row blocks each were no faster than the pair
 // (349 us), one CTA with two S buffers per tile slower (382; head_dim 128: 220 -> 268 us at 24 heads x 4608).
 //
@@ -187,11 +189,11 @@ struct Cfg {
   static constexpr int kPFirst = (L == 2) ? 2 : 1;
   // Of every 8 scores, how many take the polynomial exp2 on the FMA pipe instead of ex2 on the special-function unit
   // (16 per clock and SM). At head_dim 64 a KV block has as many scores as at 128 and half the MMAs, so the
-  // special-function unit is what both softmax groups compete for: two of eight moved off it took 5 % off 24 heads x 4429
-  // tokens, batch 2 (now 349 us in a burst, 362 us in a loop at 1845 MHz), and 7 % off 48 heads x 11.4 k x 33.7 k (5.71 ms,
-  // 6.25 ms at 1785 MHz); four of eight are slower (the FMA and ALU work of a pair, 25 cycles of a warp, then exceeds the 16
-  // cycles of its two ex2). At head_dim 128 it is neutral in long runs (24 x 4608, 1 %) and 4 % slower where the SMs run at
-  // full clock (3 x 4608).
+  // special-function unit is what the softmax groups compete for. Decided with two lanes: two of eight moved off it took 5 %
+  // off 24 heads x 4429 tokens, batch 2 (to 349 us in a burst, 362 us in a loop at 1845 MHz), and 7 % off 48 heads x 11.4 k x
+  // 33.7 k (to 5.71 ms, 6.25 ms at 1785 MHz); four of eight are slower (the FMA and ALU work of a pair, 25 cycles of a warp,
+  // then exceeds the 16 cycles of its two ex2). Three lanes have the same share, not varied there. At head_dim 128 it is
+  // neutral in long runs (24 x 4608, 1 %) and 4 % slower where the SMs run at full clock (3 x 4608).
   static constexpr int kPoly8 = (D == 64) ? 2 : 0;
 };
 
@@ -1152,7 +1154,7 @@ int attn_fwd_impl(const hdit_attn_args* a, int n_split, float* split_out, float*
   // tiles, head_dim 64. Fewest waves of CTAs, each weighted by its length in KV blocks of 128 rows that a pair walks.
   // Measured at 3 heads x 4608 tokens, head_dim 128: an interleaved iteration (two KV blocks, each ring effectively half as
   // deep) costs 1.12 paired blocks; about 6 blocks' worth of fixed cost per CTA. A block of 96 rows of three tiles costs
-  // 1.08: pair -> three tiles 349 -> 318 us at 2 x 24 heads x 4429 (6 waves of 41 blocks -> 4 of 53), 38.6 -> 26 us at 2 x 24
+  // 1.08: pair -> three tiles 344 -> 317 us at 2 x 24 heads x 4429 (6 waves of 41 blocks -> 4 of 53), 41 -> 29 us at 2 x 24
   // heads x 1101 (2 waves -> 1), 112 -> 150 us at 2 x 24 heads x 1178 x 4250 (2 waves either way: the pair stays).
   int lanes = 2;
   if (n_split <= 1) {

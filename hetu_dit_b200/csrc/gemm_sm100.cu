@@ -41,12 +41,13 @@
 //                         the even CTA's barrier, and tcgen05.commit multicasts "stage consumed" / "accumulator
 //                         ready" to both CTAs. No TMA multicast is used.
 //   pair, 256 x 192 and 256 x 128   the same with narrower tiles (each CTA loads 96 or 64 rows of W), for launches whose
-//                         256 x 256 tiles would leave much of the last wave idle. They ask L2 for 73 and 96 bytes per clock
-//                         and SM instead of 64; a wave of them takes 0.78 and 0.55 of a wave of 256 x 256 tiles. Against the
-//                         best of the other shapes (256 x 256 pair / 128 x 128), us in bursts of 20 ms: 1961 + 231 rows,
-//                         K = 12288, N = 3072 (108 tiles on 74 pairs) 175 -> 138 with 192 columns; 2192 rows, K = 15360
-//                         217 -> 168; 11056 rows, K = 15360 920 -> 766; 2 x (1024 + 77) rows, K = 6144 48 -> 40; Q, K, V of
-//                         1024 + 256 rows, K = 3072, 75 -> 70 with 128 columns; 2 x (600 + 120) rows, K = 6144 29 -> 26.
+//                         256 x 256 tiles would leave much of the last wave idle. They ask L2 for 75 and 96 bytes per clock
+//                         and SM instead of 64; in loops at the power limit a wave of them takes 0.8 and 0.57 of a wave of
+//                         256 x 256 tiles. Against the best of the other shapes, us in bursts of 20 ms | in such loops:
+//                         1961 + 231 rows, K = 12288, N = 3072 (108 tiles of 256 x 256 on 74 pairs) 152 -> 127 | 178 -> 153
+//                         with 192 columns, K = 3072 41 -> 36 | 48 -> 42; 2 x (1024 + 77) rows, K = 6144, N = 1536 46 -> 37 |
+//                         48 -> 43; Q, K, V of 1024 + 256 rows, K = 3072, 76 -> 68 | 88 -> 79 with 128 columns; 2 x (600 +
+//                         120) rows, K = 6144 31 -> 25 | 33 -> 29.
 //
 // Biases, norm weights and rotary tables are read with __ldg(): parameters, which no kernel writes that lets another one
 // start before it has finished (host_common.h). Everything else, the gate among it, is read with plain loads. Behind plain
@@ -81,11 +82,13 @@ constexpr uint32_t kSpinLimit = 8u * 1000u * 1000u;
 constexpr int kMaxSmem = 232448;  // 227 KiB opt-in limit per CTA
 // Relative time per 128 x 128 of output for each work-unit shape, from measurement; used only to choose a shape. 256 x 256
 // pair : 128 x 256 : 128 x 128, us per wave: 10.6 : 11.8 : 6.8 per (2 : 2 : 1) blocks at K = 1536, 20.8 : 25 : 15.5 at 12464
-// rows and K = 3072, 30 : 31 : 15.2 at 1280 rows, where the clock is not held down. Pairs of 192 and 128 columns against
-// 256, us per wave: 69 : 48 : 87.5 and 18 : 12.5 : 23 at 2192 rows (K = 12288, 3072), 33.4 : 23.8 : 46 at 8858 rows and
-// K = 6144, 63 : 47 : 86 at 11056 rows and K = 12288, i.e. 1.09 and 1.16. The narrow ones count 5 % more than that: they move
-// more operand bytes per flop, which at the power limit is time. In a HunyuanVideo-shaped step (10800 + 256 rows), where the waves
-// promise 3 % for half of the layers, 192 columns gave nothing (207.1 ms against 206.2 with 256, within what runs differ by).
+// rows and K = 3072, 30 : 31 : 15.2 at 1280 rows, where the clock is not held down. Pairs of 256, 192 and 128 columns, us per
+// wave in loops at the power limit, N = 3072: 108.3 : 86.8 : 62.3 at 11056 rows and 108.6 : 88.3 : 61.1 at 5696, K = 15360;
+// 84.2 : 69.8 : 49.7 and 87.6 : 71.5 : 49.2, K = 12288. Against 1.05 for 256 columns that is 1.12 to 1.16 for 192 and 1.18 to
+// 1.24 for 128 (1.10 and 1.17 at 8900 rows, 1.27 and 1.36 at 2192, where half of the second wave of 256 leaves power to the
+// rest). In bursts, at full clock, 1.09 and 1.17 at 11056 rows: there 192 columns would win 724 : 743 us, in loops they lose
+// 868 : 866 (K = 12288 580 : 576 and 698 : 673), and a HunyuanVideo-shaped step of 11056 rows takes as long with either
+// (207.1 and 206.2 ms).
 constexpr double kCost128x256 = 1.18, kCost128x128 = 1.25, kCost256x256 = 1.3, kCostPair = 1.05,
                  kCostPair192 = 1.15, kCostPair128 = 1.2;
 
@@ -108,8 +111,8 @@ struct GemmCfg {
   static constexpr int kHalves = BM / 128;                 // 128-row MMA blocks per CTA tile
   static constexpr int kAccBufs = (kHalves == 1) ? 2 : 1;  // accumulator tiles resident in TMEM
   // Four warps reach all 128 lanes of an accumulator block; the accumulators of a pair and those of 256 columns have two
-  // such teams, each with half of the columns (128 and 64 of 192). With one team the norm + rotation tail took 28.6 k cycles per 128 x 256 accumulator, longer than the
-  // 24.6 k of the main loop at K = 3072 that it hides behind.
+  // such teams, each with half of the columns (128 and 64 of 192). With one team the norm + rotation tail took 28.6 k cycles
+  // per 128 x 256 accumulator, longer than the 24.6 k of the main loop at K = 3072 that it hides behind.
   static constexpr int kColTeams = (kHalves == 1 && (PAIR || BN == 256)) ? 2 : 1;
   static constexpr int kPieces = BN / 64;                                    // 64-column pieces of the accumulator
   static constexpr int kTeamPieces = (kPieces + kColTeams - 1) / kColTeams;  // the last team may have fewer

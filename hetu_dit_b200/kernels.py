@@ -848,9 +848,9 @@ def _group_pays(shapes, k):
     """Whether one launch over these outputs, (rows, n) each or (rows, n, 128) with a norm + rotation tail over heads of
     128, beats a library GEMM and a tail kernel per layer: what the partly filled last wave wastes (the library splits K
     there) has to stay below what the launches and the extra pass over the output cost. Measured in bursts of 20 ms, us,
-    this kernel / library: 2 layers of 1961 + 231 rows, K = 12288: 138 / 162 (192-column tiles); K = 3072: 38 / 47; 1024 +
-    256 rows, K = 12288: 83 / 93; 256 + 77 rows, K = 12288: 47 / 46 (not taken); 4096 + 512 rows, K = 12288: 253 / 274;
-    12240 + 224 rows: 671 / 660 (taken although 2 % slower alone); Q, K, V of 2 x (1024 + 77) rows, K = 1536: 34 / 50, of
+    this kernel / library: 2 layers of 1961 + 231 rows, K = 12288: 127 / 132 (192-column tiles); K = 3072: 36 / 44; 1024 +
+    256 rows, K = 12288: 83 / 93; 256 + 77 rows, K = 12288: 45 / 45 (not taken); 4096 + 512 rows, K = 12288: 253 / 274;
+    12240 + 224 rows: 671 / 660 (taken although 2 % slower alone); Q, K, V of 2 x (1024 + 77) rows, K = 1536: 27 / 41, of
     4096 + 512 rows, K = 3072 with norm and rotation: 193 / 252.
 
     The narrow tiles of a pair count for several layers only: for one the library has narrow tiles and split K as well.

@@ -433,7 +433,8 @@ HDIT_API int hdit_cfg_euler_step(int32_t dtype, const void* uncond, const void* 
  * multiples of 8; m, n, k ragged against the tile sizes are handled. `out` may alias `residual`. bias may be NULL.
  * tile_m x tile_n: output tile of one CTA, 128 x 256, 128 x 128 or 256 x 256; cta_pair = 2 makes two CTAs of a
  * cluster (an SM pair) share 256 x 256 tiles with tcgen05.mma.cta_group::2, each loading half of the W tile. Zeros
- * let the library choose by the number of waves, then among 256 x 192 and 256 x 128 tiles of a pair, too. max_ctas: 0 = one persistent CTA per SM.
+ * let the library choose by the number of waves, then among 256 x 192 and 256 x 128 tiles of a pair, too. max_ctas:
+ * 0 = one persistent CTA per SM.
  *
  * In the reference these are the torch.nn.Linear layers of the blocks it wraps followed by eager elementwise
  * kernels: the MLP of hetuDiTFeedForwardWrapper.forward (layers/feedforward.py:73-78: linear, GELU, linear) and the
